@@ -21,16 +21,21 @@ struct WaveMaps {
 
 // Tile height of the single-instance wave stage kernel (see wave_ty).
 inline int wave_tile_height(int elem_bytes, int kind = WK_HOM) {
-  if (elem_bytes == 8) return kind == WK_HOM ? wave_ty<double, WK_HOM>() : wave_ty<double, WK_VAR>();
+  if (elem_bytes == 8)
+    return kind == WK_HOM ? wave_ty<double, WK_HOM>()
+                          : (kind == WK_VAR ? wave_ty<double, WK_VAR>() : wave_ty<double, WK_MMS>());
   return kind == WK_VAR ? wave_ty<float, WK_VAR>() : wave_ty<float, WK_HOM>();
 }
+
+// The interior stencil's common denominator (FixDen).
+inline double fixed_denominator(int order) { return order == 2 ? 2.0 : (order == 4 ? 12.0 : 60.0); }
 
 // Scales of the fixed-point FP64 stages (wave2d_fixed.cuh) for one launch: the
 // RHS in units of sigma = -hi/den per direction, and the stage's RK4
 // coefficients times sigma of each component (u and p: x, v: y). Every launch of
-// a constant-coefficient FP64 stage sets them; the kernel refuses to run without.
+// an FP64 stage sets them; the kernel refuses to run without.
 inline void set_fixed_scales(WaveParams<double>& p, int order, double hix, double hiy) {
-  const double den = order == 2 ? 2.0 : (order == 4 ? 12.0 : 60.0);
+  const double den = fixed_denominator(order);
   p.fx_sig[0] = -hix / den;
   p.fx_sig[1] = -hiy / den;
   p.fx_isig[0] = -den / hix;
@@ -128,6 +133,12 @@ inline cudaError_t launch_batch(int order, bool wave, int stage, int cfg, const 
     default: return cudaErrorInvalidValue;
   }
 }
+
+// The manufactured-solution problem's coefficient planes at `out` (three planes of ny
+// rows of `pitch`): 1/rho = 1/(2 + x y), then the forcing of u and v without its time
+// factor, in units of sigma_x and sigma_y (set_fixed_scales).
+cudaError_t launch_mms_coefficients(double* out, int nx, int ny, long long pitch, long long plane, double xl0,
+                                    double xl1, double hix, double hiy, int order, cudaStream_t s);
 
 // AoS FP64 (reference layout) <-> SoA planes of T with a row pitch.
 template <typename T>

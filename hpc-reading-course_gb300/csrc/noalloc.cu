@@ -173,7 +173,6 @@ extern "C" int sbp_wave_rhs_noalloc(const sbp_desc* d, double t, const double* s
   p.bc = d->bc == SBP_BC_CHARACTERISTIC ? BC_CHARACTERISTIC : BC_FREE_SURFACE;
   p.in = in;
   p.kout = out;
-  p.t = t;
   p.err = err;
   set_fixed_scales(p, d->order, hix, hiy);
 

@@ -66,7 +66,8 @@ struct sbp_ctx {
   double* io = nullptr;       // AoS FP64 staging, nscalar
   double* partial = nullptr;  // reduction scratch, 2 * kReduceBlocks
   double* red = nullptr;      // reduction result, 4
-  void *rinv = nullptr, *kmod = nullptr;     // WAVE_VAR: T planes
+  void *rinv = nullptr, *kmod = nullptr;     // WAVE_VAR: T planes; WAVE_MMS: 1/rho and two forcing planes at rinv
+  double* ct_tab = nullptr;                  // WAVE_MMS: the forcing's time factor per stage of a step graph
   void *va = nullptr, *vb = nullptr;         // advection with velocity fields: T planes (pitched)
   double *va64 = nullptr, *vb64 = nullptr;   // the same in FP64, nx*ny row-major (SAT)
   double *rho64 = nullptr, *k64 = nullptr;   // WAVE_VAR: nx*ny FP64
@@ -153,12 +154,14 @@ int make_maps(sbp_ctx* ctx, void* base, WaveMaps& m) {
     m.k = m.p;  // no coefficient fields: the map is never used
     return SBP_OK;
   }
-  // [1/rho | K]: two planes at rinv (kmod follows it), as a 2-component point box
+  // the coefficient planes at rinv ([1/rho | K], or the manufactured solution's three), as
+  // one point box
+  const int nk = ctx->d.problem == SBP_WAVE_MMS_2D ? 3 : 2;
   EncodeTiledFn enc = encode_tiled();
-  const cuuint64_t dims[3] = {(cuuint64_t)ctx->nx, (cuuint64_t)ctx->ny, 2};
+  const cuuint64_t dims[3] = {(cuuint64_t)ctx->nx, (cuuint64_t)ctx->ny, (cuuint64_t)nk};
   const cuuint64_t strides[2] = {(cuuint64_t)(ctx->pitch * ctx->es), (cuuint64_t)(ctx->plane * ctx->es)};
   const cuuint32_t estr[3] = {1, 1, 1};
-  const cuuint32_t boxK[3] = {(cuuint32_t)kWaveTX, (cuuint32_t)TY, 2};
+  const cuuint32_t boxK[3] = {(cuuint32_t)kWaveTX, (cuuint32_t)TY, (cuuint32_t)nk};
   const CUtensorMapDataType dt = ctx->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64;
   if (enc(&m.k, dt, 3, ctx->rinv, dims, strides, boxK, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -186,10 +189,6 @@ WaveParams<T> wave_params(sbp_ctx* ctx) {
   p.bwy = ctx->hiy * hi0;
   p.bc = ctx->d.bc == SBP_BC_CHARACTERISTIC ? BC_CHARACTERISTIC : BC_FREE_SURFACE;
   p.ysplit = ctx->ysplit;
-  p.xl0 = ctx->d.xl[0];
-  p.xl1 = ctx->d.xl[1];
-  p.hix = ctx->hix;
-  p.hiy = ctx->hiy;
   p.err = ctx->err;
   return p;
 }
@@ -234,11 +233,15 @@ int line_kind(const sbp_ctx* ctx) {
   return ctx->d.problem == SBP_ADVECTION_1D ? LK_ADV1D : (ctx->d.problem == SBP_REFLECTION_1D ? LK_REFL1D : LK_ADV2D);
 }
 
+// The time factor of the manufactured solution's forcing (code/demo/wave/wave_eq_rhs.h:51-64).
+double mms_time_factor(double t) { return std::cos(5 * 3.14159265358979323846264 * t); }
+
 // Launches one kernel of the stage sequence. `in` is the state the RHS is
 // evaluated on; `in_maps` its TMA descriptors (2D wave only).
 template <typename T>
 int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in, const WaveMaps* in_maps,
-                 void* kout, int bc_on, const Rk45Ctrl* ctl = nullptr, double tc = 0.0) {
+                 void* kout, int bc_on, const Rk45Ctrl* ctl = nullptr, double tc = 0.0,
+                 const double* ctp = nullptr) {
   T c_acc = 0, c_w = 0;
   if (stage == ST_FIRST) {
     c_acc = (T)(dt / 6);
@@ -260,7 +263,10 @@ int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in,
     p.comp = (T*)ctx->comp;
     p.c_acc = c_acc;
     p.c_w = c_w;
-    p.t = t;
+    if (ctx->time_dependent) {
+      p.ct = mms_time_factor(t);
+      p.ctp = ctp;
+    }
     p.wait_ns = ctx->wait_ns;
     p.sched = ctx->sched;
     if constexpr (sizeof(T) == 8) set_fixed_scales(p, ctx->d.order, ctx->hix, ctx->hiy);
@@ -324,13 +330,28 @@ int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in,
 // One classical RK4 step on the resident state (time_stepping.h:127-142):
 // stage 1 reads u^n and writes acc, wa; stage 2 reads wa, writes acc, wb;
 // stage 3 reads wb, writes acc, wa; stage 4 reads wa, acc and writes u^{n+1}.
+// Time-dependent problems: `ct` is where in device memory the step's three stage-time
+// factors are when the step runs (at t, t + dt/2, t + dt); null, they come from t.
 template <typename T>
-int enqueue_step(sbp_ctx* ctx, double t, double dt) {
-  int rc;
-  if ((rc = launch_stage<T>(ctx, ST_FIRST, 1, t, dt, ctx->un, &ctx->maps_un, nullptr, 1))) return rc;
-  if ((rc = launch_stage<T>(ctx, ST_MID, 2, t + 0.5 * dt, dt, ctx->wa, &ctx->maps_wa, nullptr, 1))) return rc;
-  if ((rc = launch_stage<T>(ctx, ST_MID, 3, t + 0.5 * dt, dt, ctx->wb, &ctx->maps_wb, nullptr, 1))) return rc;
-  return launch_stage<T>(ctx, ST_LAST, 4, t + dt, dt, ctx->wa, &ctx->maps_wa, nullptr, 1);
+int enqueue_step(sbp_ctx* ctx, double t, double dt, const double* ct = nullptr) {
+  struct Part {
+    int stage;
+    double t;
+    void* in;
+    const WaveMaps* maps;
+    int at;  // the stage time's place in ct
+  };
+  const Part parts[4] = {{ST_FIRST, t, ctx->un, &ctx->maps_un, 0},
+                         {ST_MID, t + 0.5 * dt, ctx->wa, &ctx->maps_wa, 1},
+                         {ST_MID, t + 0.5 * dt, ctx->wb, &ctx->maps_wb, 1},
+                         {ST_LAST, t + dt, ctx->wa, &ctx->maps_wa, 2}};
+  for (int s = 0; s < 4; s++) {
+    const Part& p = parts[s];
+    const int rc = launch_stage<T>(ctx, p.stage, s + 1, p.t, dt, p.in, p.maps, nullptr, 1, nullptr, 0.0,
+                                   ct ? ct + p.at : nullptr);
+    if (rc) return rc;
+  }
+  return SBP_OK;
 }
 
 void drop_graphs(sbp_ctx* ctx) {
@@ -338,8 +359,13 @@ void drop_graphs(sbp_ctx* ctx) {
   ctx->graphs.clear();
 }
 
+constexpr long long kRk4Chunk = 50;  // steps per graph launch
+
+// `steps` (at most kRk4Chunk) steps from time t as one graph, captured once per step count
+// and dt. Time-dependent problems: the steps' stage-time factors go to ct_tab, in stream
+// order before the graph that reads them.
 template <typename T>
-int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt) {
+int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt, double* t) {
   if (ctx->graph_dt != dt) {
     drop_graphs(ctx);
     ctx->graph_dt = dt;
@@ -350,7 +376,8 @@ int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt) {
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     const long long before = ctx->launches;
     int rc = SBP_OK;
-    for (long long s = 0; s < steps && rc == SBP_OK; s++) rc = enqueue_step<T>(ctx, 0.0, dt);
+    for (long long s = 0; s < steps && rc == SBP_OK; s++)
+      rc = enqueue_step<T>(ctx, 0.0, dt, ctx->ct_tab ? ctx->ct_tab + 3 * s : nullptr);
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
     ctx->launches = before;  // captured, not yet run
     if (rc) {
@@ -364,6 +391,16 @@ int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt) {
     CK(ie);
     it = ctx->graphs.emplace(steps, ex).first;
   }
+  if (ctx->ct_tab) {
+    double h[3 * kRk4Chunk];
+    for (long long s = 0; s < steps; s++) {
+      h[3 * s] = mms_time_factor(*t);
+      h[3 * s + 1] = mms_time_factor(*t + 0.5 * dt);
+      h[3 * s + 2] = mms_time_factor(*t + dt);
+      *t = *t + dt;
+    }
+    CK(cudaMemcpyAsync(ctx->ct_tab, h, 3 * steps * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+  }
   CK(cudaGraphLaunch(it->second, ctx->stream));
   ctx->launches += 4 * steps;
   return SBP_OK;
@@ -371,23 +408,24 @@ int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt) {
 
 template <typename T>
 int rk4_resident_t(sbp_ctx* ctx, double t0, double dt, long long nsteps) {
-  if (ctx->time_dependent) {  // stage times change every step: direct launches
-    double t = t0;
-    for (long long s = 0; s < nsteps; s++) {
+  double t = t0;
+  long long left = nsteps;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (ctx->time_dependent) CK(cudaStreamIsCapturing(ctx->stream, &cap));
+  if (cap != cudaStreamCaptureStatusNone) {  // the caller is capturing: launches with the stage times as values
+    for (; left > 0; left--) {
       int rc = enqueue_step<T>(ctx, t, dt);
       if (rc) return rc;
       t = t + dt;
     }
     return SBP_OK;
   }
-  const long long chunk = 50;
-  long long left = nsteps;
-  while (left >= chunk) {
-    int rc = run_chunk_graph<T>(ctx, chunk, dt);
+  while (left >= kRk4Chunk) {
+    int rc = run_chunk_graph<T>(ctx, kRk4Chunk, dt, &t);
     if (rc) return rc;
-    left -= chunk;
+    left -= kRk4Chunk;
   }
-  if (left > 0) return run_chunk_graph<T>(ctx, left, dt);
+  if (left > 0) return run_chunk_graph<T>(ctx, left, dt, &t);
   return SBP_OK;
 }
 
@@ -510,6 +548,7 @@ int launch_rkf_wave_stage(sbp_ctx* ctx, int s, void* in, const WaveMaps* in_maps
   p.rkatol = ctx->rk_atol;
   p.rkrtol = ctx->rk_rtol;
   p.wait_ns = ctx->wait_ns;
+  set_fixed_scales(p, ctx->d.order, ctx->hix, ctx->hiy);
   CK(launch_wave<double>(ctx->d.order, wave_kind(ctx), ST_RKF1 + s - 1, *in_maps, p, ctx->stream));
   ctx->launches++;
   return SBP_OK;
@@ -608,7 +647,7 @@ void release(sbp_ctx* ctx) {
   if (ctx->rk_unew) cudaFree(ctx->rk_unew);
   if (ctx->rk_ctrl) cudaFree(ctx->rk_ctrl);
   void* bufs[] = {ctx->un, ctx->acc, ctx->wa, ctx->wb, ctx->comp, ctx->io, ctx->partial, ctx->red,
-                  ctx->rinv, ctx->rho64, ctx->k64, ctx->err, ctx->sched, ctx->va, ctx->va64};
+                  ctx->rinv, ctx->rho64, ctx->k64, ctx->err, ctx->sched, ctx->va, ctx->va64, ctx->ct_tab};
   // kmod lives inside the rinv allocation, vb and vb64 inside those of va and va64
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -750,6 +789,16 @@ int sbp_create(const sbp_desc* desc, sbp_ctx** out) {
     e = cudaDeviceSynchronize();
     cudaFree(tmp);
     if (e != cudaSuccess) return cuda_fail("coefficient upload", e);
+  }
+  if (d.problem == SBP_WAVE_MMS_2D) {
+    if ((e = cudaMalloc(&ctx->rinv, 3 * ctx->plane * ctx->es)) != cudaSuccess ||
+        (e = cudaMalloc((void**)&ctx->ct_tab, 3 * kRk4Chunk * sizeof(double))) != cudaSuccess)
+      return cuda_fail("cudaMalloc(coefficients)", e);
+    cudaMemset(ctx->rinv, 0, 3 * ctx->plane * ctx->es);
+    if ((e = launch_mms_coefficients((double*)ctx->rinv, (int)ctx->nx, (int)ctx->ny, ctx->pitch, ctx->plane, d.xl[0],
+                                     d.xl[1], ctx->hix, ctx->hiy, d.order, 0)) != cudaSuccess ||
+        (e = cudaDeviceSynchronize()) != cudaSuccess)
+      return cuda_fail("coefficients", e);
   }
   const bool adv = d.problem == SBP_ADVECTION_1D || d.problem == SBP_ADVECTION_2D;
   if (!adv && (d.a_field || d.b_field)) {

@@ -40,16 +40,12 @@ enum Stage : int { ST_RHS = 0, ST_FIRST = 1, ST_MID = 2, ST_LAST = 4, ST_RKF1 = 
 // error partial sum (s = 6).
 constexpr bool is_rkf_stage(int stage) { return stage >= ST_RKF1 && stage <= ST_RKF6; }
 
-// The constant-coefficient FP64 stages (RHS and RK4; rho = K = 1) evaluate their
-// interior stencils in exact integer arithmetic (wave2d_fixed.cuh) instead of
-// FP64 FMAs, which GB300 issues at about 1/64 of its FP32 rate. The build may set
-// SBP_FP64_FIXED=0 to compare with the FP64 tap chains.
-#ifndef SBP_FP64_FIXED
-#define SBP_FP64_FIXED 1
-#endif
-template <typename T, int KIND, int STAGE> constexpr bool wave_fixed() {
-  return SBP_FP64_FIXED != 0 && sizeof(T) == 8 && KIND == WK_HOM && !is_rkf_stage(STAGE);
-}
+// Every FP64 stage of the single grid (RHS, RK4 and Fehlberg stages; constant, variable
+// and manufactured-solution coefficients) evaluates its interior stencils in exact
+// integer arithmetic (wave2d_fixed.cuh) instead of FP64 FMAs, which GB300 issues at
+// about 1/64 of its FP32 rate: the tap chains are 16 of the 24 FP64 instructions of a
+// variable-coefficient point-stage at order 4, and 96 of the 225 of a Fehlberg attempt.
+template <typename T, int KIND, int STAGE> constexpr bool wave_fixed() { return sizeof(T) == 8; }
 
 struct FxSub;   // a subdomain of a decomposed grid (wave2d_fixed.cuh)
 struct FxTile;  // a tile of a decomposed grid (wave2d_fixed.cuh)
@@ -77,7 +73,11 @@ template <typename T> struct WaveParams {
   int bc;             // BcKind
   int ysplit;         // 0: one block; else rows [0,ysplit) and [ysplit,ny) are two blocks
                       // sharing an interface line (WK_VAR only)
-  double t, xl0, xl1, hix, hiy;  // WK_MMS: stage time and grid geometry
+  // WK_MMS: the forcing's time factor cos(5 pi t) of the stage, as a value or (in a captured
+  // step graph) the place in device memory that holds it
+  double ct;
+  const double* ctp;
+  double hix, hiy;     // 1/h per direction (decomposed grids: the fixed-point scales)
   const double* tctl;  // the adaptive integrator's (t, h); WK_MMS stage time tctl[0] + tc * tctl[1]
   double tc;
   const int* skip;     // non-null and set: the kernel returns at entry
@@ -154,18 +154,23 @@ template <typename T> constexpr int default_wave_ty() { return sizeof(T) == 8 ? 
 #define SBP_FP64_WARPS 14
 #endif
 
-// Tile height of the single-instance kernel: the variable-coefficient FP32
-// kind also stages 1/rho and K, so it uses 24 rows to keep two stages in 227 KB.
+// Tile height of the single-instance kernels. The kinds with coefficient planes stage
+// those too, and use the height that keeps the ring depth below within 227 KB: FP32
+// variable coefficients 24 rows (two stages), FP64 variable coefficients 12 and the
+// manufactured solution 11 (three stages).
 template <typename T, int KIND> constexpr int wave_ty() {
-  return sizeof(T) == 8 ? (KIND == WK_HOM ? SBP_FP64_TILE_ROWS : 16) : (KIND == WK_VAR ? 24 : SBP_FP32_TILE_ROWS);
+  return sizeof(T) == 8 ? (KIND == WK_HOM ? SBP_FP64_TILE_ROWS : (KIND == WK_VAR ? 12 : 11))
+                        : (KIND == WK_VAR ? 24 : SBP_FP32_TILE_ROWS);
 }
+// Coefficient planes staged per tile: [1/rho | K], or the manufactured solution's
+// [1/rho | forcing u | forcing v].
+template <typename T, int KIND> constexpr int wave_coef() { return KIND == WK_VAR ? 2 : (KIND == WK_MMS ? 3 : 0); }
 // Shared-memory ring depth (tiles in flight + the one being computed).
 #ifndef SBP_FP64_RING
 #define SBP_FP64_RING 3
 #endif
 // Converter warps of the fixed-point FP64 stages: they convert tile k+1 to int64
-// while the compute warps work on tile k (0: the compute warps convert each tile
-// themselves, between two barriers).
+// while the compute warps work on tile k.
 #ifndef SBP_FP64_CONV
 #define SBP_FP64_CONV 6
 #endif
@@ -176,18 +181,19 @@ template <typename T, int KIND> constexpr int wave_ty() {
 #ifndef SBP_FP64_RING_FL
 #define SBP_FP64_RING_FL 4
 #endif
+// The Fehlberg and RHS stages load no point boxes: a ring of 6 stages.
+#ifndef SBP_FP64_RING_RKF
+#define SBP_FP64_RING_RKF 6
+#endif
 template <typename T, int KIND, int STAGE = ST_MID> constexpr int wave_ring() {
-  return (sizeof(T) == 4 && KIND != WK_VAR)
-             ? SBP_FP32_RING
-             : (sizeof(T) == 8 && KIND == WK_HOM ? ((STAGE == ST_FIRST || STAGE == ST_LAST) ? SBP_FP64_RING_FL
-                                                                                            : SBP_FP64_RING)
-                                                 : 2);
+  if (sizeof(T) == 4) return KIND != WK_VAR ? SBP_FP32_RING : 2;
+  if (is_rkf_stage(STAGE)) return KIND == WK_HOM ? SBP_FP64_RING_RKF : 4;
+  return (KIND == WK_HOM && (STAGE == ST_FIRST || STAGE == ST_LAST)) ? SBP_FP64_RING_FL : SBP_FP64_RING;
 }
-// Consumer warps of the single-instance kernel. The variable-coefficient and
-// manufactured-solution FP64 kernels need up to 166 registers a thread, which
-// leaves room for 8 warps; the constant-coefficient FP64 kernels (at most 128)
-// run 12 with one tile row each, the constant-coefficient FP32 kernels 16 with
-// two rows each (more warps hide more load latency).
+// Consumer (compute) warps of the single-instance kernels. FP64: one tile row each (the
+// Fehlberg stages of constant and variable coefficients two rows each: they hold up to
+// six derivatives of a point in registers). FP32: 16 with two rows each for constant
+// coefficients (more warps hide more load latency), 12 for variable coefficients.
 #ifndef SBP_FP32_WARPS
 #define SBP_FP32_WARPS 16
 #endif
@@ -196,18 +202,15 @@ template <typename T, int KIND, int STAGE = ST_MID> constexpr int wave_ring() {
 #ifndef SBP_FP32_VAR_WARPS
 #define SBP_FP32_VAR_WARPS 12
 #endif
-// Where the variable-coefficient kernels read 1/rho and K: 1 from the tile's
-// TMA box in shared memory, 0 with read-only global loads (no box), 2 both
-// (the box loaded but unused; kept to measure what the box costs).
-#ifndef SBP_VAR_COEF
-#define SBP_VAR_COEF 1
-#endif
-template <typename T, int KIND> constexpr int wave_warps() {
-  return sizeof(T) == 4 ? (KIND != WK_VAR ? SBP_FP32_WARPS : SBP_FP32_VAR_WARPS)
-                        : (KIND == WK_HOM ? SBP_FP64_WARPS : kWaveConsumerWarps);
+template <typename T, int KIND, int STAGE = ST_MID> constexpr int wave_warps() {
+  if (sizeof(T) == 4) return KIND != WK_VAR ? SBP_FP32_WARPS : SBP_FP32_VAR_WARPS;
+  return KIND == WK_HOM ? SBP_FP64_WARPS : wave_ty<T, KIND>();
+}
+template <int KIND, int STAGE> constexpr int wave_conv() {
+  return !is_rkf_stage(STAGE) ? SBP_FP64_CONV : (KIND == WK_VAR ? 3 : 4);
 }
 
-template <typename T, int ORD, int STAGE, int TY_ = default_wave_ty<T>(), int PRM_BYTES = 0, bool COEF = false,
+template <typename T, int ORD, int STAGE, int TY_ = default_wave_ty<T>(), int PRM_BYTES = 0, int COEF = 0,
           int NST_ = 2, int WARPS_ = kWaveConsumerWarps, bool FIX_ = false, int CONV_ = 0>
 struct WaveTile {
   static constexpr int WARPS = WARPS_;                        // consumer (compute) warps
@@ -230,7 +233,7 @@ struct WaveTile {
   static constexpr bool LOAD_UN = (STAGE == ST_MID) || (STAGE == ST_LAST && COMP) || (FIX_ && STAGE == ST_FIRST);
   static constexpr bool LOAD_ACC = (STAGE == ST_MID) || (STAGE == ST_LAST);
   static constexpr bool LOAD_COMP = (STAGE == ST_LAST && COMP);
-  static constexpr bool LOAD_COEF = COEF;  // 1/rho and K planes as one 2-component point box
+  static constexpr bool LOAD_COEF = COEF > 0;  // coefficient planes as one COEF-component point box
   static constexpr int align128(int b) { return (b + 127) / 128 * 128; }
   static constexpr int BYTES_P = PH * PW * (int)sizeof(T);
   static constexpr int BYTES_U = TY * PW * (int)sizeof(T);
@@ -241,7 +244,7 @@ struct WaveTile {
   static constexpr int OFF_N = OFF_V + align128(BYTES_V);
   static constexpr int OFF_A = OFF_N + (LOAD_UN ? BYTES_PT : 0);
   static constexpr int OFF_C = OFF_A + (LOAD_ACC ? BYTES_PT : 0);
-  static constexpr int BYTES_K = 2 * TY * kWaveTX * (int)sizeof(T);
+  static constexpr int BYTES_K = COEF * TY * kWaveTX * (int)sizeof(T);
   static constexpr int OFF_K = align128(OFF_C + (LOAD_COMP ? BYTES_PT : 0));
   static constexpr int OFF_PRM = align128(OFF_K + (LOAD_COEF ? BYTES_K : 0));  // batched: instance parameters
   // the RHS of the tile's x-face points, kept for the deferred SAT pass ([side][row][u, v, p])
@@ -252,9 +255,8 @@ struct WaveTile {
   static constexpr int OFF_DBAR = OFF_BAR + 128;              // deferred-pass barriers[NST]
   // + 192: the tile index of each stage (int[NST]; -1 marks the end)
   // Fixed-point stages, at OFF_FX: barriers[8] "exponent maxima known" (+0) and
-  // "boxes converted" (+64), then per stage the p and u/v exponent maxima: one pair
-  // per converter warp (int[8][8][2], +128) when converter warps convert, or one
-  // shared pair (int[8][2]) when the compute warps do.
+  // "boxes converted" (+64), then per stage and converter warp the p and u/v exponent
+  // maxima (int[8][8][2], +128).
   static constexpr int OFF_FX = OFF_BAR + 256;
   // Decomposed grids: eight 192-byte slots of tile geometry (that of its subdomain's
   // neighbours included): one per ring stage, the rest the exchange queue; then the
@@ -318,8 +320,6 @@ template <typename T, int ORD>
 __device__ __noinline__ T closure_line_global(const T* line, long long st, int n, int i, const T (&cls)[6][9]) {
   return closure_line<T, ORD>(line, st, n, i, cls);
 }
-
-__device__ __forceinline__ double mms_x(double xl, int i, double hi) { return xl + (double)i / hi; }
 
 template <typename T> struct Rhs3 { T u, v, p; };
 
@@ -411,9 +411,9 @@ __device__ __forceinline__ void wave_point_store(const WaveParams<T>& prm, T* wo
 
 // Fehlberg stage S = STAGE - ST_RKF1 + 1 of component c of one point: the same
 // sums, in the same order, as the unfused combination kernels (rk45.cu). kS is
-// this stage's derivative, pre[0..S-2] = k_1..k_{S-1} and pre[S-1] = u (S > 1).
+// this stage's derivative, pre[0..S-2] = k_1..k_{S-1} and pre[S-1] = u.
 template <typename T, int STAGE, int NPRE>
-__device__ __forceinline__ void wave_point_rkf(const WaveParams<T>& prm, T* wout, long long o, double kS, double cen,
+__device__ __forceinline__ void wave_point_rkf(const WaveParams<T>& prm, T* wout, long long o, double kS,
                                                const double (&pre)[NPRE], double* errsq) {
   constexpr int S = STAGE - ST_RKF1 + 1;
   const double h = prm.tctl[1];
@@ -422,8 +422,7 @@ __device__ __forceinline__ void wave_point_rkf(const WaveParams<T>& prm, T* wout
     double s = kRkfA[S][0] * (S == 1 ? kS : pre[0]);
 #pragma unroll
     for (int jj = 1; jj < S; jj++) s = fma(kRkfA[S][jj], jj == S - 1 ? kS : pre[jj], s);
-    const double u0 = S == 1 ? cen : pre[S - 1];
-    st_stream(wout + o, fma(h, s, u0));
+    st_stream(wout + o, fma(h, s, pre[S - 1]));
   } else {
     double u5, u4;
     rkf_candidate(pre[5], h, pre[0], pre[2], pre[3], pre[4], kS, u5, u4);
@@ -436,12 +435,10 @@ __device__ __forceinline__ void wave_point_rkf(const WaveParams<T>& prm, T* wout
 // does not need k2: its weights are zero).
 template <typename T, int RKS>
 __device__ __forceinline__ void wave_rkf_preload(const WaveParams<T>& prm, long long o, double (&pre)[RKS]) {
-  if constexpr (RKS > 1) {
 #pragma unroll
-    for (int jj = 0; jj < RKS - 1; jj++)
-      if (RKS < 6 || jj != 1) pre[jj] = __ldg(prm.rkk[jj] + o);
-    pre[RKS - 1] = __ldg(prm.rku + o);
-  }
+  for (int jj = 0; jj < RKS - 1; jj++)
+    if (RKS < 6 || jj != 1) pre[jj] = __ldg(prm.rkk[jj] + o);
+  pre[RKS - 1] = __ldg(prm.rku + o);
 }
 
 // One tile of the stage for the consumer warps: everything the tile needs is
@@ -451,7 +448,7 @@ template <typename T, int ORD, int KIND, int STAGE, typename Tile>
 __device__ __forceinline__ void wave_tile_compute(const WaveParams<T>& prm, const T* __restrict__ in, T* wout,
                                                   const T c_acc, const T c_w, const unsigned char* st, const int i0,
                                                   const int j0, const int warp, const int lane,
-                                                  double* errsq = nullptr, uint64_t* dbar = nullptr,
+                                                  uint64_t* dbar = nullptr,
                                                   uint32_t* dphase = nullptr, const int b = 0, const int k = 0) {
   constexpr bool COMP = Tile::COMP;
   constexpr int TY = Tile::TY, W = OpShape<ORD>::W, CS = OpShape<ORD>::CS, R = Tile::R;
@@ -475,8 +472,7 @@ __device__ __forceinline__ void wave_tile_compute(const WaveParams<T>& prm, cons
   // after every consumer warp has passed the tile's rows, one warp applies the
   // SAT and the update to all of them, one point per lane. In a row warp a single
   // x-face lane would hold the FP64 pipe for the whole SAT sequence.
-  constexpr bool DEFER_OK = true;  // every stage kind, Fehlberg stages included
-  const bool xfaces = DEFER_OK && dbar != nullptr && prm.bc != BC_NONE &&
+  const bool xfaces = dbar != nullptr && prm.bc != BC_NONE &&
                       (i0 == 0 || (nx - 1 >= i0 && nx - 1 < i0 + kWaveTX));
   T* sD = reinterpret_cast<T*>(const_cast<unsigned char*>(st) + Tile::OFF_DEF);
   (void)sD;
@@ -513,17 +509,6 @@ __device__ __forceinline__ void wave_tile_compute(const WaveParams<T>& prm, cons
       const T* colP = sP + y * PW + (x + HX);   // row y+HY-R
       const T* colV = sV + y * kWaveTX + x;     // row y+HY-R
       const T pc = rowP[R], uc = rowU[R], vc = colV[R * kWaveTX];
-      // Fehlberg stages: the point's u and k_1..k_{S-1} are loaded here, ahead of
-      // the stencil arithmetic, so that their latency overlaps it (stage 6 does
-      // not need k2: its weights are zero).
-      constexpr int RKS = is_rkf_stage(STAGE) ? STAGE - ST_RKF1 + 1 : 1;
-      double rkpre[3][RKS];  // [c][0..RKS-2] = k_1..k_{RKS-1}, [c][RKS-1] = u (RKS > 1)
-      if constexpr (RKS > 1) {
-        const long long q0 = (long long)j * pitch + i;
-#pragma unroll
-        for (int c = 0; c < 3; c++) wave_rkf_preload<T, RKS>(prm, c * plane + q0, rkpre[c]);
-      }
-      (void)rkpre;
 
       T dxp, dyp, kp;
       if (xint) {
@@ -576,27 +561,12 @@ __device__ __forceinline__ void wave_tile_compute(const WaveParams<T>& prm, cons
         kv = dyp;
         kp = prm.kconst * kp;
       } else if constexpr (KIND == WK_VAR) {
-        T ri, km;
-        if constexpr (SBP_VAR_COEF == 1) {  // the tile's [1/rho | K] box
-          ri = sK[y * kWaveTX + x];
-          km = sK[TPT + y * kWaveTX + x];
-        } else {
-          ri = __ldg(prm.rinv + q);
-          km = __ldg(prm.kmod + q);
-        }
+        // the tile's [1/rho | K] box (read-only global loads instead: 4.68e10 against
+        // 6.99e10 point-stage updates/s in FP32 at 4096^2)
+        const T ri = sK[y * kWaveTX + x], km = sK[TPT + y * kWaveTX + x];
         ku = ri * dxp;
         kv = ri * dyp;
         kp = km * kp;
-      } else {  // WK_MMS (FP64): code/demo/wave/wave_eq_rhs.h:42-64
-        const double PI = 3.14159265358979323846264;
-        const double xx = mms_x(prm.xl0, i, prm.hix), yy = mms_x(prm.xl1, j, prm.hiy);
-        const double ri = 1. / (2 + xx * yy);
-        const double ts = prm.tctl ? __dadd_rn(prm.tctl[0], __dmul_rn(prm.tc, prm.tctl[1])) : prm.t;
-        const double ct = cos(5 * PI * ts);
-        const double fu = -(3 * PI * ct * cos(3 * PI * xx) * sin(4 * PI * yy) * (xx * yy + 1)) / (xx * yy + 2);
-        const double fv = -(4 * PI * ct * cos(4 * PI * yy) * sin(3 * PI * xx) * (xx * yy + 1)) / (xx * yy + 2);
-        ku = (T)(ri * (double)dxp + fu);
-        kv = (T)(ri * (double)dyp + fv);
       }
 
       // SAT boundary terms (boundary points only)
@@ -623,62 +593,46 @@ __device__ __forceinline__ void wave_tile_compute(const WaveParams<T>& prm, cons
 #pragma unroll
       for (int c = 0; c < 3; c++) {
         const long long o = c * plane + q;
-        if constexpr (STAGE == ST_RHS) {
-          prm.kout[o] = kc[c];
-        } else if constexpr (is_rkf_stage(STAGE)) {
-          wave_point_rkf<T, STAGE, RKS>(prm, wout, o, (double)kc[c], (double)cen[c], rkpre[c], errsq);
-        } else {
-          wave_point_store<T, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, sC, sp, c, o, kc[c], cen[c]);
-        }
+        wave_point_store<T, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, sC, sp, c, o, kc[c], cen[c]);
       }
     }
   }
-  if constexpr (DEFER_OK) {
-    if (xfaces) {
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dbar);  // this warp's deferred entries are in shared memory
-      const uint32_t par = (*dphase >> b) & 1u;
-      *dphase ^= 1u << b;
-      if (warp != k % Tile::WARPS) return;
-      if (!mbar_wait_bounded(dbar, par, prm.wait_ns)) {
-        if (lane == 0) atomicOr(prm.err, ERR_TMA_TIMEOUT);
-        return;
-      }
-      for (int e = lane; e < 2 * TY; e += 32) {
-        const int side = e / TY, y = e - side * TY, j = j0 + y;
-        const int i = side == 0 ? 0 : nx - 1;
-        if (i < i0 || i >= i0 + kWaveTX || j >= ny || j == 0 || j == ny - 1 ||
-            (prm.ysplit > 0 && (j == prm.ysplit - 1 || j == prm.ysplit)))
-          continue;
-        const int x = i - i0;
-        const T pc = sP[(y + HY) * PW + x + HX], uc = sU[y * PW + x + HX], vc = sV[(y + HY) * kWaveTX + x];
-        const T* d = sD + (side * TY + y) * 3;
-        const Rhs3<T> r = apply_sat<T, KIND>(prm, in, i, j, pc, uc, vc, Rhs3<T>{d[0], d[1], d[2]});
-        const T kc[3] = {r.u, r.v, r.p};
-        const T cen[3] = {uc, vc, pc};
-        const long long q = (long long)j * pitch + i;
-        const int sp = y * kWaveTX + x;
+  if (xfaces) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(dbar);  // this warp's deferred entries are in shared memory
+    const uint32_t par = (*dphase >> b) & 1u;
+    *dphase ^= 1u << b;
+    if (warp != k % Tile::WARPS) return;
+    if (!mbar_wait_bounded(dbar, par, prm.wait_ns)) {
+      if (lane == 0) atomicOr(prm.err, ERR_TMA_TIMEOUT);
+      return;
+    }
+    for (int e = lane; e < 2 * TY; e += 32) {
+      const int side = e / TY, y = e - side * TY, j = j0 + y;
+      const int i = side == 0 ? 0 : nx - 1;
+      if (i < i0 || i >= i0 + kWaveTX || j >= ny || j == 0 || j == ny - 1 ||
+          (prm.ysplit > 0 && (j == prm.ysplit - 1 || j == prm.ysplit)))
+        continue;
+      const int x = i - i0;
+      const T pc = sP[(y + HY) * PW + x + HX], uc = sU[y * PW + x + HX], vc = sV[(y + HY) * kWaveTX + x];
+      const T* d = sD + (side * TY + y) * 3;
+      const Rhs3<T> r = apply_sat<T, KIND>(prm, in, i, j, pc, uc, vc, Rhs3<T>{d[0], d[1], d[2]});
+      const T kc[3] = {r.u, r.v, r.p};
+      const T cen[3] = {uc, vc, pc};
+      const long long q = (long long)j * pitch + i;
+      const int sp = y * kWaveTX + x;
 #pragma unroll
-        for (int c = 0; c < 3; c++) {
-          if constexpr (is_rkf_stage(STAGE)) {
-            constexpr int RKS = STAGE - ST_RKF1 + 1;
-            double pre[RKS];
-            wave_rkf_preload<T, RKS>(prm, c * plane + q, pre);
-            wave_point_rkf<T, STAGE, RKS>(prm, wout, c * plane + q, (double)kc[c], (double)cen[c], pre, errsq);
-          } else {
-            wave_point_store<T, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, sC, sp, c, c * plane + q, kc[c], cen[c]);
-          }
-        }
-      }
+      for (int c = 0; c < 3; c++)
+        wave_point_store<T, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, sC, sp, c, c * plane + q, kc[c], cen[c]);
     }
   }
 }
 
 // The Tile type of the single-instance kernel for (T, order, kind, stage).
 template <typename T, int ORD, int KIND, int STAGE>
-using WaveStageTile = WaveTile<T, ORD, STAGE, wave_ty<T, KIND>(), 0, KIND == WK_VAR && SBP_VAR_COEF != 0,
-                               wave_ring<T, KIND, STAGE>(), wave_warps<T, KIND>(), wave_fixed<T, KIND, STAGE>(),
-                               wave_fixed<T, KIND, STAGE>() ? SBP_FP64_CONV : 0>;
+using WaveStageTile = WaveTile<T, ORD, STAGE, wave_ty<T, KIND>(), 0, wave_coef<T, KIND>(), wave_ring<T, KIND, STAGE>(),
+                               wave_warps<T, KIND, STAGE>(), wave_fixed<T, KIND, STAGE>(),
+                               wave_fixed<T, KIND, STAGE>() ? wave_conv<KIND, STAGE>() : 0>;
 
 // The producer (one lane): takes the CTA's tiles, from the dynamic queue or with a
 // fixed stride, writes each tile's index into its ring stage and issues the stage's
@@ -760,32 +714,18 @@ __global__ void __launch_bounds__(32 * (wave_warps<T, KIND>() + 1), 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   uint64_t* dbar = reinterpret_cast<uint64_t*>(smem + Tile::OFF_DBAR);
-  uint64_t* fxa = reinterpret_cast<uint64_t*>(smem + Tile::OFF_FX);       // fixed: exponent maxima known
-  uint64_t* fxb = fxa + 8;                                                 // fixed: boxes converted
-  int* fxmax = reinterpret_cast<int*>(smem + Tile::OFF_FX + 128);          // fixed: [NST][2] maxima
-  if constexpr (Tile::FIX) {
-    if (prm.fx_sig[0] == 0.0 || prm.fx_sig[1] == 0.0) {  // the host did not set the fixed-point scales
-      if (threadIdx.x == 0) atomicOr(prm.err, ERR_BAD_LAUNCH);
-      return;
-    }
-  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; s++) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], WARPS);
       mbar_init(&dbar[s], WARPS);
-      if constexpr (Tile::FIX) {
-        mbar_init(&fxa[s], WARPS);
-        mbar_init(&fxb[s], WARPS);
-        fxmax[2 * s] = fxmax[2 * s + 1] = 0;
-      }
     }
     fence_barrier_init();
   }
   __syncthreads();
 
   int* tslot = reinterpret_cast<int*>(smem + Tile::OFF_BAR + 192);
-  const bool dyn = prm.sched != nullptr && !is_rkf_stage(STAGE);
+  const bool dyn = prm.sched != nullptr;
 
   if (warp == WARPS) {
     if (lane == 0) wave_produce<Tile>(mapP, mapU, mapV, mapN, mapA, mapC, mapK, prm, smem, full, empty, tslot, dyn);
@@ -793,7 +733,6 @@ __global__ void __launch_bounds__(32 * (wave_warps<T, KIND>() + 1), 1)
   }
 
   // ---------------- consumers: warps 0 .. WARPS-1
-  double errsq = 0.0;  // ST_RKF6: this thread's share of the weighted error sum
   uint32_t dphase = 0;  // parity of each stage's next deferred-pass barrier phase
   for (int k = 0;; k++) {
     const int b = k % NST;
@@ -804,41 +743,11 @@ __global__ void __launch_bounds__(32 * (wave_warps<T, KIND>() + 1), 1)
     const int tile = tslot[b];
     if (tile < 0) break;
     const int i0 = (tile % ntx) * kWaveTX, j0 = (tile / ntx) * TY;
-    if constexpr (Tile::FIX) {
-      int emax[2];
-      bool bad;
-      if (!fx_convert_tile<Tile>(smem + b * Tile::STAGE_BYTES, &fxa[b], &fxb[b], fxmax + 2 * b, (k / NST) & 1,
-                                 prm.wait_ns, threadIdx.x, emax, bad)) {
-        if (lane == 0) atomicOr(prm.err, ERR_TMA_TIMEOUT);
-        break;
-      }
-      const FxGeom g{prm.nx, prm.ny, 0, 0, 0, 0, prm.pitch, prm.plane, 0};
-      wave_tile_fixed<ORD, STAGE, Tile>(prm, g, prm.in, prm.wout, prm.c_acc, prm.c_w, prm.fx_ca, prm.fx_cw,
-                                        smem + b * Tile::STAGE_BYTES, i0, j0, warp, lane, emax[0], emax[1], bad,
-                                        &dbar[b], &dphase, b, k);
-      // the converted boxes were written through the generic proxy; order those writes
-      // before the TMA (async proxy) refills the stage
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    } else {
-      wave_tile_compute<T, ORD, KIND, STAGE, Tile>(prm, prm.in, prm.wout, prm.c_acc, prm.c_w,
-                                                   smem + b * Tile::STAGE_BYTES, i0, j0, warp, lane, &errsq, &dbar[b],
-                                                   &dphase, b, k);
-    }
+    wave_tile_compute<T, ORD, KIND, STAGE, Tile>(prm, prm.in, prm.wout, prm.c_acc, prm.c_w,
+                                                 smem + b * Tile::STAGE_BYTES, i0, j0, warp, lane, &dbar[b], &dphase,
+                                                 b, k);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[b]);
-  }
-  if constexpr (STAGE == ST_RKF6) {
-    // fixed-order sum over the consumer threads -> one partial per CTA
-    __shared__ double warp_sum[WARPS];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) errsq += __shfl_down_sync(0xffffffffu, errsq, off);
-    if (lane == 0) warp_sum[warp] = errsq;
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * WARPS) : "memory");  // consumer warps only
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int q = 0; q < WARPS; q++) s += warp_sum[q];
-      prm.rkpart[blockIdx.x] = s;
-    }
   }
 }
 

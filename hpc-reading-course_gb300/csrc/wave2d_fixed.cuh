@@ -1,5 +1,6 @@
-// wave2d_fixed.cuh -- the FP64 constant-coefficient wave stage (rho = K = 1)
-// with its interior stencils in exact integer arithmetic.
+// wave2d_fixed.cuh -- the FP64 wave stages (constant and variable coefficients, the
+// manufactured solution; RHS, RK4 and Fehlberg stages) with their interior stencils in
+// exact integer arithmetic.
 //
 // GB300 issues FP64 FMAs at about 1/64 of its FP32 rate, and the FP64 tap
 // chains of wave_tile_compute (4 derivatives x 4 taps at order 4, plus the
@@ -13,20 +14,23 @@
 // stencil boxes are converted once, in place, to 64-bit integers in units of
 // 2^(Emax - 1075), where Emax is the largest biased exponent among the box
 // values of the group (p; u and v together): a double +-M 2^(E-1075) with its
-// 53-bit mantissa M becomes +-round(M / 2^(Emax - E)), |V| < 2^53. The sums
+// 53-bit mantissa M becomes +-trunc(M / 2^(Emax - E)), |V| < 2^53. The sums
 // are then exact in int64 (|S| < 110 * 2^54 < 2^61 at order 6, and the sum of
-// the u and v terms as well), and one conversion back to a double, rounded to
-// nearest, carries the only rounding of the stencil: the result is as accurate
-// as the reference's FP64 evaluation (the conversion to fixed point rounds each
-// value to 2^-53 of the box's largest magnitude, the FP64 sum rounds each
-// partial sum to 2^-53 of its own). The integer work runs on the INT pipe; the
+// the u and v terms below 2^62), and one conversion back to a double carries the only
+// other rounding of the stencil: the result is as accurate as the reference's FP64
+// evaluation (the conversion to fixed point cuts each value at 2^-52 of the box's largest
+// magnitude, the FP64 sum rounds each partial sum to 2^-53 of its own). Stages with
+// per-point coefficients and the Fehlberg stages (fx_fine) keep two more bits, units of
+// 2^(Emax - 1077), sums below 2^63, and round the conversion back to nearest: the
+// adaptive integrator's steps follow small differences of the state.
+// The integer work runs on the INT pipe; the
 // FP64 pipe is left with the RK4 stage update, 1-2 FMAs per component, into
 // which the scale sigma = -hi/den is folded (fx_ca, fx_cw).
 //
 // Closure rows (boundary strips) keep the FP64 taps read from global memory
 // and are brought to the same units by 1/sigma; SAT terms are applied in FP64
-// in true units as in wave_tile_compute. A box holding a non-finite value gives
-// NaN for every point of its tile.
+// in true units as in wave_tile_compute. Boxes with values outside the fixed-point range:
+// fx_tile_emax.
 #pragma once
 
 #include "sbp_device.cuh"
@@ -38,30 +42,50 @@ template <> struct FixDen<2> { static constexpr int value = 2; };
 template <> struct FixDen<4> { static constexpr int value = 12; };
 template <> struct FixDen<6> { static constexpr int value = 60; };
 
+// Which stages take the finer unit and round the stencil sums to nearest. The RK4 and
+// RHS stages of constant coefficients do not: it cost them 1.3 % at 4096^2 and 1024^2, and
+// their error against 64-bit arithmetic was the same with and without it.
+template <int KIND, int STAGE> constexpr bool fx_fine() {
+  return is_rkf_stage(STAGE) || KIND == WK_VAR || KIND == WK_MMS;
+}
+
 // v (given as its two 32-bit words) as a signed integer in units of
-// 2^(emax - 1075), truncated towards zero; emax >= the exponent of v. Zero and
-// subnormal values give 0, as does any shift of 64 or more.
+// 2^(emax - 1075), FINE: 2^(emax - 1077), truncated towards zero; emax >= the exponent
+// of v. Zero and subnormal values give 0, as does any shift of 64 or more.
+template <bool FINE>
 __device__ __forceinline__ long long fx_from(unsigned lo, unsigned hi, int emax) {
   const unsigned e = (hi >> 20) & 0x7FFu;
-  const unsigned mh = (hi & 0x000FFFFFu) | 0x00100000u;  // the 53-bit mantissa is mh:lo
+  unsigned mh = (hi & 0x000FFFFFu) | 0x00100000u, ml = lo;  // the 53-bit mantissa is mh:ml
+  if constexpr (FINE) {
+    mh = __funnelshift_l(ml, mh, 2);
+    ml <<= 2;
+  }
   const unsigned sh = e == 0 ? 64u : (unsigned)emax - e;
-  const unsigned rlo = sh < 32 ? __funnelshift_rc(lo, mh, sh) : __funnelshift_rc(mh, 0u, sh - 32u);
+  const unsigned rlo = sh < 32 ? __funnelshift_rc(ml, mh, sh) : __funnelshift_rc(mh, 0u, sh - 32u);
   const unsigned rhi = __funnelshift_rc(mh, 0u, sh);
   const long long r = (long long)(((unsigned long long)rhi << 32) | rlo);
   const long long sg = (long long)((int)hi >> 31);  // 0 or -1
   return (r ^ sg) - sg;
 }
 
-// s * 2^(eb - 11 - 1075) as a double, truncated towards zero (eb = emax + 11 of
-// the box; the tile guard keeps emax in [64, 2030], so the exponent stays normal).
+// The exponent base fx_to takes for integers in fx_from's units.
+template <bool FINE> __device__ __forceinline__ int fx_base(int emax) { return emax + (FINE ? 9 : 11); }
+
+// s in fx_from's units as a double; eb = fx_base(emax), |s| < 2^63 (the tile guard keeps
+// emax in [64, 2030], so the exponent stays normal). FINE: rounded to nearest (ties away
+// from zero; a carry out of the mantissa moves into the exponent field), else truncated
+// towards zero.
+template <bool FINE>
 __device__ __forceinline__ double fx_to(long long s, int eb) {
+  constexpr int TOP = FINE ? 62 : 63;  // the bit the leading one is shifted to
   const long long sg = s >> 63;
   const unsigned long long a = (unsigned long long)((s ^ sg) - sg);
-  const int lz = __clzll((long long)a);                        // >= 2: |s| < 2^62
-  const unsigned long long n = a << (lz & 63);                  // leading one at bit 63
-  const unsigned mh = (unsigned)(n >> 43);                      // leading one + 20 fraction bits
-  const unsigned ml = (unsigned)(n >> 11);                      // the other 32 fraction bits
-  const unsigned hw = (((unsigned)(eb - lz - 1)) << 20) + mh;   // the leading one adds the last 1 to the exponent
+  const int lz = __clzll((long long)a);  // >= 1, without FINE >= 2
+  unsigned long long n = a << ((lz - (63 - TOP)) & 63);
+  if constexpr (FINE) n += 0x200ull;
+  const unsigned mh = (unsigned)(n >> (TOP - 20));             // leading one + 20 fraction bits
+  const unsigned ml = (unsigned)(n >> (TOP - 52));             // the other 32 fraction bits
+  const unsigned hw = (((unsigned)(eb - lz - 1)) << 20) + mh;  // the leading one adds the last 1 to the exponent
   const double r = __hiloint2double((int)(hw | ((unsigned)sg & 0x80000000u)), (int)ml);
   return a == 0 ? 0.0 : r;
 }
@@ -78,84 +102,16 @@ __device__ __forceinline__ long long fx_stencil(const long long* c, int st) {
   }
 }
 
-// Converts the p, u and v boxes of one ring stage to int64 in place (all
-// consumer threads). Each thread keeps its elements in registers between the
-// two barriers, both with bounded waits: the exponent maxima are known (fxa),
-// the boxes are converted (fxb). Returns false if a wait ran out. emax[0..1]
-// are the p and u/v maxima; a box whose maximum is below 64 (values under
-// 2^-959) converts to zeros, and one at 2031 or more (values from 2^1008, Inf,
-// NaN) marks the tile bad: its points get NaN.
-template <typename Tile>
-__device__ __forceinline__ bool fx_convert_tile(unsigned char* st, uint64_t* fxa, uint64_t* fxb, int* fxmax,
-                                                uint32_t parity, unsigned long long wait_ns, int tid, int (&emax)[2],
-                                                bool& bad) {
-  constexpr int NT = 32 * Tile::WARPS;
-  constexpr int NP = Tile::PH * Tile::PW, NU = Tile::TY * Tile::PW, NV = Tile::PH * kWaveTX;
-  constexpr int CP = (NP + NT - 1) / NT, CU = (NU + NT - 1) / NT, CV = (NV + NT - 1) / NT;
-  uint2* wP = reinterpret_cast<uint2*>(st);
-  uint2* wU = reinterpret_cast<uint2*>(st + Tile::OFF_U);
-  uint2* wV = reinterpret_cast<uint2*>(st + Tile::OFF_V);
-  const int lane = tid & 31;
-  uint2 rp[CP], ru[CU], rv[CV];
-  unsigned mp = 0, muv = 0;
+// The interior stencil at the point c of an FP64 line in global memory (scaled taps, the
+// order of the FP64 tap kernels), for tiles whose values leave the fixed-point range.
+template <int ORD>
+__device__ __noinline__ double fx_taps_global(const double* c, long long st, const double (&taps)[7]) {
+  constexpr int W = OpShape<ORD>::W, R = (W - 1) / 2;
+  double s = taps[0] * c[-R * st];
 #pragma unroll
-  for (int c = 0; c < CP; c++) {
-    const int e = tid + c * NT;
-    rp[c] = (c < NP / NT || e < NP) ? wP[e] : make_uint2(0u, 0u);
-    mp = max(mp, rp[c].y & 0x7FF00000u);
-  }
-#pragma unroll
-  for (int c = 0; c < CU; c++) {
-    const int e = tid + c * NT;
-    ru[c] = (c < NU / NT || e < NU) ? wU[e] : make_uint2(0u, 0u);
-    muv = max(muv, ru[c].y & 0x7FF00000u);
-  }
-#pragma unroll
-  for (int c = 0; c < CV; c++) {
-    const int e = tid + c * NT;
-    rv[c] = (c < NV / NT || e < NV) ? wV[e] : make_uint2(0u, 0u);
-    muv = max(muv, rv[c].y & 0x7FF00000u);
-  }
-  mp = __reduce_max_sync(0xffffffffu, mp);
-  muv = __reduce_max_sync(0xffffffffu, muv);
-  if (lane == 0) {
-    atomicMax(&fxmax[0], (int)(mp >> 20));
-    atomicMax(&fxmax[1], (int)(muv >> 20));
-  }
-  __syncwarp();
-  if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(fxa)) : "memory");
-  if (!mbar_wait_bounded(fxa, parity, wait_ns)) return false;
-  int ep = fxmax[0], euv = fxmax[1];
-  bad = ep >= 2031 || euv >= 2031;
-  if (ep < 64) ep = 2111;  // every value converts to 0
-  if (euv < 64) euv = 2111;
-  long long* iP = reinterpret_cast<long long*>(wP);
-  long long* iU = reinterpret_cast<long long*>(wU);
-  long long* iV = reinterpret_cast<long long*>(wV);
-#pragma unroll
-  for (int c = 0; c < CP; c++) {
-    const int e = tid + c * NT;
-    if (c < NP / NT || e < NP) iP[e] = fx_from(rp[c].x, rp[c].y, ep);
-  }
-#pragma unroll
-  for (int c = 0; c < CU; c++) {
-    const int e = tid + c * NT;
-    if (c < NU / NT || e < NU) iU[e] = fx_from(ru[c].x, ru[c].y, euv);
-  }
-#pragma unroll
-  for (int c = 0; c < CV; c++) {
-    const int e = tid + c * NT;
-    if (c < NV / NT || e < NV) iV[e] = fx_from(rv[c].x, rv[c].y, euv);
-  }
-  __syncwarp();
-  if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(fxb)) : "memory");
-  if (!mbar_wait_bounded(fxb, parity, wait_ns)) return false;
-  // every consumer has read the maxima: clear them for the stage's next tile (its
-  // atomics come after this warp's arrivals on the next tile's barriers)
-  if (tid == 0) fxmax[0] = fxmax[1] = 0;
-  emax[0] = ep;
-  emax[1] = euv;
-  return true;
+  for (int k = 1; k < W; k++)
+    if (k != R) s = fma(taps[k], c[(k - R) * st], s);
+  return s;
 }
 
 // Where a tile's points live: the interior extent of the arrays holding them
@@ -433,16 +389,25 @@ __device__ __forceinline__ void decomp_produce(const WaveParams<double>& prm, un
 // the ghost lines the boxes include. `in`, `wout` and the stage's RK4 coefficients
 // (c_acc, c_w in true units, fx_ca / fx_cw scaled per component) come from the
 // caller: the single grid passes prm's, a batch its instance's for the stage.
-// KIND: WK_HOM (rho = K = 1) or WK_CONST (rho = 1, constant K, folded into fx_sigp
-// and the p coefficients; the SAT takes K).
+// KIND: WK_HOM (rho = K = 1); WK_CONST (rho = 1, constant K, folded into fx_sigp
+// and the p coefficients; the SAT takes K); WK_VAR (1/rho and K from the tile's
+// coefficient box multiply the scaled RHS; with prm.ysplit two blocks, each with its own
+// y closures, and the interface SAT on the rows between them); WK_MMS (1/rho and the
+// forcing, the latter in units of sigma and times `ct`, the stage's time factor).
+// The variable kinds exist on a single grid only (no subdomain offsets).
+// Fehlberg stages: u and k_1..k_{S-1} of the point are loaded ahead of the stencil
+// arithmetic; stage 6 adds this thread's error terms to *errsq.
 template <int ORD, int STAGE, typename Tile, int KIND = WK_HOM>
 __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, const FxGeom& g, const double* in0,
                                                 double* wout, const double c_acc, const double c_w,
                                                 const double* fx_ca, const double* fx_cw, const unsigned char* st,
                                                 const int i0, const int j0, const int warp, const int lane,
                                                 const int ep, const int euv, const bool bad, uint64_t* dbar,
-                                                uint32_t* dphase, const int b, const int k) {
-  static_assert(KIND == WK_HOM || KIND == WK_CONST, "fixed-point stencils: constant coefficients");
+                                                uint32_t* dphase, const int b, const int k, const double ct = 0.0,
+                                                double* errsq = nullptr) {
+  constexpr int RKS = is_rkf_stage(STAGE) ? STAGE - ST_RKF1 + 1 : 1;
+  constexpr bool FINE = fx_fine<KIND, STAGE>();
+  constexpr int CW = OpShape<ORD>::CW;
   constexpr int TY = Tile::TY, CS = OpShape<ORD>::CS;
   constexpr int HX = Tile::HX, HY = Tile::HY, PW = Tile::PW;
   constexpr int ROWS = TY / Tile::WARPS;
@@ -455,22 +420,30 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
   const long long* iV = reinterpret_cast<const long long*>(st + Tile::OFF_V);
   const double* sN = reinterpret_cast<const double*>(st + Tile::OFF_N);
   const double* sA = reinterpret_cast<const double*>(st + Tile::OFF_A);
+  const double* sK = reinterpret_cast<const double*>(st + Tile::OFF_K);  // coefficient planes
   double* sD = reinterpret_cast<double*>(const_cast<unsigned char*>(st) + Tile::OFF_DEF);
   // x faces of the global grid inside this tile (their SAT goes to the deferred pass)
   const int iw = -g.xoff, ie = NX - 1 - g.xoff;  // local indices of global columns 0 and NX - 1
   const bool xfaces = dbar != nullptr && prm.bc != BC_NONE &&
                       ((iw >= i0 && iw < i0 + kWaveTX) || (ie >= i0 && ie < i0 + kWaveTX && ie < g.nx));
   const double sg[3] = {prm.fx_sig[0], prm.fx_sig[1], prm.fx_sigp};
-  const int ebp = ep + 11, ebuv = euv + 11;  // fx_to's exponent bases
+  const int ebp = fx_base<FINE>(ep), ebuv = fx_base<FINE>(euv);
   (void)sN;
   (void)sA;
-#pragma unroll
+  (void)sK;
+  // rows that close a block from inside (two-block problems): the interface lines
+  const int ys = KIND == WK_VAR ? prm.ysplit : 0;
+  const auto interface_row = [&](int J) { return KIND == WK_VAR && ys > 0 && (J == ys - 1 || J == ys); };
+#pragma unroll 1
   for (int rr = 0; rr < ROWS; rr++) {
     const int y = warp * ROWS + rr;
     const int j = j0 + y;
     if (j >= g.ny) continue;
     const int J = g.yoff + j;
-    const bool yint = (J >= CS) && (J < NY - CS);
+    // the block's first row and height (one block unless ysplit is set)
+    const int jb0 = (ys > 0 && J >= ys) ? ys : 0;
+    const int nyb = ys > 0 ? (J >= ys ? NY - ys : ys) : NY;
+    const bool yint = (J - jb0 >= CS) && (J - jb0 < nyb - CS);
     const long long rowq = (long long)(j + g.row0) * pitch;
 #pragma unroll
     for (int cc = 0; cc < kWaveTX / 32; cc++) {
@@ -485,35 +458,60 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
       // closure lines start at the global first point of the line (inside the arrays
       // for a subdomain at the physical boundary, which holds a whole closure block)
       const double* xline = in + rowq + g.col0 - g.xoff;
-      const double* yline = in + (long long)(g.row0 - g.yoff) * pitch + (i + g.col0);
+      const double* yline = in + (long long)(g.row0 - g.yoff + jb0) * pitch + (i + g.col0);
+      // Fehlberg stages: u and the earlier derivatives, in flight during the stencil arithmetic
+      double pre[3][RKS];
+      if constexpr (is_rkf_stage(STAGE)) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) wave_rkf_preload<double, RKS>(prm, c * plane + rowq + i + g.col0, pre[c]);
+      }
+      (void)pre;
       // RHS in units of sigma per component: F_u = sx ku, F_v = sy kv, F_p = sx kp
+      // (tiles outside the fixed-point range, finer unit only: FP64 taps for the interior)
+      const bool taps = FINE && bad, xfx = xint && !taps, yfx = yint && !taps;
+      const auto other_x = [&](const double* line) {
+        if (FINE && xint) return fx_taps_global<ORD>(line + I, 1, prm.dx.taps) * prm.fx_isig[0];
+        return closure_line<double, ORD>(line, 1, NX, I, prm.dx.cls) * prm.fx_isig[0];
+      };
+      const auto other_y = [&](const double* line) {
+        if (FINE && yint) return fx_taps_global<ORD>(line + (J - jb0) * pitch, pitch, prm.dy.taps) * prm.fx_isig[1];
+        return closure_line<double, ORD>(line, pitch, nyb, J - jb0, prm.dy.cls) * prm.fx_isig[1];
+      };
       double ku, kv, kp;
-      if (xint) {
-        ku = fx_to(fx_stencil<ORD>(cP, 1), ebp);
+      if (xfx) {
+        ku = fx_to<FINE>(fx_stencil<ORD>(cP, 1), ebp);
       } else {
-        ku = closure_line<double, ORD>(xline + 2 * plane, 1, NX, I, prm.dx.cls) * prm.fx_isig[0];
+        ku = other_x(xline + 2 * plane);
       }
-      if (yint) {
-        kv = fx_to(fx_stencil<ORD>(cP, PW), ebp);
+      if (yfx) {
+        kv = fx_to<FINE>(fx_stencil<ORD>(cP, PW), ebp);
       } else {
-        kv = closure_line<double, ORD>(yline + 2 * plane, pitch, NY, J, prm.dy.cls) * prm.fx_isig[1];
+        kv = other_y(yline + 2 * plane);
       }
-      if (xint && yint && prm.fx_square) {
-        kp = fx_to(fx_stencil<ORD>(cU, 1) + fx_stencil<ORD>(cV, kWaveTX), ebuv);
+      if (xfx && yfx && prm.fx_square) {
+        kp = fx_to<FINE>(fx_stencil<ORD>(cU, 1) + fx_stencil<ORD>(cV, kWaveTX), ebuv);
       } else {
-        const double ax = xint ? fx_to(fx_stencil<ORD>(cU, 1), ebuv)
-                               : closure_line<double, ORD>(xline, 1, NX, I, prm.dx.cls) * prm.fx_isig[0];
-        const double ay = yint ? fx_to(fx_stencil<ORD>(cV, kWaveTX), ebuv)
-                               : closure_line<double, ORD>(yline + plane, pitch, NY, J, prm.dy.cls) * prm.fx_isig[1];
+        const double ax = xfx ? fx_to<FINE>(fx_stencil<ORD>(cU, 1), ebuv) : other_x(xline);
+        const double ay = yfx ? fx_to<FINE>(fx_stencil<ORD>(cV, kWaveTX), ebuv) : other_y(yline + plane);
         kp = fma(prm.fx_rho, ay, ax);
       }
-      if (bad) ku = kv = kp = __longlong_as_double(0x7FF8000000000000ll);
+      if (!FINE && bad) ku = kv = kp = __longlong_as_double(0x7FF8000000000000ll);
 
       const long long q = rowq + i + g.col0;
       const int sp = y * kWaveTX + x;  // point within a 3-component smem box
-      const bool edge = (I == 0) || (J == 0) || (I == NX - 1) || (J == NY - 1);
+      if constexpr (KIND == WK_VAR) {
+        const double ri = sK[sp];
+        ku *= ri;
+        kv *= ri;
+        kp *= sK[TPT + sp];
+      } else if constexpr (KIND == WK_MMS) {
+        const double ri = sK[sp];
+        ku = fma(ct, sK[TPT + sp], ri * ku);
+        kv = fma(ct, sK[2 * TPT + sp], ri * kv);
+      }
+      const bool edge = (I == 0) || (J == 0) || (I == NX - 1) || (J == NY - 1) || interface_row(J);
       if (prm.bc != BC_NONE && edge) {
-        if (xfaces && J != 0 && J != NY - 1) {
+        if (xfaces && J != 0 && J != NY - 1 && !interface_row(J)) {
           double* d = sD + ((I == 0 ? 0 : TY) + y) * 3;  // an x-face point only: deferred
           d[0] = ku;
           d[1] = kv;
@@ -527,9 +525,13 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
         const double kt[3] = {r.u, r.v, r.p};
 #pragma unroll
         for (int c = 0; c < 3; c++) {
-          const double cen = (STAGE == ST_FIRST) ? sN[c * TPT + sp] : 0.0;
-          wave_point_store<double, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, nullptr, sp, c,
-                                                g.base + c * plane + q, kt[c], cen);
+          if constexpr (is_rkf_stage(STAGE)) {
+            wave_point_rkf<double, STAGE, RKS>(prm, wout, c * plane + q, kt[c], pre[c], errsq);
+          } else {
+            const double cen = (STAGE == ST_FIRST) ? sN[c * TPT + sp] : 0.0;
+            wave_point_store<double, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, nullptr, sp, c,
+                                                  g.base + c * plane + q, kt[c], cen);
+          }
         }
         continue;
       }
@@ -539,6 +541,8 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
         const long long o = g.base + c * plane + q;
         if constexpr (STAGE == ST_RHS) {
           prm.kout[o] = sg[c] * kf[c];
+        } else if constexpr (is_rkf_stage(STAGE)) {
+          wave_point_rkf<double, STAGE, RKS>(prm, wout, o, sg[c] * kf[c], pre[c], errsq);
         } else {
           const double cen = (STAGE == ST_FIRST) ? sN[c * TPT + sp] : 0.0;
           wave_point_store<double, STAGE, Tile>(prm, wout, fx_ca[c], fx_cw[c], sA, sN, nullptr, sp, c, o,
@@ -560,7 +564,7 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
     for (int e = lane; e < 2 * TY; e += 32) {
       const int side = e / TY, y = e - side * TY, j = j0 + y;
       const int I = side == 0 ? 0 : NX - 1, i = I - g.xoff, J = g.yoff + j;
-      if (i < i0 || i >= i0 + kWaveTX || i >= g.nx || j >= g.ny || J == 0 || J == NY - 1) continue;
+      if (i < i0 || i >= i0 + kWaveTX || i >= g.nx || j >= g.ny || J == 0 || J == NY - 1 || interface_row(J)) continue;
       const int x = i - i0;
       const long long q = (long long)(j + g.row0) * pitch + i + g.col0;
       const double pc = in[2 * plane + q], uc = in[q], vc = in[plane + q];
@@ -571,9 +575,15 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
       const int sp = y * kWaveTX + x;
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        const double cen = (STAGE == ST_FIRST) ? sN[c * TPT + sp] : 0.0;
-        wave_point_store<double, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, nullptr, sp, c,
-                                              g.base + c * plane + q, kt[c], cen);
+        if constexpr (is_rkf_stage(STAGE)) {
+          double pre[RKS];
+          wave_rkf_preload<double, RKS>(prm, c * plane + q, pre);
+          wave_point_rkf<double, STAGE, RKS>(prm, wout, c * plane + q, kt[c], pre, errsq);
+        } else {
+          const double cen = (STAGE == ST_FIRST) ? sN[c * TPT + sp] : 0.0;
+          wave_point_store<double, STAGE, Tile>(prm, wout, c_acc, c_w, sA, sN, nullptr, sp, c,
+                                                g.base + c * plane + q, kt[c], cen);
+        }
       }
     }
   }
@@ -585,15 +595,17 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
 // warp writes its own p and u/v maxima to wmax[warp][0..1], every converter then
 // takes the maximum over them, and so does every compute warp later (fx_tile_emax),
 // so nothing has to be reset between tiles. Returns false if the wait ran out.
-template <typename Tile>
+template <typename Tile, bool FINE>
 __device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fxa, int* wmax, uint32_t parity,
                                                  unsigned long long wait_ns, int t);
 
 // The p and u/v exponent maxima of a converted stage from its converter warps'
 // pairs, with the tile guard applied: a box whose maximum is below 64 (values
 // under 2^-959) converts to zeros, and one at 2031 or more (values from 2^1008,
-// Inf, NaN) marks the tile bad.
-template <int CONV>
+// Inf, NaN) marks the tile bad. A bad tile is NaN throughout in the stages that do
+// not take the finer unit; those that do evaluate it with FP64 taps from global memory,
+// and tiles whose largest value is nonzero but below 2^-959 as well.
+template <int CONV, bool FINE>
 __device__ __forceinline__ void fx_tile_emax(const int* wmax, int& ep, int& euv, bool& bad) {
   ep = 0;
   euv = 0;
@@ -603,11 +615,12 @@ __device__ __forceinline__ void fx_tile_emax(const int* wmax, int& ep, int& euv,
     euv = max(euv, wmax[2 * c + 1]);
   }
   bad = ep >= 2031 || euv >= 2031;
+  if (FINE) bad = bad || (ep > 0 && ep < 64) || (euv > 0 && euv < 64);
   if (ep < 64) ep = 2111;  // every value converts to 0
   if (euv < 64) euv = 2111;
 }
 
-template <typename Tile>
+template <typename Tile, bool FINE>
 __device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fxa, int* wmax, uint32_t parity,
                                                  unsigned long long wait_ns, int t) {
   constexpr int NT = 32 * Tile::CONV;
@@ -631,7 +644,7 @@ __device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fx
   if (!mbar_wait_bounded(fxa, parity, wait_ns)) return false;
   int ep, euv;
   bool bad;
-  fx_tile_emax<Tile::CONV>(wmax, ep, euv, bad);
+  fx_tile_emax<Tile::CONV, FINE>(wmax, ep, euv, bad);
   (void)bad;
   long long* iP = reinterpret_cast<long long*>(wP);
   long long* iU = reinterpret_cast<long long*>(wU);
@@ -639,17 +652,17 @@ __device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fx
 #pragma unroll 4
   for (int e = t; e < NP; e += NT) {
     const uint2 w = wP[e];
-    iP[e] = fx_from(w.x, w.y, ep);
+    iP[e] = fx_from<FINE>(w.x, w.y, ep);
   }
 #pragma unroll 4
   for (int e = t; e < NU; e += NT) {
     const uint2 w = wU[e];
-    iU[e] = fx_from(w.x, w.y, euv);
+    iU[e] = fx_from<FINE>(w.x, w.y, euv);
   }
 #pragma unroll 4
   for (int e = t; e < NV; e += NT) {
     const uint2 w = wV[e];
-    iV[e] = fx_from(w.x, w.y, euv);
+    iV[e] = fx_from<FINE>(w.x, w.y, euv);
   }
   // the converted boxes were written through the generic proxy; order those writes
   // before the TMA (async proxy) refills the stage
@@ -666,13 +679,14 @@ __device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fx
 // compute warps meet no barrier but the deferred x-face pass. Every wait is
 // bounded (prm.wait_ns); a wait that runs out sets the error word and the warp
 // stops, so the others' waits run out in turn.
-template <int ORD, int STAGE, bool DEC = false>
-__global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, WK_HOM, STAGE>, DEC>(), 1)
+template <int ORD, int STAGE, bool DEC = false, int KIND = WK_HOM>
+__global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, KIND, STAGE>, DEC>(), 1)
     wave_fixed_kernel(const __grid_constant__ CUtensorMap mapP, const __grid_constant__ CUtensorMap mapU,
                       const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapN,
                       const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapC,
                       const __grid_constant__ CUtensorMap mapK, const __grid_constant__ WaveParams<double> prm) {
-  using Tile = WaveStageTile<double, ORD, WK_HOM, STAGE>;
+  using Tile = WaveStageTile<double, ORD, KIND, STAGE>;
+  static_assert(KIND == WK_HOM || !DEC, "decomposed grids: rho = K = 1");
   constexpr int TY = Tile::TY, NST = Tile::NST, WARPS = Tile::WARPS, CONV = Tile::CONV;
   static_assert(CONV >= 1, "the converter-warp kernel needs converter warps");
   extern __shared__ __align__(128) unsigned char smem[];
@@ -705,6 +719,13 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, W
     }
     fence_barrier_init();
   }
+  __shared__ double s_ct;  // WK_MMS: the forcing's time factor, one cosine per CTA at most
+  if constexpr (KIND == WK_MMS) {
+    if (threadIdx.x == 32)
+      s_ct = prm.tctl ? cos(5 * 3.14159265358979323846264 *
+                            __dadd_rn(prm.tctl[0], __dmul_rn(prm.tc, prm.tctl[1])))
+                      : (prm.ctp ? *prm.ctp : prm.ct);
+  }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntx = (prm.nx + kWaveTX - 1) / kWaveTX;
@@ -734,7 +755,7 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, W
         break;
       }
       const int tile = tslot[b];
-      if (tile >= 0 && !fx_convert_stage<Tile>(smem + b * Tile::STAGE_BYTES, &fxa[b], wmax + 16 * b, (k / NST) & 1,
+      if (tile >= 0 && !fx_convert_stage<Tile, fx_fine<KIND, STAGE>()>(smem + b * Tile::STAGE_BYTES, &fxa[b], wmax + 16 * b, (k / NST) & 1,
                                                 prm.wait_ns, t)) {
         if (lane == 0) atomicOr(prm.err, ERR_TMA_TIMEOUT);
         break;
@@ -747,6 +768,8 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, W
   }
   // ---------------- compute warps
   uint32_t dphase = 0;  // parity of each stage's next deferred-pass barrier phase
+  double errsq = 0.0;   // ST_RKF6: this thread's share of the weighted error sum
+  const double ct = KIND == WK_MMS ? s_ct : 0.0;
   for (int k = 0;; k++) {
     const int b = k % NST;
     if (!mbar_wait_bounded(&conv[b], (k / NST) & 1, prm.wait_ns)) {
@@ -769,12 +792,25 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, W
     }
     int ep, euv;
     bool bad;
-    fx_tile_emax<CONV>(wmax + 16 * b, ep, euv, bad);
-    wave_tile_fixed<ORD, STAGE, Tile>(prm, g, prm.in, prm.wout, prm.c_acc, prm.c_w, prm.fx_ca, prm.fx_cw,
-                                      smem + b * Tile::STAGE_BYTES, i0, j0, warp, lane, ep, euv, bad, &dbar[b], &dphase,
-                                      b, k);
+    fx_tile_emax<CONV, fx_fine<KIND, STAGE>()>(wmax + 16 * b, ep, euv, bad);
+    wave_tile_fixed<ORD, STAGE, Tile, KIND>(prm, g, prm.in, prm.wout, prm.c_acc, prm.c_w, prm.fx_ca, prm.fx_cw,
+                                            smem + b * Tile::STAGE_BYTES, i0, j0, warp, lane, ep, euv, bad, &dbar[b],
+                                            &dphase, b, k, ct, &errsq);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[b]);
+  }
+  if constexpr (STAGE == ST_RKF6) {
+    // fixed-order sum over the compute threads -> one partial per CTA
+    __shared__ double warp_sum[WARPS];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) errsq += __shfl_down_sync(0xffffffffu, errsq, off);
+    if (lane == 0) warp_sum[warp] = errsq;
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * WARPS) : "memory");  // compute warps only
+    if (threadIdx.x == 0) {
+      double s = 0.0;
+      for (int q = 0; q < WARPS; q++) s += warp_sum[q];
+      prm.rkpart[blockIdx.x] = s;
+    }
   }
 }
 

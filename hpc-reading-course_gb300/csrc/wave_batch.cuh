@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(BatchWaveTile<T, ORD, STAGE, CFG>::THREADS, ba
     T* wout;
     T c_acc, c_w;
     batch_stage_buffers(I, rk, in, wout, c_acc, c_w);
-    wave_tile_compute<T, ORD, WK_CONST, STAGE, Tile>(I.prm, in, wout, c_acc, c_w, st, i0, j0, warp, lane, nullptr,
+    wave_tile_compute<T, ORD, WK_CONST, STAGE, Tile>(I.prm, in, wout, c_acc, c_w, st, i0, j0, warp, lane,
                                                      &dbar[b], &dphase, b, k);
     __syncwarp();
     if (lane == 0) mbar_arrive(&empty[b]);
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(BatchWaveTile<double, ORD, STAGE, CFG>::THREAD
       }
       const int tile = tslot[b];
       if (tile >= 0 &&
-          !fx_convert_stage<Tile>(smem + b * Tile::STAGE_BYTES, &fxa[b], wmax + 16 * b, (k / NST) & 1, 0, t)) {
+          !fx_convert_stage<Tile, fx_fine<WK_CONST, STAGE>()>(smem + b * Tile::STAGE_BYTES, &fxa[b], wmax + 16 * b, (k / NST) & 1, 0, t)) {
         if (lane == 0) atomicOr(err, ERR_TMA_TIMEOUT);
         break;
       }
@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(BatchWaveTile<double, ORD, STAGE, CFG>::THREAD
     batch_stage_buffers(I, rk, in, wout, c_acc, c_w);
     int ep, euv;
     bool bad;
-    fx_tile_emax<CONV>(wmax + 16 * b, ep, euv, bad);
+    fx_tile_emax<CONV, false>(wmax + 16 * b, ep, euv, bad);
     const FxGeom g{I.prm.nx, I.prm.ny, 0, 0, 0, 0, I.prm.pitch, I.prm.plane, 0};
     wave_tile_fixed<ORD, STAGE, Tile, WK_CONST>(I.prm, g, in, wout, c_acc, c_w, I.fxa[rk - 1], I.fxw[rk - 1], st, o0.x,
                                                 o0.y, warp, lane, ep, euv, bad, &dbar[b], &dphase, b, k);
