@@ -6,12 +6,33 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <utility>
+
 #include "line_kernels.cuh"
 #include "wave2d.cuh"
+#include "wave_cell.cuh"
 #include "wave3d.cuh"
 #include "wave_batch.cuh"
 
 namespace sbp {
+
+// Launches a kernel that waits for its predecessors itself (grid_dependency_wait): it may
+// start while the last CTAs of the kernel before it run.
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                     A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 struct WaveMaps {
   CUtensorMap p, u, v;  // the stage input seen with the p, u and v tile boxes (with halos)
@@ -82,6 +103,24 @@ inline cudaError_t launch_wave(int order, int kind, int stage, const WaveMaps& m
     case 6: return launch_wave_o6<T>(kind, stage, m, prm, grid, s);
     default: return cudaErrorInvalidValue;
   }
+}
+
+// The cell form of a stage (wave_cell.cuh); aos: ST_RHS on AoS FP64 arrays.
+template <typename T> cudaError_t launch_cell_o2(int kind, int stage, bool aos, const WaveParams<T>& prm, cudaStream_t s);
+template <typename T> cudaError_t launch_cell_o4(int kind, int stage, bool aos, const WaveParams<T>& prm, cudaStream_t s);
+template <typename T> cudaError_t launch_cell_o6(int kind, int stage, bool aos, const WaveParams<T>& prm, cudaStream_t s);
+template <typename T>
+inline cudaError_t launch_cell(int order, int kind, int stage, bool aos, const WaveParams<T>& prm, cudaStream_t s) {
+  switch (order) {
+    case 2: return launch_cell_o2<T>(kind, stage, aos, prm, s);
+    case 4: return launch_cell_o4<T>(kind, stage, aos, prm, s);
+    case 6: return launch_cell_o6<T>(kind, stage, aos, prm, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+// The CTAs a grid takes.
+inline dim3 cell_grid(long long nx, long long ny) {
+  return dim3((unsigned)((nx + kCellTX - 1) / kCellTX), (unsigned)((ny + kCellTY - 1) / kCellTY));
 }
 
 // Shared memory bytes of one wave tile (for occupancy reports).

@@ -113,6 +113,14 @@ __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
+// Programmatic stream serialization: lets the next kernel of the stream start its prologue
+// while this one runs, and waits for the kernels before this one (all their memory
+// operations visible). Both do nothing in a kernel launched without the attribute.
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // Streaming loads/stores for values touched once per stage.
 template <typename T> __device__ __forceinline__ T ld_stream(const T* p) { return __ldcs(p); }
 template <typename T> __device__ __forceinline__ void st_stream(T* p, T v) { __stcs(p, v); }

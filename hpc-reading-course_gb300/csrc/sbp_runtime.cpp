@@ -71,12 +71,13 @@ struct sbp_ctx {
   void *va = nullptr, *vb = nullptr;         // advection with velocity fields: T planes (pitched)
   double *va64 = nullptr, *vb64 = nullptr;   // the same in FP64, nx*ny row-major (SAT)
   double *rho64 = nullptr, *k64 = nullptr;   // WAVE_VAR: nx*ny FP64
-  int* err = nullptr;
+  int* err = nullptr;  // error word in page-locked host memory the kernels reach: no copy to read it
   int* sched = nullptr;  // the wave stage kernels' dynamic tile queue (2 ints, zero between launches)
   WaveMaps maps_un{}, maps_wa{}, maps_wb{};
   // adaptive RK45 (FP64; allocated on first use)
   double* rk_k[6] = {};
   double* rk_unew = nullptr;
+  double* rk_partial = nullptr;  // error partial sums: one per CTA of the last Fehlberg stage, or kReduceBlocks
   Rk45Ctrl* rk_ctrl = nullptr;
   double rk_atol = 0, rk_rtol = 0;  // tolerances baked into the fused wave stages
   cudaGraphExec_t rk_graph = nullptr;
@@ -117,6 +118,22 @@ void fill_taps(DirTaps<T>& t, int order, double scale) {
 int wave_kind(const sbp_ctx* ctx) {
   if (ctx->d.problem == SBP_WAVE_HOM_2D) return WK_HOM;
   return has_fields(ctx->d.problem) ? WK_VAR : WK_MMS;
+}
+
+// Whether a stage of a 2D wave context runs in its cell form (wave_cell.cuh) rather than
+// the persistent one. The cell form's short CTAs win until a grid gives every SM enough
+// tiles to fill the persistent pipeline. Measured, us per RK4 stage at order 4, cell /
+// persistent:
+//                    129^2       513^2        769^2        1025^2       1281^2       1537^2
+//   FP64 rho=K=1   6.3 / 11.5  10.3 / 18.2  17.1 / 22.4  27.6 / 30.3  42.6 / 41.4  58.2 / 54.0
+//   FP64 var.      7.8 / 13.2  13.1 / 21.1  21.8 / 27.5  37.8 / 39.8  55.7 / 55.5  76.7 / 72.4
+//   FP64 forced    7.3 / 11.9  12.6 / 19.3  21.0 / 27.3  36.1 / 39.9  52.6 / 55.4  72.0 / 72.7
+//   FP32 rho=K=1   4.7 / 7.9    6.5 / 10.4  10.2 / 13.4  15.2 / 15.8  23.0 / 20.6  36.0 / 28.6
+//   FP32 var.      5.7 / 8.6    7.7 / 12.8  12.1 / 15.1  18.6 / 19.5  30.7 / 26.0  46.2 / 37.5
+// (Fehlberg stages at 1024^2: 0.2 ms per attempt in either form.)
+bool use_cell(const sbp_ctx* ctx) {
+  const bool early = ctx->fp32 || wave_kind(ctx) == WK_HOM;
+  return ctx->npts <= (early ? 1150000 : 1600000);
 }
 
 // Encodes one 3D tensor map (x, y, component) over a state buffer of the context.
@@ -280,7 +297,10 @@ int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in,
       p.skip = &ctl->done;
     }
     if (!bc_on) p.bc = BC_NONE;
-    CK(launch_wave<T>(ctx->d.order, wave_kind(ctx), stage, *in_maps, p, ctx->stream));
+    if (p.test_drop_tile == 0 && use_cell(ctx))
+      CK(launch_cell<T>(ctx->d.order, wave_kind(ctx), stage, false, p, ctx->stream));
+    else
+      CK(launch_wave<T>(ctx->d.order, wave_kind(ctx), stage, *in_maps, p, ctx->stream));
   } else if (ctx->three_d) {
     Wave3Params<T> p;
     std::memset(&p, 0, sizeof(p));
@@ -430,12 +450,10 @@ int rk4_resident_t(sbp_ctx* ctx, double t0, double dt, long long nsteps) {
 }
 
 int check_device_errors(sbp_ctx* ctx) {
-  int h = 0;
-  CK(cudaMemcpyAsync(&h, ctx->err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  const int h = *static_cast<volatile int*>(ctx->err);
   if (h) {
-    cudaMemsetAsync(ctx->err, 0, sizeof(int), ctx->stream);
-    cudaStreamSynchronize(ctx->stream);
+    *static_cast<volatile int*>(ctx->err) = 0;
     return fail(ctx, SBP_ERR_DEVICE, (h & ERR_TMA_TIMEOUT) ? "a TMA tile wait timed out in a stage kernel"
                                                            : "a kernel reported an error");
   }
@@ -483,12 +501,41 @@ int unpack_to(sbp_ctx* ctx, const void* soa, double* dst, int where) {
   return SBP_OK;
 }
 
+// RHS of a 2D wave problem from and to AoS FP64 device arrays, which must not overlap.
+template <typename T>
+int launch_rhs_aos(sbp_ctx* ctx, double t, const double* src, double* dst, int bc_on) {
+  WaveParams<T> p = wave_params<T>(ctx);
+  p.aos_in = src;
+  p.aos_out = dst;
+  if (ctx->time_dependent) p.ct = mms_time_factor(t);
+  if constexpr (sizeof(T) == 8) set_fixed_scales(p, ctx->d.order, ctx->hix, ctx->hiy);
+  if (!bc_on) p.bc = BC_NONE;
+  CK(launch_cell<T>(ctx->d.order, wave_kind(ctx), ST_RHS, true, p, ctx->stream));
+  ctx->launches++;
+  return SBP_OK;
+}
+
+// Where the RHS of device arrays runs on the AoS arrays themselves: the 2D wave problems
+// (order 4, us per call, AoS / planes with the conversions: FP64 257^2 26 / 29, 1025^2 41 / 76,
+// 4097^2 400 / 614; FP32 40 / 58 and 300 / 462 at the latter two),
+// unless the arrays overlap (the cells read neighbours' points), a tile is to be dropped
+// (the test aid lives in the persistent kernels) or the problem has two blocks (the
+// interface SAT reads the other block's line from the planes).
+bool rhs_takes_aos(const sbp_ctx* ctx, const double* src, const double* dst, int where) {
+  const double *se = src + ctx->nscalar, *de = dst + ctx->nscalar;
+  return where == SBP_DEVICE && ctx->wave && !ctx->ysplit && !ctx->drop_tile && (se <= dst || de <= src);
+}
+
 int rhs_impl(sbp_ctx* ctx, double t, const double* src, double* dst, int where, int bc_on) {
   if (!ctx) return SBP_ERR_INVALID;
   CK(cudaSetDevice(ctx->d.device));
   const double* dev = nullptr;
   int rc;
   if ((rc = stage_in(ctx, src, where, &dev))) return rc;
+  if (dst && rhs_takes_aos(ctx, src, dst, where)) {
+    rc = ctx->fp32 ? launch_rhs_aos<float>(ctx, t, src, dst, bc_on) : launch_rhs_aos<double>(ctx, t, src, dst, bc_on);
+    return rc ? rc : check_device_errors(ctx);
+  }
   if ((rc = pack_into(ctx, dev, ctx->wa))) return rc;
   if (ctx->fp32)
     rc = launch_stage<float>(ctx, ST_RHS, 0, t, 0.0, ctx->wa, &ctx->maps_wa, ctx->wb, bc_on);
@@ -512,8 +559,21 @@ Rk45Buffers rk45_buffers(sbp_ctx* ctx) {
   b.w = (double*)ctx->wa;
   for (int s = 0; s < 6; s++) b.k[s] = ctx->rk_k[s];
   b.unew = ctx->rk_unew;
-  b.partial = ctx->partial;
+  b.partial = ctx->rk_partial;
   return b;
+}
+
+// CTAs of the last Fehlberg stage of a 2D wave problem (as launch_cell and launch_wave
+// size their grids).
+int wave_grid(const sbp_ctx* ctx) {
+  if (use_cell(ctx)) {
+    const dim3 g = cell_grid(ctx->nx, ctx->ny);
+    return (int)(g.x * g.y);
+  }
+  const int ty = wave_tile_height(8, wave_kind(ctx));
+  const long long ntiles = ((ctx->nx + kWaveTX - 1) / kWaveTX) * ((ctx->ny + ty - 1) / ty);
+  const int nsm = device_sm_count();
+  return (int)(ntiles < nsm ? ntiles : nsm);
 }
 
 int rk45_prepare(sbp_ctx* ctx) {
@@ -522,6 +582,8 @@ int rk45_prepare(sbp_ctx* ctx) {
   for (int s = 0; s < 6; s++) CK(cudaMalloc((void**)&ctx->rk_k[s], bytes));
   CK(cudaMalloc((void**)&ctx->rk_unew, bytes));
   CK(cudaMemsetAsync(ctx->rk_unew, 0, bytes, ctx->stream));  // row padding stays zero
+  const int parts = ctx->wave ? wave_grid(ctx) : 0;
+  CK(cudaMalloc((void**)&ctx->rk_partial, sizeof(double) * (parts > kReduceBlocks ? parts : kReduceBlocks)));
   CK(cudaMalloc((void**)&ctx->rk_ctrl, sizeof(Rk45Ctrl)));
   return SBP_OK;
 }
@@ -544,22 +606,17 @@ int launch_rkf_wave_stage(sbp_ctx* ctx, int s, void* in, const WaveMaps* in_maps
   for (int j = 0; j < 6; j++) p.rkk[j] = ctx->rk_k[j];
   p.rku = (const double*)ctx->un;
   p.rkunew = ctx->rk_unew;
-  p.rkpart = ctx->partial;
+  p.rkpart = ctx->rk_partial;
   p.rkatol = ctx->rk_atol;
   p.rkrtol = ctx->rk_rtol;
   p.wait_ns = ctx->wait_ns;
   set_fixed_scales(p, ctx->d.order, ctx->hix, ctx->hiy);
-  CK(launch_wave<double>(ctx->d.order, wave_kind(ctx), ST_RKF1 + s - 1, *in_maps, p, ctx->stream));
+  if (use_cell(ctx))
+    CK(launch_cell<double>(ctx->d.order, wave_kind(ctx), ST_RKF1 + s - 1, false, p, ctx->stream));
+  else
+    CK(launch_wave<double>(ctx->d.order, wave_kind(ctx), ST_RKF1 + s - 1, *in_maps, p, ctx->stream));
   ctx->launches++;
   return SBP_OK;
-}
-
-// CTAs of the persistent wave kernel (as launch_wave sizes its grid).
-int wave_grid(const sbp_ctx* ctx) {
-  const int ty = wave_tile_height(8, wave_kind(ctx));
-  const long long ntiles = ((ctx->nx + kWaveTX - 1) / kWaveTX) * ((ctx->ny + ty - 1) / ty);
-  const int nsm = device_sm_count();
-  return (int)(ntiles < nsm ? ntiles : nsm);
 }
 
 // One attempted step: six RHS evaluations with the stage combinations between
@@ -645,12 +702,14 @@ void release(sbp_ctx* ctx) {
   for (int s = 0; s < 6; s++)
     if (ctx->rk_k[s]) cudaFree(ctx->rk_k[s]);
   if (ctx->rk_unew) cudaFree(ctx->rk_unew);
+  if (ctx->rk_partial) cudaFree(ctx->rk_partial);
   if (ctx->rk_ctrl) cudaFree(ctx->rk_ctrl);
   void* bufs[] = {ctx->un, ctx->acc, ctx->wa, ctx->wb, ctx->comp, ctx->io, ctx->partial, ctx->red,
-                  ctx->rinv, ctx->rho64, ctx->k64, ctx->err, ctx->sched, ctx->va, ctx->va64, ctx->ct_tab};
+                  ctx->rinv, ctx->rho64, ctx->k64, ctx->sched, ctx->va, ctx->va64, ctx->ct_tab};
   // kmod lives inside the rinv allocation, vb and vb64 inside those of va and va64
   for (void* b : bufs)
     if (b) cudaFree(b);
+  if (ctx->err) cudaFreeHost(ctx->err);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
 }
 
@@ -751,8 +810,9 @@ int sbp_create(const sbp_desc* desc, sbp_ctx** out) {
   if ((e = cudaMalloc((void**)&ctx->partial, 2 * kReduceBlocks * sizeof(double))) != cudaSuccess)
     return cuda_fail("cudaMalloc(partial)", e);
   if ((e = cudaMalloc((void**)&ctx->red, 4 * sizeof(double))) != cudaSuccess) return cuda_fail("cudaMalloc(red)", e);
-  if ((e = cudaMalloc((void**)&ctx->err, sizeof(int))) != cudaSuccess) return cuda_fail("cudaMalloc(err)", e);
-  cudaMemset(ctx->err, 0, sizeof(int));
+  if ((e = cudaHostAlloc((void**)&ctx->err, sizeof(int), cudaHostAllocMapped)) != cudaSuccess)
+    return cuda_fail("cudaHostAlloc(err)", e);
+  *ctx->err = 0;
   if ((e = cudaMalloc((void**)&ctx->sched, 2 * sizeof(int))) != cudaSuccess) return cuda_fail("cudaMalloc(sched)", e);
   cudaMemset(ctx->sched, 0, 2 * sizeof(int));
 

@@ -59,6 +59,8 @@ template <typename T> struct WaveParams {
   T* acc;             // RK4 accumulator (3 planes)
   T* wout;            // next stage input (3 planes)
   T* kout;            // ST_RHS output (3 planes)
+  const double* aos_in;  // ST_RHS on AoS FP64 arrays (wave_cell_kernel): source and destination
+  double* aos_out;
   T* comp;            // FP32: compensation term of the summed update (3 planes)
   const T* rinv;      // WK_VAR: 1/rho (1 plane)
   const T* kmod;      // WK_VAR: K (1 plane)
@@ -704,7 +706,6 @@ __global__ void __launch_bounds__(32 * (wave_warps<T, KIND>() + 1), 1)
   using Tile = WaveStageTile<T, ORD, KIND, STAGE>;
   constexpr int TY = Tile::TY, HX = Tile::HX, HY = Tile::HY, NST = Tile::NST, WARPS = Tile::WARPS;
   extern __shared__ __align__(128) unsigned char smem[];
-  if (prm.skip && *prm.skip) return;  // uniform over the grid: set before this launch
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + Tile::OFF_BAR);
   uint64_t* empty = full + NST;
 

@@ -694,7 +694,7 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, K
     if (threadIdx.x == 0) atomicOr(prm.err, ERR_BAD_LAUNCH);
     return;
   }
-  if (prm.skip && *prm.skip) return;
+  if (prm.skip && *prm.skip) return;  // uniform over the grid: set before this launch
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + Tile::OFF_BAR);
   uint64_t* empty = full + NST;
   uint64_t* dbar = reinterpret_cast<uint64_t*>(smem + Tile::OFF_DBAR);

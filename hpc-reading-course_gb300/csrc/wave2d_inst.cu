@@ -11,6 +11,7 @@
 #define CAT(a, b) CAT_(a, b)
 #define LAUNCH_WAVE CAT(launch_wave_o, SBP_ORDER)
 #define CONFIGURE_WAVE CAT(configure_wave_o, SBP_ORDER)
+#define LAUNCH_CELL CAT(launch_cell_o, SBP_ORDER)
 
 namespace sbp {
 
@@ -52,7 +53,8 @@ template <typename T, int KIND, int STAGE>
 cudaError_t launch_one(const WaveMaps& m, const WaveParams<T>& prm, dim3 grid, cudaStream_t s) {
   using Tile = WaveStageTile<T, SBP_ORDER, KIND, STAGE>;
   if constexpr (wave_fixed<T, KIND, STAGE>())
-    wave_fixed_kernel<SBP_ORDER, STAGE, false, KIND><<<grid, Tile::THREADS, Tile::SMEM, s>>>(m.p, m.u, m.v, m.n, m.a, m.c, m.k, prm);
+    wave_fixed_kernel<SBP_ORDER, STAGE, false, KIND><<<grid, Tile::THREADS, Tile::SMEM, s>>>(m.p, m.u, m.v, m.n, m.a,
+                                                                                            m.c, m.k, prm);
   else
     wave_stage_kernel<T, SBP_ORDER, KIND, STAGE>
         <<<grid, Tile::THREADS, Tile::SMEM, s>>>(m.p, m.u, m.v, m.n, m.a, m.c, m.k, prm);
@@ -82,7 +84,56 @@ cudaError_t launch_kind(int stage, const WaveMaps& m, const WaveParams<T>& prm, 
   return cudaErrorInvalidValue;
 }
 
+template <typename T, int KIND, int STAGE, bool AOS = false>
+cudaError_t cell_one(const WaveParams<T>& prm, cudaStream_t s) {
+  return launch_overlapped(wave_cell_kernel<T, SBP_ORDER, KIND, STAGE, AOS>,
+                           cell_grid(prm.nx, prm.ny), kCellThreads, 0, s, prm);
+}
+
+template <typename T, int KIND>
+cudaError_t cell_kind(int stage, bool aos, const WaveParams<T>& prm, cudaStream_t s) {
+  if (aos) return stage == ST_RHS ? cell_one<T, KIND, ST_RHS, true>(prm, s) : cudaErrorInvalidValue;
+  switch (stage) {
+    case ST_RHS: return cell_one<T, KIND, ST_RHS>(prm, s);
+    case ST_FIRST: return cell_one<T, KIND, ST_FIRST>(prm, s);
+    case ST_MID: return cell_one<T, KIND, ST_MID>(prm, s);
+    case ST_LAST: return cell_one<T, KIND, ST_LAST>(prm, s);
+    default: break;
+  }
+  if constexpr (sizeof(T) == 8) {
+    switch (stage) {
+      case ST_RKF1: return cell_one<T, KIND, ST_RKF1>(prm, s);
+      case ST_RKF1 + 1: return cell_one<T, KIND, ST_RKF1 + 1>(prm, s);
+      case ST_RKF1 + 2: return cell_one<T, KIND, ST_RKF1 + 2>(prm, s);
+      case ST_RKF1 + 3: return cell_one<T, KIND, ST_RKF1 + 3>(prm, s);
+      case ST_RKF1 + 4: return cell_one<T, KIND, ST_RKF1 + 4>(prm, s);
+      case ST_RKF6: return cell_one<T, KIND, ST_RKF6>(prm, s);
+      default: break;
+    }
+  }
+  return cudaErrorInvalidValue;
+}
+
 }  // namespace
+
+template <>
+cudaError_t LAUNCH_CELL<double>(int kind, int stage, bool aos, const WaveParams<double>& prm, cudaStream_t s) {
+  switch (kind) {
+    case WK_HOM: return cell_kind<double, WK_HOM>(stage, aos, prm, s);
+    case WK_VAR: return cell_kind<double, WK_VAR>(stage, aos, prm, s);
+    case WK_MMS: return cell_kind<double, WK_MMS>(stage, aos, prm, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+template <>
+cudaError_t LAUNCH_CELL<float>(int kind, int stage, bool aos, const WaveParams<float>& prm, cudaStream_t s) {
+  switch (kind) {
+    case WK_HOM: return cell_kind<float, WK_HOM>(stage, aos, prm, s);
+    case WK_VAR: return cell_kind<float, WK_VAR>(stage, aos, prm, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 template <>
 cudaError_t CONFIGURE_WAVE<double>(int kind) {
