@@ -10,6 +10,7 @@
 #include <map>
 #include <new>
 #include <string>
+#include <vector>
 
 #include "../../include/sbpgpu.h"
 #include "launch.h"
@@ -70,7 +71,7 @@ struct sbp_ctx {
   double* ct_tab = nullptr;                  // WAVE_MMS: the forcing's time factor per stage of a step graph
   void *va = nullptr, *vb = nullptr;         // advection with velocity fields: T planes (pitched)
   double *va64 = nullptr, *vb64 = nullptr;   // the same in FP64, nx*ny row-major (SAT)
-  double *rho64 = nullptr, *k64 = nullptr;   // WAVE_VAR: nx*ny FP64
+  double* satc = nullptr;                    // WAVE_VAR: SAT coefficients per boundary point (sat_point)
   int* err = nullptr;  // error word in page-locked host memory the kernels reach: no copy to read it
   int* sched = nullptr;  // the wave stage kernels' dynamic tile queue (2 ints, zero between launches)
   WaveMaps maps_un{}, maps_wa{}, maps_wb{};
@@ -197,8 +198,7 @@ WaveParams<T> wave_params(sbp_ctx* ctx) {
   p.plane = ctx->plane;
   p.rinv = (const T*)ctx->rinv;
   p.kmod = (const T*)ctx->kmod;
-  p.rho64 = ctx->rho64;
-  p.k64 = ctx->k64;
+  p.satc = ctx->satc;
   fill_taps<T>(p.dx, ctx->d.order, -ctx->hix);
   fill_taps<T>(p.dy, ctx->d.order, -ctx->hiy);
   const double hi0 = ops::get(ctx->d.order).hinv0;
@@ -345,6 +345,32 @@ int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in,
   }
   ctx->launches++;
   return SBP_OK;
+}
+
+// The SAT coefficients of the boundary points of a problem with coefficient fields
+// (apply_sat, sat_point): 1/(2 rho), Z = sqrt(rho K), c/2 = sqrt(K/rho)/2, K/2.
+cudaError_t make_sat_table(sbp_ctx* ctx) {
+  const int nx = (int)ctx->nx, ny = (int)ctx->ny, ys = ctx->ysplit;
+  std::vector<double> t(4 * sat_points(nx, ny, ys));
+  const auto put = [&](long long at, int i, int j) {
+    const double rho = ctx->d.rho[(long long)j * nx + i], k = ctx->d.K[(long long)j * nx + i];
+    double* o = &t[4 * at];
+    o[0] = 0.5 / rho;
+    o[1] = std::sqrt(rho * k);
+    o[2] = 0.5 * std::sqrt(k / rho);
+    o[3] = 0.5 * k;
+  };
+  std::vector<int> rows = {0, ny - 1};
+  if (ys > 0) rows.insert(rows.end(), {ys - 1, ys});
+  for (int j : rows)
+    for (int i = 0; i < nx; i++) put(sat_point(nx, ny, ys, i, j), i, j);
+  for (int j = 0; j < ny; j++) {
+    put(2LL * nx + j, 0, j);
+    put(2LL * nx + ny + j, nx - 1, j);
+  }
+  cudaError_t e = cudaMalloc((void**)&ctx->satc, t.size() * sizeof(double));
+  if (e == cudaSuccess) e = cudaMemcpy(ctx->satc, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice);
+  return e;
 }
 
 // One classical RK4 step on the resident state (time_stepping.h:127-142):
@@ -705,7 +731,7 @@ void release(sbp_ctx* ctx) {
   if (ctx->rk_partial) cudaFree(ctx->rk_partial);
   if (ctx->rk_ctrl) cudaFree(ctx->rk_ctrl);
   void* bufs[] = {ctx->un, ctx->acc, ctx->wa, ctx->wb, ctx->comp, ctx->io, ctx->partial, ctx->red,
-                  ctx->rinv, ctx->rho64, ctx->k64, ctx->sched, ctx->va, ctx->va64, ctx->ct_tab};
+                  ctx->rinv, ctx->satc, ctx->sched, ctx->va, ctx->va64, ctx->ct_tab};
   // kmod lives inside the rinv allocation, vb and vb64 inside those of va and va64
   for (void* b : bufs)
     if (b) cudaFree(b);
@@ -818,36 +844,31 @@ int sbp_create(const sbp_desc* desc, sbp_ctx** out) {
 
   if (has_fields(d.problem)) {
     const size_t np = (size_t)ctx->npts;
-    double* rinv_h = new (std::nothrow) double[np];
+    // 1/rho and K as padded planes of T, via the AoS->SoA kernel (dofs = 1)
+    double *rinv_h = new (std::nothrow) double[np], *tmp = nullptr;
     if (!rinv_h) return cuda_fail("host allocation", cudaErrorMemoryAllocation);
     for (size_t q = 0; q < np; q++) rinv_h[q] = 1.0 / d.rho[q];
-    if ((e = cudaMalloc((void**)&ctx->rho64, np * sizeof(double))) != cudaSuccess ||
-        (e = cudaMalloc((void**)&ctx->k64, np * sizeof(double))) != cudaSuccess ||
+    if ((e = cudaMalloc((void**)&tmp, 2 * np * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc(&ctx->rinv, 2 * ctx->plane * ctx->es)) != cudaSuccess) {
+      cudaFree(tmp);
       delete[] rinv_h;
       return cuda_fail("cudaMalloc(coefficients)", e);
     }
     cudaMemset(ctx->rinv, 0, 2 * ctx->plane * ctx->es);
     ctx->kmod = static_cast<unsigned char*>(ctx->rinv) + ctx->plane * ctx->es;  // second plane
-    cudaMemcpy(ctx->rho64, d.rho, np * sizeof(double), cudaMemcpyHostToDevice);
-    cudaMemcpy(ctx->k64, d.K, np * sizeof(double), cudaMemcpyHostToDevice);
-    // pack 1/rho and K into padded planes of T via the AoS->SoA kernel (dofs = 1)
-    double* tmp = nullptr;
-    if ((e = cudaMalloc((void**)&tmp, np * sizeof(double))) != cudaSuccess) {
-      delete[] rinv_h;
-      return cuda_fail("cudaMalloc(tmp)", e);
-    }
     cudaMemcpy(tmp, rinv_h, np * sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemcpy(tmp + np, d.K, np * sizeof(double), cudaMemcpyHostToDevice);
     delete[] rinv_h;
-    if (ctx->fp32) {
-      launch_pack<float>(tmp, (float*)ctx->rinv, (int)ctx->nx, (int)ctx->ny, 1, ctx->pitch, ctx->plane, 0);
-      launch_pack<float>(ctx->k64, (float*)ctx->kmod, (int)ctx->nx, (int)ctx->ny, 1, ctx->pitch, ctx->plane, 0);
-    } else {
-      launch_pack<double>(tmp, (double*)ctx->rinv, (int)ctx->nx, (int)ctx->ny, 1, ctx->pitch, ctx->plane, 0);
-      launch_pack<double>(ctx->k64, (double*)ctx->kmod, (int)ctx->nx, (int)ctx->ny, 1, ctx->pitch, ctx->plane, 0);
+    for (int f = 0; f < 2; f++) {
+      void* dst = f == 0 ? ctx->rinv : ctx->kmod;
+      if (ctx->fp32)
+        launch_pack<float>(tmp + f * np, (float*)dst, (int)ctx->nx, (int)ctx->ny, 1, ctx->pitch, ctx->plane, 0);
+      else
+        launch_pack<double>(tmp + f * np, (double*)dst, (int)ctx->nx, (int)ctx->ny, 1, ctx->pitch, ctx->plane, 0);
     }
     e = cudaDeviceSynchronize();
     cudaFree(tmp);
+    if (e == cudaSuccess) e = make_sat_table(ctx);
     if (e != cudaSuccess) return cuda_fail("coefficient upload", e);
   }
   if (d.problem == SBP_WAVE_MMS_2D) {

@@ -17,8 +17,8 @@
 //     Kahan term for the FP32 stage 4.
 //   * variable coefficients: [1/rho | K] as one 2-component box.
 // Consumers touch global memory only for their outputs (coalesced streaming
-// stores), for closure-row taps (boundary strips) and for the FP64 copies of
-// the coefficients at boundary points. The SAT of x-face points runs in a
+// stores), for closure-row taps (boundary strips) and for the SAT coefficients of
+// boundary points. The SAT of x-face points runs in a
 // separate pass per tile (see wave_tile_compute).
 // Every mbarrier wait is bounded by %globaltimer; a timeout sets an error bit
 // that the host reads and the CTA stops after letting its copies land.
@@ -64,8 +64,7 @@ template <typename T> struct WaveParams {
   T* comp;            // FP32: compensation term of the summed update (3 planes)
   const T* rinv;      // WK_VAR: 1/rho (1 plane)
   const T* kmod;      // WK_VAR: K (1 plane)
-  const double* rho64;  // WK_VAR: rho in FP64, read at boundary points
-  const double* k64;    // WK_VAR: K in FP64, read at boundary points
+  const double* satc;   // WK_VAR: the SAT's coefficients per boundary point (sat_point), FP64
   DirTaps<T> dx, dy;  // -hix * stencils, -hiy * stencils
   double bwx, bwy;    // hix * HI[0], hiy * HI[0]: SAT weights (FP64)
   T c_acc, c_w;       // acc (+)= c_acc * k ; w = u^n + c_w * k
@@ -325,6 +324,19 @@ __device__ __noinline__ T closure_line_global(const T* line, long long st, int n
 
 template <typename T> struct Rhs3 { T u, v, p; };
 
+// Where boundary point (i, j)'s SAT coefficients are in the table of a problem with
+// coefficient fields: rows j = 0 and ny - 1, columns i = 0 and nx - 1, then (two blocks) the
+// two interface lines; 4 doubles a point. A corner is listed with its row and its column.
+__host__ __device__ inline long long sat_point(int nx, int ny, int ysplit, int i, int j) {
+  if (j == 0) return i;
+  if (j == ny - 1) return (long long)nx + i;
+  if (ysplit > 0 && (j == ysplit - 1 || j == ysplit)) return 2LL * (nx + ny) + (j == ysplit ? nx : 0) + i;
+  return 2LL * nx + (i == 0 ? 0 : ny) + j;
+}
+__host__ __device__ inline long long sat_points(int nx, int ny, int ysplit) {
+  return 2LL * (nx + ny) + (ysplit > 0 ? 2LL * nx : 0);
+}
+
 // SAT boundary terms at a boundary point, FP64 weights, in the reference's
 // order west, south, east, north. Kept out of line so interior points branch
 // around it instead of issuing its FP64 instructions under a predicate.
@@ -332,31 +344,35 @@ template <typename T, int KIND>
 __device__ __noinline__ Rhs3<T> apply_sat(const WaveParams<T>& prm, const T* in, int i, int j, T pc, T uc, T vc,
                                           Rhs3<T> k) {
   const int nx = prm.nx, ny = prm.ny;
-  double rho = 1.0, kk = 1.0;
+  // 1/(2 rho), the impedance Z, c/2 and K/2 of the point; with variable coefficients from
+  // a table made with the context (square roots and divisions on GB300's FP64 pipe cost a
+  // boundary warp about 2 us each stage), with a constant K from the parameters
+  double hr = 0.5, z = 1.0, hc = 0.5, hk = 0.5;
   if constexpr (KIND == WK_VAR) {
-    rho = prm.rho64[(long long)j * nx + i];
-    kk = prm.k64[(long long)j * nx + i];
+    const double2* t = reinterpret_cast<const double2*>(prm.satc) + 2 * sat_point(nx, ny, prm.ysplit, i, j);
+    const double2 a = __ldg(t), b = __ldg(t + 1);
+    hr = a.x;
+    z = a.y;
+    hc = b.x;
+    hk = b.y;
   } else if constexpr (KIND == WK_CONST) {
-    kk = (double)prm.kconst;
+    z = prm.kz;
+    hc = 0.5 * prm.kc;
   }
+  (void)hk;
   const double p64 = (double)pc;
   double ku64 = (double)k.u, kv64 = (double)k.v, kp64 = (double)k.p;
   if (prm.bc == BC_NONE) {
     // matrix-free apply only
   } else if (prm.bc == BC_FREE_SURFACE) {
     // free_surface_bc_* (code/demo/wave_hom/wave_eq_hom_rhs.h:389-441); rho^-1 for WK_VAR
-    const double ri = (KIND == WK_VAR) ? 1.0 / rho : 1.0;
+    const double ri = 2.0 * hr;  // 1/rho, exactly
     if (i == 0) ku64 = (KIND == WK_VAR) ? ku64 - ri * (prm.bwx * p64) : ku64 - prm.bwx * p64;
     if (j == 0) kv64 = (KIND == WK_VAR) ? kv64 - ri * (prm.bwy * p64) : kv64 - prm.bwy * p64;
     if (i == nx - 1) ku64 = (KIND == WK_VAR) ? ku64 + ri * (prm.bwx * p64) : ku64 + prm.bwx * p64;
     if (j == ny - 1) kv64 = (KIND == WK_VAR) ? kv64 + ri * (prm.bwy * p64) : kv64 + prm.bwy * p64;
   } else {
-    // characteristic SAT on the incoming characteristic p + Z u_n; WK_CONST reads
-    // Z = c = sqrt(K) from the parameters (computed once on the host: an FP64
-    // square root per boundary point is long on the FP64 pipe)
-    const double z = KIND == WK_CONST ? prm.kz : sqrt(rho * kk);
-    const double c = KIND == WK_CONST ? prm.kc : sqrt(kk / rho);
-    const double hr = 0.5 / rho, hc = 0.5 * c;
+    // characteristic SAT on the incoming characteristic p + Z u_n
     const double u64 = (double)uc, v64 = (double)vc;
     if (i == 0) { const double g = prm.bwx * (p64 + z * u64); ku64 -= hr * g; kp64 -= hc * g; }
     if (j == 0) { const double g = prm.bwy * (p64 + z * v64); kv64 -= hr * g; kp64 -= hc * g; }
@@ -373,8 +389,8 @@ __device__ __noinline__ Rhs3<T> apply_sat(const WaveParams<T>& prm, const T* in,
       const long long qo = (long long)jo * prm.pitch + i;
       const double po = (double)in[2 * prm.plane + qo], vo = (double)in[prm.plane + qo];
       const double s = (j == ys - 1) ? 1.0 : -1.0;
-      kv64 += s * (0.5 / rho) * (prm.bwy * (p64 - po));
-      kp64 += s * (0.5 * kk) * (prm.bwy * ((double)vc - vo));
+      kv64 += s * hr * (prm.bwy * (p64 - po));
+      kp64 += s * hk * (prm.bwy * ((double)vc - vo));
     }
   }
   return Rhs3<T>{(T)ku64, (T)kv64, (T)kp64};
