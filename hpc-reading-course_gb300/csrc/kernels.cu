@@ -2,6 +2,7 @@
 // layout kernels at the reference boundary, the FP64 norm reductions and the
 // FP64 throughput probe.
 #include "launch.h"
+#include "line_steps.cuh"
 
 namespace sbp {
 
@@ -63,6 +64,78 @@ cudaError_t launch_line(int order, int kind, int stage, const LineParams<T>& prm
 }
 template cudaError_t launch_line<double>(int, int, int, const LineParams<double>&, cudaStream_t);
 template cudaError_t launch_line<float>(int, int, int, const LineParams<float>&, cudaStream_t);
+
+// ---------------------------------------------------------------- 1D step loops
+namespace {
+// CTAs of the cluster: 128 points each, up to the eight CTAs that every device can place
+// (32 to 128 points per CTA measured the same, 256 or more slower: 201 points 3.4 us a step
+// at 128, 3.8 at 256; 1601 points 4.0 at 8 CTAs, 5.5 at 512 points each).
+inline int line_ctas(long long nx) {
+  long long c = (nx + 127) / 128;
+  if (c > kLineMaxCtas) c = kLineMaxCtas;
+  while (c > 1 && nx / c < kLineMinChunk) c--;
+  return (int)(c < 1 ? 1 : c);
+}
+inline int line_chunk(long long nx) {
+  const int c = line_ctas(nx);
+  return (int)((nx + c - 1) / c);
+}
+constexpr size_t kLineSmemMax = 200 * 1024;
+
+template <typename T, int ORD, int KIND>
+cudaError_t steps_one(const LineParams<T>& prm, double dt, int steps, cudaStream_t s) {
+  const int chunk = line_chunk(prm.nx), ctas = (prm.nx + chunk - 1) / chunk;
+  int threads = (chunk + 8 * (OpShape<ORD>::W / 2) + 31) / 32 * 32;
+  if (threads > 512) threads = 512;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = LineSteps<T, ORD, KIND>::smem(chunk);
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, line_steps_kernel<T, ORD, KIND>, prm, chunk, steps, (T)(dt / 6), (T)(dt / 3),
+                            (T)(0.5 * dt), (T)dt);
+}
+template <typename T, int ORD, int KIND> cudaError_t steps_configure() {
+  return cudaFuncSetAttribute(line_steps_kernel<T, ORD, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)kLineSmemMax);
+}
+}  // namespace
+
+// Above about 6000 points eight CTAs' FP64 pipes take as long as the launches they replace
+// (reflection at 6401 points: 13.9 us a step against 12.8).
+bool line_steps_takes(long long nx, int kind, int elem_bytes) {
+  return nx <= (elem_bytes == 4 ? 8192 : (kind == LK_REFL1D ? 5000 : 6500));
+}
+
+template <typename T>
+cudaError_t launch_line_steps(int order, int kind, const LineParams<T>& prm, double dt, int steps, cudaStream_t s) {
+  const bool adv = kind == LK_ADV1D;
+  switch (order) {
+    case 2: return adv ? steps_one<T, 2, LK_ADV1D>(prm, dt, steps, s) : steps_one<T, 2, LK_REFL1D>(prm, dt, steps, s);
+    case 4: return adv ? steps_one<T, 4, LK_ADV1D>(prm, dt, steps, s) : steps_one<T, 4, LK_REFL1D>(prm, dt, steps, s);
+    case 6: return adv ? steps_one<T, 6, LK_ADV1D>(prm, dt, steps, s) : steps_one<T, 6, LK_REFL1D>(prm, dt, steps, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+template <typename T> cudaError_t configure_line_steps(int order, int kind) {
+  const bool adv = kind == LK_ADV1D;
+  switch (order) {
+    case 2: return adv ? steps_configure<T, 2, LK_ADV1D>() : steps_configure<T, 2, LK_REFL1D>();
+    case 4: return adv ? steps_configure<T, 4, LK_ADV1D>() : steps_configure<T, 4, LK_REFL1D>();
+    case 6: return adv ? steps_configure<T, 6, LK_ADV1D>() : steps_configure<T, 6, LK_REFL1D>();
+    default: return cudaErrorInvalidValue;
+  }
+}
+template cudaError_t launch_line_steps<double>(int, int, const LineParams<double>&, double, int, cudaStream_t);
+template cudaError_t launch_line_steps<float>(int, int, const LineParams<float>&, double, int, cudaStream_t);
+template cudaError_t configure_line_steps<double>(int, int);
+template cudaError_t configure_line_steps<float>(int, int);
 
 // ---------------------------------------------------------------- manufactured solution
 // code/demo/wave/wave_eq_rhs.h:42-64 with the time factor cos(5 pi t) left out. Run once

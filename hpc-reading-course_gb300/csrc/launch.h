@@ -129,6 +129,14 @@ int wave_smem_bytes(int order, bool fp32);
 template <typename T>
 cudaError_t launch_line(int order, int kind, int stage, const LineParams<T>& prm, cudaStream_t s);
 
+// `steps` RK4 steps of size dt of a 1D problem (kind LK_ADV1D or LK_REFL1D) in one launch
+// (line_steps.cuh), in place on prm.un and prm.comp; and the grids it takes.
+template <typename T>
+cudaError_t launch_line_steps(int order, int kind, const LineParams<T>& prm, double dt, int steps, cudaStream_t s);
+// Shared-memory opt-in of those kernels for one order and kind (outside stream capture).
+template <typename T> cudaError_t configure_line_steps(int order, int kind);
+bool line_steps_takes(long long nx, int kind, int elem_bytes);
+
 // The 3D wave stage kernel (wave3d.cu).
 template <typename T>
 cudaError_t launch_wave3d(int order, int stage, const Wave3Params<T>& prm, cudaStream_t s);

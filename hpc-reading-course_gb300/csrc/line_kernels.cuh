@@ -108,6 +108,19 @@ __device__ __forceinline__ T adv2d_sat(const LineParams<T>& prm, int i, int j, T
   return k;
 }
 
+// SAT_bc_l / SAT_bc_r of 1D advection (advection_rhs.h:94-119), FP64.
+template <typename T>
+__device__ __forceinline__ T adv1d_sat(const LineParams<T>& prm, int i, T k, T cen) {
+  const int nx = prm.nx;
+  if (!prm.bc || (i != 0 && i != nx - 1)) return k;
+  if (prm.va64) {
+    const double a = prm.va64[i];
+    const double tau = i == 0 ? -0.5 * (a + fabs(a)) : 0.5 * (a - fabs(a));
+    return (T)((double)k + 0.5 * tau * prm.bw[0] * (double)cen);
+  }
+  return (T)((double)k + prm.sat[i == 0 ? 0 : 2] * (double)cen);
+}
+
 // One grid point of a stage: RHS, boundary terms and the RK4 stage update.
 template <typename T, int ORD, int KIND, int STAGE>
 __device__ __forceinline__ void line_point(const LineParams<T>& prm, const T* __restrict__ in, T* wout, const T c_acc,
@@ -122,18 +135,7 @@ __device__ __forceinline__ void line_point(const LineParams<T>& prm, const T* __
     k[0] = d1_line<T, ORD>(in, 1, nx, i, prm.dx);
     if (prm.va) k[0] = -prm.va[q] * k[0];  // -a(i) D1 u
     cen[0] = in[q];
-    if (prm.bc) {  // SAT_bc_l / SAT_bc_r (advection_rhs.h:94-119)
-      if (prm.va64) {
-        if (i == 0 || i == nx - 1) {
-          const double a = prm.va64[i];
-          const double tau = i == 0 ? -0.5 * (a + fabs(a)) : 0.5 * (a - fabs(a));
-          k[0] = (T)((double)k[0] + 0.5 * tau * prm.bw[0] * (double)cen[0]);
-        }
-      } else {
-        if (i == 0) k[0] = (T)((double)k[0] + prm.sat[0] * (double)cen[0]);
-        if (i == nx - 1) k[0] = (T)((double)k[0] + prm.sat[2] * (double)cen[0]);
-      }
-    }
+    k[0] = adv1d_sat<T>(prm, i, k[0], cen[0]);
   } else if constexpr (KIND == LK_ADV2D) {
     const T* row = in + (long long)j * pitch;
     const T* col = in + i;

@@ -406,6 +406,12 @@ void drop_graphs(sbp_ctx* ctx) {
 }
 
 constexpr long long kRk4Chunk = 50;  // steps per graph launch
+constexpr long long kLineStepsPerLaunch = 1000;
+
+// Whether a context's RK4 steps run as whole step loops on one cluster (line_steps.cuh).
+bool line_steps_runs(const sbp_ctx* ctx) {
+  return !ctx->two_d && !ctx->three_d && line_steps_takes(ctx->nx, line_kind(ctx), (int)ctx->es);
+}
 
 // `steps` (at most kRk4Chunk) steps from time t as one graph, captured once per step count
 // and dt. Time-dependent problems: the steps' stage-time factors go to ct_tab, in stream
@@ -456,6 +462,18 @@ template <typename T>
 int rk4_resident_t(sbp_ctx* ctx, double t0, double dt, long long nsteps) {
   double t = t0;
   long long left = nsteps;
+  if (line_steps_runs(ctx)) {
+    // as many steps per launch as keep a launch within some milliseconds
+    LineParams<T> p = line_params<T>(ctx);
+    p.un = (T*)ctx->un;
+    p.comp = (T*)ctx->comp;
+    for (; left > 0; left -= kLineStepsPerLaunch) {
+      const int n = (int)(left < kLineStepsPerLaunch ? left : kLineStepsPerLaunch);
+      CK(launch_line_steps<T>(ctx->d.order, line_kind(ctx), p, dt, n, ctx->stream));
+      ctx->launches++;
+    }
+    return SBP_OK;
+  }
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (ctx->time_dependent) CK(cudaStreamIsCapturing(ctx->stream, &cap));
   if (cap != cudaStreamCaptureStatusNone) {  // the caller is capturing: launches with the stage times as values
@@ -931,6 +949,11 @@ int sbp_create(const sbp_desc* desc, sbp_ctx** out) {
     // shared-memory opt-in of the stage kernels, done here (not under stream capture)
     e = ctx->fp32 ? configure_wave<float>(d.order, wave_kind(ctx)) : configure_wave<double>(d.order, wave_kind(ctx));
     if (e != cudaSuccess) return cuda_fail("configure stage kernels", e);
+  }
+  if (line_steps_runs(ctx)) {
+    e = ctx->fp32 ? configure_line_steps<float>(d.order, line_kind(ctx))
+                  : configure_line_steps<double>(d.order, line_kind(ctx));
+    if (e != cudaSuccess) return cuda_fail("configure step-loop kernel", e);
   }
   if (ctx->three_d) {
     e = ctx->fp32 ? configure_wave3d<float>(d.order) : configure_wave3d<double>(d.order);
