@@ -1,6 +1,7 @@
 // kernels.cu -- launchers for the scalar/1D stage kernels, the AoS <-> SoA
 // layout kernels at the reference boundary, the FP64 norm reductions and the
 // FP64 throughput probe.
+#include "adv_cell.cuh"
 #include "launch.h"
 #include "line_steps.cuh"
 
@@ -28,8 +29,32 @@ int device_sm_count() {
 
 // ---------------------------------------------------------------- line kernels
 namespace {
+template <int ORD, bool FIELDS, int ROWS>
+cudaError_t adv_cell_stage(int stage, const LineParams<double>& prm, cudaStream_t s) {
+  constexpr int TY = kCellThreads / 32 * ROWS;
+  const dim3 grid((prm.nx + kCellTX - 1) / kCellTX, (prm.ny + TY - 1) / TY);
+  switch (stage) {
+    case ST_RHS: return launch_overlapped(adv_cell_kernel<ORD, ST_RHS, FIELDS, ROWS>, grid, kCellThreads, 0, s, prm);
+    case ST_FIRST: return launch_overlapped(adv_cell_kernel<ORD, ST_FIRST, FIELDS, ROWS>, grid, kCellThreads, 0, s, prm);
+    case ST_MID: return launch_overlapped(adv_cell_kernel<ORD, ST_MID, FIELDS, ROWS>, grid, kCellThreads, 0, s, prm);
+    case ST_LAST: return launch_overlapped(adv_cell_kernel<ORD, ST_LAST, FIELDS, ROWS>, grid, kCellThreads, 0, s, prm);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 template <typename T, int ORD, int KIND>
 cudaError_t line_stage(int stage, const LineParams<T>& prm, cudaStream_t s) {
+  if constexpr (KIND == LK_ADV2D && sizeof(T) == 8) {
+    // us per stage at order 4, line form / cells of one / two rows per thread: 129^2 3.2 / 3.5 /
+    // 4.5, 257^2 4.4 / 4.0 / 5.4, 513^2 11.7 / 5.9 / 6.2, 801^2 19.6 / 10.3 / 10.0, 1025^2 29.3 /
+    // 14.9 / 13.9, 2049^2 103 / 56 / 47 (four rows: 49)
+    const long long points = (long long)prm.nx * prm.ny;
+    if (points > 40000) {
+      if (points <= 450000)
+        return prm.va ? adv_cell_stage<ORD, true, 1>(stage, prm, s) : adv_cell_stage<ORD, false, 1>(stage, prm, s);
+      return prm.va ? adv_cell_stage<ORD, true, 2>(stage, prm, s) : adv_cell_stage<ORD, false, 2>(stage, prm, s);
+    }
+  }
   const dim3 block(KIND == LK_ADV2D ? 32 : 128, KIND == LK_ADV2D ? 8 : 1);
   const dim3 grid((prm.nx + block.x - 1) / block.x, (prm.ny + block.y - 1) / block.y);
   switch (stage) {

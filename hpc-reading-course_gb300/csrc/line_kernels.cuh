@@ -33,6 +33,7 @@ template <typename T> struct LineParams {
   const double* va64;
   const double* vb64;
   double bw[2];
+  double fx_sig[2];   // 2D, FP64 cells: a direction's derivative is fx_sig times the integer stencil sum
   int bc;             // 0: none, 1: the reference's boundary treatment
   int compensated;
   T c_acc, c_w;

@@ -242,6 +242,9 @@ LineParams<T> line_params(sbp_ctx* ctx) {
   }
   p.bc = 1;
   p.compensated = ctx->fp32 ? 1 : 0;
+  const double den = fixed_denominator(ctx->d.order);
+  p.fx_sig[0] = ctx->va ? ctx->hix / den : -a * ctx->hix / den;
+  p.fx_sig[1] = ctx->va ? ctx->hiy / den : -b * ctx->hiy / den;
   p.err = ctx->err;
   return p;
 }
