@@ -570,7 +570,8 @@ int launch_rhs_aos(sbp_ctx* ctx, double t, const double* src, double* dst, int b
 // interface SAT reads the other block's line from the planes).
 bool rhs_takes_aos(const sbp_ctx* ctx, const double* src, const double* dst, int where) {
   const double *se = src + ctx->nscalar, *de = dst + ctx->nscalar;
-  return where == SBP_DEVICE && ctx->wave && !ctx->ysplit && !ctx->drop_tile && (se <= dst || de <= src);
+  return where == SBP_DEVICE && ctx->wave && !ctx->ysplit && !ctx->drop_tile && (se <= dst || de <= src) &&
+         ctx->ny <= 65535LL * kCellTY;  // the rows a grid of cells can have
 }
 
 int rhs_impl(sbp_ctx* ctx, double t, const double* src, double* dst, int where, int bc_on) {
