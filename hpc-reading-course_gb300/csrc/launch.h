@@ -12,6 +12,7 @@
 #include "wave2d.cuh"
 #include "wave_cell.cuh"
 #include "wave3d.cuh"
+#include "wave3d_fixed.cuh"
 #include "wave_batch.cuh"
 
 namespace sbp {
@@ -137,9 +138,10 @@ cudaError_t launch_line_steps(int order, int kind, const LineParams<T>& prm, dou
 template <typename T> cudaError_t configure_line_steps(int order, int kind);
 bool line_steps_takes(long long nx, int kind, int elem_bytes);
 
-// The 3D wave stage kernel (wave3d.cu).
+// The 3D wave stage kernel (wave3d.cu). maps: of the stage input (FP64; null: the kernels
+// that need none).
 template <typename T>
-cudaError_t launch_wave3d(int order, int stage, const Wave3Params<T>& prm, cudaStream_t s);
+cudaError_t launch_wave3d(int order, int stage, const Wave3Params<T>& prm, const Wave3Maps* maps, cudaStream_t s);
 // Shared-memory opt-in of the 3D stage kernels of one order (outside stream capture).
 template <typename T> cudaError_t configure_wave3d(int order);
 

@@ -75,6 +75,7 @@ struct sbp_ctx {
   int* err = nullptr;  // error word in page-locked host memory the kernels reach: no copy to read it
   int* sched = nullptr;  // the wave stage kernels' dynamic tile queue (2 ints, zero between launches)
   WaveMaps maps_un{}, maps_wa{}, maps_wb{};
+  Wave3Maps maps3[3]{};  // 3D FP64: stage inputs un, wa, wb
   // adaptive RK45 (FP64; allocated on first use)
   double* rk_k[6] = {};
   double* rk_unew = nullptr;
@@ -184,6 +185,31 @@ int make_maps(sbp_ctx* ctx, void* base, WaveMaps& m) {
   if (enc(&m.k, dt, 3, ctx->rinv, dims, strides, boxK, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return fail(ctx, SBP_ERR_CUDA, "cuTensorMapEncodeTiled failed for the coefficient planes");
+  return SBP_OK;
+}
+
+// The 3D FP64 kernel's maps of stage input `base`: (x, y, z, component).
+int make_maps3(sbp_ctx* ctx, void* base, Wave3Maps& m) {
+  EncodeTiledFn enc = encode_tiled();
+  if (!enc) return fail(ctx, SBP_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const unsigned R = ctx->d.order / 2, HX = (R + 1) / 2 * 2;
+  const cuuint64_t dims[4] = {(cuuint64_t)ctx->nx, (cuuint64_t)ctx->ny, (cuuint64_t)ctx->nz, 4};
+  const cuuint64_t strides[3] = {(cuuint64_t)ctx->pitch * 8, (cuuint64_t)(ctx->pitch * ctx->ny) * 8,
+                                 (cuuint64_t)ctx->plane * 8};
+  const cuuint32_t estr[4] = {1, 1, 1, 1};
+  const struct {
+    CUtensorMap* map;
+    void* base;
+    cuuint32_t box[4];
+  } all[] = {{&m.p, base, {kF3X + 2 * HX, kF3Y + 2 * R, 1, 1}}, {&m.w, base, {kF3X, kF3Y, 1, 1}},
+             {&m.u, base, {kF3X + 2 * HX, kF3Y, 1, 1}},         {&m.v, base, {kF3X, kF3Y + 2 * R, 1, 1}},
+             {&m.n, ctx->un, {kF3X, kF3Y, 1, 4}},               {&m.a, ctx->acc, {kF3X, kF3Y, 1, 4}}};
+  for (const auto& e : all) {
+    const CUresult r =
+        enc(e.map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, e.base, dims, strides, e.box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return fail(ctx, SBP_ERR_CUDA, "cuTensorMapEncodeTiled failed: " + std::to_string(r));
+  }
   return SBP_OK;
 }
 
@@ -330,8 +356,21 @@ int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in,
     p.compensated = ctx->fp32 ? 1 : 0;
     p.c_acc = c_acc;
     p.c_w = c_w;
+    const double hi[3] = {ctx->hix, ctx->hiy, ctx->hiz}, den = fixed_denominator(ctx->d.order);
+    for (int c = 0; c < 4; c++) {
+      const double sig = -hi[c % 3] / den;  // p (c = 3): x
+      p.fx_ca[c] = (double)c_acc * sig;
+      p.fx_cw[c] = (double)c_w * sig;
+      if (c == 3) continue;
+      p.fx_sig[c] = sig;
+      p.fx_isig[c] = -den / hi[c];
+    }
+    p.fx_rho[0] = ctx->hiy / ctx->hix;
+    p.fx_rho[1] = ctx->hiz / ctx->hix;
     if (ctl) p.skip = &ctl->done;
-    CK(launch_wave3d<T>(ctx->d.order, stage, p, ctx->stream));
+    p.err = ctx->err;
+    const Wave3Maps* maps = ctx->fp32 ? nullptr : (in == ctx->un ? &ctx->maps3[0] : (in == ctx->wa ? &ctx->maps3[1] : &ctx->maps3[2]));
+    CK(launch_wave3d<T>(ctx->d.order, stage, p, maps, ctx->stream));
   } else {
     LineParams<T> p = line_params<T>(ctx);
     p.in = (const T*)in;
@@ -960,6 +999,13 @@ int sbp_create(const sbp_desc* desc, sbp_ctx** out) {
     if (e != cudaSuccess) return cuda_fail("configure step-loop kernel", e);
   }
   if (ctx->three_d) {
+    if (!ctx->fp32 && (make_maps3(ctx, ctx->un, ctx->maps3[0]) || make_maps3(ctx, ctx->wa, ctx->maps3[1]) ||
+                       make_maps3(ctx, ctx->wb, ctx->maps3[2]))) {
+      g_create_error = ctx->msg;
+      release(ctx);
+      delete ctx;
+      return SBP_ERR_CUDA;
+    }
     e = ctx->fp32 ? configure_wave3d<float>(d.order) : configure_wave3d<double>(d.order);
     if (e != cudaSuccess) return cuda_fail("configure 3D stage kernels", e);
   }

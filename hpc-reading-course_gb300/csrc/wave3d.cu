@@ -1,14 +1,13 @@
 // wave3d.cu -- fused RHS + SAT + RK4-stage kernels of the 3D acoustic wave
 // system (wave3d.cuh), orders 2, 4 and 6, FP64 or compensated FP32.
 //
-// Two forms. The plane-ring kernel (the default for both precisions) stages each z
-// plane of the block's column tile in shared memory with 16-byte cp.async copies
-// running ahead of the plane it computes, so its loads are in flight while it
-// computes; measured at 256^3, order 4: FP32 6.35e10 point-stage updates/s (0.67
-// of the measured HBM copy bandwidth) against 3.48e10 for the column kernel, FP64
-// 1.32e10 against 1.22e10 (FP64-pipe bound). The column kernel (one thread per
-// (i, j) column marching 16 planes, every tap a read-only global load) runs where
-// the ring kernel's 32-bit offsets or 16-byte alignment do not hold.
+// Three forms. FP32: the plane-ring kernel stages each z plane of the block's column tile in
+// shared memory with 16-byte cp.async copies running ahead of the plane it computes, so its
+// loads are in flight while it computes; measured at 256^3, order 4: 6.7e10 point-stage
+// updates/s (0.7 of the measured HBM copy bandwidth) against 3.48e10 for the column kernel.
+// FP64: wave3d_fixed_kernel (wave3d_fixed.cuh), integer stencils on TMA boxes. The column
+// kernel (one thread per (i, j) column marching 16 planes, every tap a read-only global load)
+// runs where their 32-bit offsets or 16-byte alignment do not hold.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -19,52 +18,6 @@
 namespace sbp {
 
 constexpr int kW3X = 64, kW3Y = 4, kW3Z = 16;
-
-// Boundary terms on the faces the point lies on (FP64 arithmetic, as the 2D kernels):
-// free surface (wave_eq_hom_rhs.h:389-441 per face): lower face F_ud -= bw_d p, upper F_ud += bw_d p;
-// characteristic (Z = c = 1): lower face g = bw_d (p + u_d): F_ud -= g/2, F_p -= g/2;
-// upper face g = bw_d (p - u_d): F_ud += g/2, F_p -= g/2.
-template <typename T> struct Rhs4 { T u, v, w, p; };
-
-template <typename T>
-__device__ __noinline__ Rhs4<T> wave3d_sat(const Wave3Params<T>& prm, int i, int j, int k, T uc, T vc, T wc, T pc,
-                                           Rhs4<T> kc) {
-  // values and results by value: a noinline function taking arrays by reference
-  // would keep the caller's arrays in local memory on every point. Only the
-  // components a face changes go through FP64 (the others would round-trip
-  // exactly), in the order of the faces, so that a point on one face costs about
-  // ten FP64-pipe instructions.
-  const T cen[3] = {uc, vc, wc};
-  T f[3] = {kc.u, kc.v, kc.w};
-  const int idx[3] = {i, j, k};
-  const int n[3] = {prm.nx, prm.ny, prm.nz};
-  const double p = (double)pc;
-  double fp = (double)kc.p;
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    const bool lo = idx[d] == 0, hi = idx[d] == n[d] - 1;
-    if (!lo && !hi) continue;
-    const double ud = (double)cen[d];
-    double fd = (double)f[d];
-    if (prm.bc == BC_CHARACTERISTIC) {
-      if (lo) {
-        const double g = prm.bw[d] * (p + ud);
-        fd -= 0.5 * g;
-        fp -= 0.5 * g;
-      }
-      if (hi) {
-        const double g = prm.bw[d] * (p - ud);
-        fd += 0.5 * g;
-        fp -= 0.5 * g;
-      }
-    } else {
-      if (lo) fd -= prm.bw[d] * p;
-      if (hi) fd += prm.bw[d] * p;
-    }
-    f[d] = (T)fd;
-  }
-  return Rhs4<T>{f[0], f[1], f[2], (T)fp};
-}
 
 // FP64: the z neighbours of p and w come from a per-thread register window (one new
 // value of each per plane instead of the five taps); measured at 256^3, order 4:
@@ -246,9 +199,6 @@ __global__ void __launch_bounds__(kW3X * kW3Y, sizeof(T) == 8 ? SBP_W3_BLOCKS_F6
 #ifndef SBP_R3_BLOCKS
 #define SBP_R3_BLOCKS 8
 #endif
-#ifndef SBP_R3_BLOCKS_F64
-#define SBP_R3_BLOCKS_F64 3
-#endif
 constexpr int kR3X = SBP_R3_X, kR3Y = SBP_R3_Y, kR3Z = SBP_R3_Z, kR3D = SBP_R3_D;
 constexpr int kR3Threads = kR3X * kR3Y;
 
@@ -321,7 +271,8 @@ __device__ __forceinline__ T taps_smem(const DirTaps<T>& d, const T* c, int st) 
 }
 
 template <typename T, int ORD, int STAGE>
-__global__ void __launch_bounds__(kR3Threads, sizeof(T) == 8 ? SBP_R3_BLOCKS_F64 : SBP_R3_BLOCKS) wave3d_ring_kernel(const __grid_constant__ Wave3Params<T> prm) {
+__global__ void __launch_bounds__(kR3Threads, SBP_R3_BLOCKS)
+    wave3d_ring_kernel(const __grid_constant__ Wave3Params<T> prm) {
   using G = Ring3<T, ORD, STAGE>;
   constexpr int W = OpShape<ORD>::W, R = G::R, CS = OpShape<ORD>::CS, D = G::D;
   constexpr int TX = G::TX, TY = G::TY, PX = G::PX, SA = G::SA, SB = G::SB;
@@ -455,16 +406,6 @@ __global__ void __launch_bounds__(kR3Threads, sizeof(T) == 8 ? SBP_R3_BLOCKS_F64
   cp_async_wait<0>();
 }
 
-// Which form runs per precision: the plane-ring kernel for both (figures at the
-// top of this file).
-#ifndef SBP_W3_RING_F32
-#define SBP_W3_RING_F32 1
-#endif
-#ifndef SBP_W3_RING_F64
-#define SBP_W3_RING_F64 1
-#endif
-template <typename T> constexpr bool w3_ring() { return sizeof(T) == 8 ? SBP_W3_RING_F64 : SBP_W3_RING_F32; }
-
 namespace {
 
 // SBP_WAVE3D_COLUMN=1 in the environment selects the column kernel (read at each
@@ -474,9 +415,40 @@ inline bool w3_force_column() {
   return e != nullptr && e[0] == '1';
 }
 
+// z planes per CTA of the fixed-point kernel. A CTA converts 2R planes more than it computes,
+// but CTAs on a face take longer than inner ones, so a grid wants several waves of them: 12
+// planes where that leaves four waves of two CTAs per SM, fewer (down to 4) on smaller grids.
+// us per stage at order 4 with 4 / 6 / 8 / 12 / 24 / 48 planes: 49^3 38 / 36 / 45 / 65 / 122 / 239,
+// 97^3 111 / 116 / 115 / 143 / 174 / 240, 201 x 193 x 161 406 / 394 / 389 / 382 / 406 / 471,
+// 256^3 896 / 851 / 841 / 817 / 824 / 891.
+inline int fixed3_chunk(long long columns, int nz) {
+  const long long z = columns * nz / (4 * 2 * device_sm_count());
+  return (int)(z < 4 ? 4 : (z > 12 ? 12 : z));
+}
+
+template <int ORD, int STAGE>
+cudaError_t fixed3_one(const Wave3Params<double>& prm, const Wave3Maps& maps, cudaStream_t s) {
+  const long long gx = (prm.nx + kF3X - 1) / kF3X, gy = (prm.ny + kF3Y - 1) / kF3Y;
+  const int chunk = fixed3_chunk(gx * gy, prm.nz);
+  const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)((prm.nz + chunk - 1) / chunk));
+  wave3d_fixed_kernel<ORD, STAGE><<<grid, kF3Threads, Fixed3<ORD, STAGE>::SMEM, s>>>(maps, prm, chunk);
+  return cudaGetLastError();
+}
+
 template <typename T, int ORD>
-cudaError_t wave3d_order(int stage, const Wave3Params<T>& prm, cudaStream_t s) {
-  if constexpr (w3_ring<T>()) {
+cudaError_t wave3d_order(int stage, const Wave3Params<T>& prm, const Wave3Maps* maps, cudaStream_t s) {
+  if constexpr (sizeof(T) == 8) {
+    // element offsets are 32-bit
+    if (!w3_force_column() && maps && 4 * prm.plane < (1LL << 31) && prm.ny <= 65535 * kF3Y && prm.nz <= 65535 * 4) {
+      switch (stage) {
+        case ST_RHS: return fixed3_one<ORD, ST_RHS>(prm, *maps, s);
+        case ST_FIRST: return fixed3_one<ORD, ST_FIRST>(prm, *maps, s);
+        case ST_MID: return fixed3_one<ORD, ST_MID>(prm, *maps, s);
+        case ST_LAST: return fixed3_one<ORD, ST_LAST>(prm, *maps, s);
+        default: return cudaErrorInvalidValue;
+      }
+    }
+  } else {
     // the ring kernel's element offsets are 32-bit and its copies 16-byte aligned
     const auto al16 = [](const void* q) { return q == nullptr || ((uintptr_t)q & 15) == 0; };
     if (!w3_force_column() && 4 * prm.plane < (1LL << 31) && prm.pitch % 64 == 0 && al16(prm.in) &&
@@ -510,46 +482,46 @@ cudaError_t wave3d_order(int stage, const Wave3Params<T>& prm, cudaStream_t s) {
 }  // namespace
 
 template <typename T>
-cudaError_t launch_wave3d(int order, int stage, const Wave3Params<T>& prm, cudaStream_t s) {
+cudaError_t launch_wave3d(int order, int stage, const Wave3Params<T>& prm, const Wave3Maps* maps, cudaStream_t s) {
   if (prm.nz > 65535 * kW3Z || prm.ny > 65535 * kW3Y || prm.nz > 65535 * kR3Z || prm.ny > 65535 * kR3Y)
     return cudaErrorInvalidValue;
   switch (order) {
-    case 2: return wave3d_order<T, 2>(stage, prm, s);
-    case 4: return wave3d_order<T, 4>(stage, prm, s);
-    case 6: return wave3d_order<T, 6>(stage, prm, s);
+    case 2: return wave3d_order<T, 2>(stage, prm, maps, s);
+    case 4: return wave3d_order<T, 4>(stage, prm, maps, s);
+    case 6: return wave3d_order<T, 6>(stage, prm, maps, s);
     default: return cudaErrorInvalidValue;
   }
 }
 namespace {
-template <typename T, int ORD, int STAGE> cudaError_t configure_ring() {
-  return cudaFuncSetAttribute(wave3d_ring_kernel<T, ORD, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)Ring3<T, ORD, STAGE>::SMEM);
+template <typename T, int ORD, int STAGE> cudaError_t configure_stage() {
+  if constexpr (sizeof(T) == 8)
+    return cudaFuncSetAttribute(wave3d_fixed_kernel<ORD, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                Fixed3<ORD, STAGE>::SMEM);
+  else
+    return cudaFuncSetAttribute(wave3d_ring_kernel<T, ORD, STAGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)Ring3<T, ORD, STAGE>::SMEM);
 }
-template <typename T, int ORD> cudaError_t configure_ring_order() {
+template <typename T, int ORD> cudaError_t configure_order() {
   cudaError_t e;
-  if ((e = configure_ring<T, ORD, ST_RHS>()) != cudaSuccess) return e;
-  if ((e = configure_ring<T, ORD, ST_FIRST>()) != cudaSuccess) return e;
-  if ((e = configure_ring<T, ORD, ST_MID>()) != cudaSuccess) return e;
-  return configure_ring<T, ORD, ST_LAST>();
+  if ((e = configure_stage<T, ORD, ST_RHS>()) != cudaSuccess) return e;
+  if ((e = configure_stage<T, ORD, ST_FIRST>()) != cudaSuccess) return e;
+  if ((e = configure_stage<T, ORD, ST_MID>()) != cudaSuccess) return e;
+  return configure_stage<T, ORD, ST_LAST>();
 }
 }  // namespace
 
 template <typename T> cudaError_t configure_wave3d(int order) {
-  if constexpr (!w3_ring<T>()) {
-    return cudaSuccess;
-  } else {
-    switch (order) {
-      case 2: return configure_ring_order<T, 2>();
-      case 4: return configure_ring_order<T, 4>();
-      case 6: return configure_ring_order<T, 6>();
-      default: return cudaErrorInvalidValue;
-    }
+  switch (order) {
+    case 2: return configure_order<T, 2>();
+    case 4: return configure_order<T, 4>();
+    case 6: return configure_order<T, 6>();
+    default: return cudaErrorInvalidValue;
   }
 }
 template cudaError_t configure_wave3d<double>(int);
 template cudaError_t configure_wave3d<float>(int);
 
-template cudaError_t launch_wave3d<double>(int, int, const Wave3Params<double>&, cudaStream_t);
-template cudaError_t launch_wave3d<float>(int, int, const Wave3Params<float>&, cudaStream_t);
+template cudaError_t launch_wave3d<double>(int, int, const Wave3Params<double>&, const Wave3Maps*, cudaStream_t);
+template cudaError_t launch_wave3d<float>(int, int, const Wave3Params<float>&, const Wave3Maps*, cudaStream_t);
 
 }  // namespace sbp

@@ -33,6 +33,11 @@ template <typename T> struct Wave3Params {
   int compensated;        // FP32 state with the Kahan-summed final update
   T c_acc, c_w;           // acc (+)= c_acc * k ; w = u^n + c_w * k
   const int* skip;        // non-null and set: the kernel returns at entry
+  int* err;               // error word
+  // FP64 (wave3d_fixed_kernel): the RHS is formed in units of sigma_d = -hi_d/den per direction
+  // (u, v, w: their own, p: sigma_x); sigma, 1/sigma, sigma_y/sigma_x and sigma_z/sigma_x,
+  // and the stage's RK4 coefficients times each component's sigma
+  double fx_sig[3], fx_isig[3], fx_rho[2], fx_ca[4], fx_cw[4];
 };
 
 }  // namespace sbp
