@@ -11,6 +11,7 @@
 #include "line_kernels.cuh"
 #include "wave2d.cuh"
 #include "wave_cell.cuh"
+#include "wave_step.cuh"
 #include "wave3d.cuh"
 #include "wave3d_fixed.cuh"
 #include "wave_batch.cuh"
@@ -119,6 +120,32 @@ inline cudaError_t launch_cell(int order, int kind, int stage, bool aos, const W
     default: return cudaErrorInvalidValue;
   }
 }
+// A whole RK4 step of a small FP64 grid (wave_step.cuh): from prm.in to prm.wout.
+cudaError_t launch_step_o2(int kind, const WaveParams<double>& prm, const WaveStepCoef& cf, cudaStream_t s);
+cudaError_t launch_step_o4(int kind, const WaveParams<double>& prm, const WaveStepCoef& cf, cudaStream_t s);
+cudaError_t launch_step_o6(int kind, const WaveParams<double>& prm, const WaveStepCoef& cf, cudaStream_t s);
+inline cudaError_t launch_step(int order, int kind, const WaveParams<double>& prm, const WaveStepCoef& cf,
+                               cudaStream_t s) {
+  switch (order) {
+    case 2: return launch_step_o2(kind, prm, cf, s);
+    case 4: return launch_step_o4(kind, prm, cf, s);
+    case 6: return launch_step_o6(kind, prm, cf, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+// The grids it takes: at most one CTA of the larger cell per SM (figures in wave_step.cuh).
+inline bool step_takes(int order, long long nx, long long ny) {
+  const int t = step_large(order);
+  return ((nx + t - 1) / t) * ((ny + t - 1) / t) <= device_sm_count();
+}
+// Its shared-memory opt-in (outside stream capture).
+cudaError_t configure_step_o2(int kind);
+cudaError_t configure_step_o4(int kind);
+cudaError_t configure_step_o6(int kind);
+inline cudaError_t configure_step(int order, int kind) {
+  return order == 2 ? configure_step_o2(kind) : (order == 4 ? configure_step_o4(kind) : configure_step_o6(kind));
+}
+
 // The CTAs a grid takes.
 inline dim3 cell_grid(long long nx, long long ny) {
   return dim3((unsigned)((nx + kCellTX - 1) / kCellTX), (unsigned)((ny + kCellTY - 1) / kCellTY));

@@ -442,6 +442,51 @@ int enqueue_step(sbp_ctx* ctx, double t, double dt, const double* ct = nullptr) 
   return SBP_OK;
 }
 
+// Whether a context's RK4 steps run as one launch each (wave_step.cuh).
+bool use_step(const sbp_ctx* ctx) {
+  return ctx->wave && !ctx->fp32 && step_takes(ctx->d.order, ctx->nx, ctx->ny);
+}
+
+// One RK4 step from `in` to `out` in one launch; ct as for enqueue_step.
+int enqueue_whole_step(sbp_ctx* ctx, void* in, void* out, double dt, const double* ct) {
+  WaveParams<double> p = wave_params<double>(ctx);
+  p.in = (const double*)in;
+  p.wout = (double*)out;
+  p.ctp = ct;
+  p.c_acc = dt / 6;
+  p.c_w = 0.5 * dt;
+  set_fixed_scales(p, ctx->d.order, ctx->hix, ctx->hiy);
+  WaveStepCoef cf = {};
+  const double sg[3] = {p.fx_sig[0], p.fx_sig[1], p.fx_sigp};
+  for (int c = 0; c < 3; c++) {
+    cf.ca[0][c] = (dt / 6) * sg[c];
+    cf.ca[1][c] = (dt / 3) * sg[c];
+    cf.cw[0][c] = (0.5 * dt) * sg[c];
+    cf.cw[1][c] = dt * sg[c];
+  }
+  CK(launch_step(ctx->d.order, wave_kind(ctx), p, cf, ctx->stream));
+  ctx->launches++;
+  return SBP_OK;
+}
+
+// `steps` steps for a step graph: stage by stage in place, or as whole steps alternating
+// between u^n and wa (a copy brings an odd count's result back).
+template <typename T>
+int enqueue_steps(sbp_ctx* ctx, long long steps, double dt) {
+  const auto ct = [&](long long s) { return ctx->ct_tab ? ctx->ct_tab + 3 * s : nullptr; };
+  int rc = SBP_OK;
+  if (!use_step(ctx)) {
+    for (long long s = 0; s < steps && rc == SBP_OK; s++) rc = enqueue_step<T>(ctx, 0.0, dt, ct(s));
+    return rc;
+  }
+  for (long long s = 0; s < steps && rc == SBP_OK; s++)
+    rc = enqueue_whole_step(ctx, s % 2 ? ctx->wa : ctx->un, s % 2 ? ctx->un : ctx->wa, dt, ct(s));
+  if (rc == SBP_OK && steps % 2)
+    CK(cudaMemcpyAsync(ctx->un, ctx->wa, (size_t)ctx->dofs * ctx->plane * ctx->es, cudaMemcpyDeviceToDevice,
+                       ctx->stream));
+  return rc;
+}
+
 void drop_graphs(sbp_ctx* ctx) {
   for (auto& kv : ctx->graphs) cudaGraphExecDestroy(kv.second);
   ctx->graphs.clear();
@@ -469,9 +514,7 @@ int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt, double* t) {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     const long long before = ctx->launches;
-    int rc = SBP_OK;
-    for (long long s = 0; s < steps && rc == SBP_OK; s++)
-      rc = enqueue_step<T>(ctx, 0.0, dt, ctx->ct_tab ? ctx->ct_tab + 3 * s : nullptr);
+    const int rc = enqueue_steps<T>(ctx, steps, dt);
     cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
     ctx->launches = before;  // captured, not yet run
     if (rc) {
@@ -496,7 +539,7 @@ int run_chunk_graph(sbp_ctx* ctx, long long steps, double dt, double* t) {
     CK(cudaMemcpyAsync(ctx->ct_tab, h, 3 * steps * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
   }
   CK(cudaGraphLaunch(it->second, ctx->stream));
-  ctx->launches += 4 * steps;
+  ctx->launches += use_step(ctx) ? steps : 4 * steps;
   return SBP_OK;
 }
 
@@ -989,6 +1032,8 @@ int sbp_create(const sbp_desc* desc, sbp_ctx** out) {
       delete ctx;
       return SBP_ERR_CUDA;
     }
+    if (use_step(ctx) && (e = configure_step(d.order, wave_kind(ctx))) != cudaSuccess)
+      return cuda_fail("configure step kernel", e);
     // shared-memory opt-in of the stage kernels, done here (not under stream capture)
     e = ctx->fp32 ? configure_wave<float>(d.order, wave_kind(ctx)) : configure_wave<double>(d.order, wave_kind(ctx));
     if (e != cudaSuccess) return cuda_fail("configure stage kernels", e);

@@ -12,6 +12,8 @@
 #define LAUNCH_WAVE CAT(launch_wave_o, SBP_ORDER)
 #define CONFIGURE_WAVE CAT(configure_wave_o, SBP_ORDER)
 #define LAUNCH_CELL CAT(launch_cell_o, SBP_ORDER)
+#define LAUNCH_STEP CAT(launch_step_o, SBP_ORDER)
+#define CONFIGURE_STEP CAT(configure_step_o, SBP_ORDER)
 
 namespace sbp {
 
@@ -114,7 +116,52 @@ cudaError_t cell_kind(int stage, bool aos, const WaveParams<T>& prm, cudaStream_
   return cudaErrorInvalidValue;
 }
 
+template <int KIND, int TC>
+constexpr int step_smem() {
+  return WaveStep<SBP_ORDER, TC>::smem(KIND == WK_VAR ? 2 : (KIND == WK_MMS ? 3 : 0));
+}
+
+template <int KIND, int TC>
+cudaError_t step_one(const WaveParams<double>& prm, const WaveStepCoef& cf, cudaStream_t s) {
+  const dim3 grid((prm.nx + TC - 1) / TC, (prm.ny + TC - 1) / TC);
+  return launch_overlapped(wave_step_kernel<SBP_ORDER, KIND, TC>, grid, kStepThreads, step_smem<KIND, TC>(), s, prm, cf);
+}
+
+// The smaller cell where its CTAs fit the SMs at once, else the larger.
+template <int KIND>
+cudaError_t step_kind(const WaveParams<double>& prm, const WaveStepCoef& cf, cudaStream_t s) {
+  const long long small = (long long)((prm.nx + kStepSmall - 1) / kStepSmall) * ((prm.ny + kStepSmall - 1) / kStepSmall);
+  if (small <= device_sm_count()) return step_one<KIND, kStepSmall>(prm, cf, s);
+  return step_one<KIND, step_large(SBP_ORDER)>(prm, cf, s);
+}
+
+template <int KIND, int TC> cudaError_t step_configure_one() {
+  return cudaFuncSetAttribute(wave_step_kernel<SBP_ORDER, KIND, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              step_smem<KIND, TC>());
+}
+template <int KIND> cudaError_t step_configure() {
+  const cudaError_t e = step_configure_one<KIND, kStepSmall>();
+  return e != cudaSuccess ? e : step_configure_one<KIND, step_large(SBP_ORDER)>();
+}
+
 }  // namespace
+
+cudaError_t LAUNCH_STEP(int kind, const WaveParams<double>& prm, const WaveStepCoef& cf, cudaStream_t s) {
+  switch (kind) {
+    case WK_HOM: return step_kind<WK_HOM>(prm, cf, s);
+    case WK_VAR: return step_kind<WK_VAR>(prm, cf, s);
+    case WK_MMS: return step_kind<WK_MMS>(prm, cf, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+cudaError_t CONFIGURE_STEP(int kind) {
+  switch (kind) {
+    case WK_HOM: return step_configure<WK_HOM>();
+    case WK_VAR: return step_configure<WK_VAR>();
+    case WK_MMS: return step_configure<WK_MMS>();
+    default: return cudaErrorInvalidValue;
+  }
+}
 
 template <>
 cudaError_t LAUNCH_CELL<double>(int kind, int stage, bool aos, const WaveParams<double>& prm, cudaStream_t s) {
