@@ -111,6 +111,7 @@ template <typename T, int ORD, int KIND>
 cudaError_t steps_one(const LineParams<T>& prm, double dt, int steps, cudaStream_t s) {
   const int chunk = line_chunk(prm.nx), ctas = (prm.nx + chunk - 1) / chunk;
   int threads = (chunk + 8 * (OpShape<ORD>::W / 2) + 31) / 32 * 32;
+  if (sizeof(T) == 8) threads += ctas == 1 ? 64 : 32;  // the closure points' warps
   if (threads > 512) threads = 512;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(ctas);

@@ -9,11 +9,11 @@
 // barrier ends the step. The state is double-buffered: a CTA may write its neighbour's next
 // halo while the neighbour still reads the current one.
 // Measured, us per step, stages launched one by one -> this: FP64 advection order 4, 201
-// points 9.4 -> 3.3, 1601 9.0 -> 3.9, 6401 10.2 -> 8.7; reflection 201 13.6 -> 4.9; FP32
-// advection 201 7.8 -> 2.1. What bounds it: a warp's FP64 instruction takes 64 clocks, so a
-// stage's chain of about eight is 0.25 us, and the cluster barrier ends each step.
-// The operations of a point are those of line_point (line_kernels.cuh), in its order, so FP32
-// states get the same bits from both.
+// points 9.4 -> 3.0, 1601 9.0 -> 3.1, 6401 10.2 -> 6.5; reflection 201 13.6 -> 4.3; FP32
+// advection 201 7.8 -> 2.1. What bounds it: a warp's FP64 instruction takes 64 clocks, and the
+// cluster barrier ends each step. FP64 interior stencils are integer sums (with FP64 taps: 201
+// points 3.3, 6401 8.7).
+// FP32: the operations of line_point (line_kernels.cuh), in its order, the same bits.
 #pragma once
 
 #include <cooperative_groups.h>
@@ -36,6 +36,34 @@ template <typename T, int ORD, int KIND> struct LineSteps {
   static size_t smem(int chunk) { return sizeof(T) * NC * planes * (size_t)(chunk + 2 * H); }
 };
 
+// den times the interior stencil sum around c by integer arithmetic with the exponent of its
+// own largest value (wave2d_fixed.cuh, the finer unit): some 100 integer instructions take half
+// the time of four FP64 FMAs at 64 clocks each. False where the values leave the fixed-point
+// range.
+template <int ORD>
+__device__ __forceinline__ bool fx_local(const double* c, double& out) {
+  constexpr int R = OpShape<ORD>::W / 2;
+  unsigned m = 0;
+#pragma unroll
+  for (int k = 1; k <= R; k++) {
+    m = max(m, (unsigned)__double2hiint(c[k]) & 0x7FF00000u);
+    m = max(m, (unsigned)__double2hiint(c[-k]) & 0x7FF00000u);
+  }
+  const int emax = (int)(m >> 20);
+  long long d[R];  // v_k - v_-k
+#pragma unroll
+  for (int k = 1; k <= R; k++) {
+    const double a = c[k], b = c[-k];
+    d[k - 1] = fx_from<true>((unsigned)__double2loint(a), (unsigned)__double2hiint(a), emax) -
+               fx_from<true>((unsigned)__double2loint(b), (unsigned)__double2hiint(b), emax);
+  }
+  long long s = d[0];
+  if constexpr (ORD == 4) s = 8 * d[0] - d[1];
+  if constexpr (ORD == 6) s = 45 * d[0] - 9 * d[1] + d[2];
+  out = fx_to<true>(s, fx_base<true>(emax));
+  return emax == 0 || (emax >= 64 && emax < 2031);
+}
+
 template <typename T, int ORD, int KIND>
 __global__ void __launch_bounds__(512) line_steps_kernel(const __grid_constant__ LineParams<T> prm, const int chunk,
                                                           const int steps, const T ca1, const T ca2, const T cw1,
@@ -51,6 +79,7 @@ __global__ void __launch_bounds__(512) line_steps_kernel(const __grid_constant__
   T* const sm = reinterpret_cast<T*>(line_smem);
   const auto plane_of = [&](int p, int c) { return sm + (p * NC + c) * len; };  // u: 0, 1; w: 2, 3; acc 4; comp 5
   const int tid = threadIdx.x, nt = blockDim.x;
+  const T sig = (T)prm.fx_sig[0], sa1 = ca1 * sig, sa2 = ca2 * sig, sw1 = cw1 * sig, sw3 = cw3 * sig;
   // the closure block: from the parameters, each row that a warp's lanes read is a
   // constant-bank access of its own (order 6: 4.5 us a step against 4.1)
   __shared__ T s_cls[6][9];
@@ -62,23 +91,47 @@ __global__ void __launch_bounds__(512) line_steps_kernel(const __grid_constant__
       plane_of(0, c)[l] = in ? prm.un[c * prm.plane + i] : T(0);
       plane_of(5, c)[l] = in && prm.compensated && i >= a && i < b ? prm.comp[c * prm.plane + i] : T(0);
     }
+  // Where thread slots are. FP64: the closure points of an end this CTA owns have a warp to themselves
+  // (their rows of FP64 taps would hold up a warp of interior points), the other points follow.
+  // FP32: point after point.
+  const bool left = cta == 0, right = cta == ctas - 1;
+  const int m0 = left ? CS : base, m1 = right ? nx - CS : base + len;  // the middle points
+  const int s0 = left ? 32 : 0, s1 = s0 + ((m1 - m0 + 31) & ~31);
+  const int slots = sizeof(T) == 8 ? s1 + (right ? 32 : 0) : len;
+  const auto point_of = [&](int s) {  // the grid index of a slot, or -1
+    if constexpr (sizeof(T) == 4) return base + s;
+    if (s < s0) return s < CS ? s : -1;
+    if (s < s1) return m0 + s - s0 < m1 ? m0 + s - s0 : -1;
+    return s - s1 < CS ? nx - CS + s - s1 : -1;
+  };
   cluster.sync();  // every CTA has read its halo from global memory and may be written to
 
   // stage rk of this CTA's points and (4 - rk) R halo points per side, from plane `in` to `out`
   const auto stage = [&](auto rk_, int u, int in, int out) {
     constexpr int rk = decltype(rk_)::value;
     const int lo = a - (4 - rk) * R > 0 ? a - (4 - rk) * R : 0, hi = b + (4 - rk) * R < nx ? b + (4 - rk) * R : nx;
-    const T ca = (rk == 1 || rk == 4) ? ca1 : ca2, cw = rk == 3 ? cw3 : cw1;
-    for (int l = tid; l < len; l += nt) {  // a point keeps its thread through the stages
-      const int i = base + l;
+    for (int s = tid; s < slots; s += nt) {  // a point keeps its thread through the stages
+      const int i = point_of(s), l = i - base;
       if (i < lo || i >= hi) continue;
+      T ca = (rk == 1 || rk == 4) ? ca1 : ca2, cw = rk == 3 ? cw3 : cw1;
       const auto d1 = [&](int c) {
         const T* line = plane_of(in, c) - base;
         const auto ld = [&](int q) { return line[q]; };
         return (i >= CS && i < nx - CS) ? taps_by<T, ORD>(ld, i, prm.dx.taps) : closure_by<T, ORD>(ld, nx, i, s_cls);
       };
       T k[NC];
-      if constexpr (KIND == LK_ADV1D) {
+      bool scaled = false;  // FP64 interior: k in units of fx_sig, folded into ca and cw
+      if constexpr (sizeof(T) == 8) {
+        if (i >= CS && i < nx - CS) {
+          scaled = fx_local<ORD>(plane_of(in, 0) + l, k[NC - 1]);
+          if constexpr (NC == 2) scaled = fx_local<ORD>(plane_of(in, 1) + l, k[0]) && scaled;
+        }
+      }
+      if (scaled) {
+        ca = (rk == 1 || rk == 4) ? sa1 : sa2, cw = rk == 3 ? sw3 : sw1;
+        if constexpr (KIND == LK_ADV1D)
+          if (prm.va) k[0] = -prm.va[i] * k[0];
+      } else if constexpr (KIND == LK_ADV1D) {
         k[0] = d1(0);
         if (prm.va) k[0] = -prm.va[i] * k[0];
         k[0] = adv1d_sat<T>(prm, i, k[0], plane_of(in, 0)[l]);

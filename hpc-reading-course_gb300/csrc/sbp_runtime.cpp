@@ -269,7 +269,7 @@ LineParams<T> line_params(sbp_ctx* ctx) {
   p.bc = 1;
   p.compensated = ctx->fp32 ? 1 : 0;
   const double den = fixed_denominator(ctx->d.order);
-  p.fx_sig[0] = ctx->va ? ctx->hix / den : -a * ctx->hix / den;
+  p.fx_sig[0] = (ctx->va || ctx->d.problem == SBP_REFLECTION_1D) ? ctx->hix / den : -a * ctx->hix / den;
   p.fx_sig[1] = ctx->va ? ctx->hiy / den : -b * ctx->hiy / den;
   p.err = ctx->err;
   return p;
