@@ -170,11 +170,18 @@ struct TcConv {
 // tcgen05.commit, and commits each pixel tile into one of two accumulators (32 columns
 // each); warps 2-5 read an accumulator (warp w: lanes 32 (w % 4) ..), release it, and add
 // bias, apply ReLU and store while the next tile accumulates in the other. Bounded waits.
-template <int CIN, int COUT, bool RELU, bool OUT_F32>
+//
+// MASK (input gradients): the ReLU backward pass through `mask`, the post-activation
+// values the output is the gradient of -- y is zero where the mask is not above zero.
+// Each thread fetches its pixel's 64 mask bytes before it waits for the accumulator, so
+// the fetch hides behind the MMAs; a separate pass reads and writes the gradient once
+// more (8 x 258 x 257: 34 MB of mask instead of 102 MB).
+template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::CTAS)
     conv3x3_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
-                      const float* __restrict__ bias, void* __restrict__ y, int B, int H, int W, int tw, int th,
-                      int* err) {
+                      const float* __restrict__ bias, const bf16* __restrict__ mask, void* __restrict__ y, int B, int H,
+                      int W, int tw, int th, int* err) {
+  static_assert(!MASK || (!RELU && !OUT_F32), "the mask is the input gradient's, in BF16");
   using L = TcConv<CIN, COUT>;
   constexpr int NS = L::NS;
   extern __shared__ unsigned char smem_raw[];
@@ -266,6 +273,16 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
     int it = 0;
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
       const int buf = it & 1;
+      const int w0 = (tile % ntw) * tw, h0 = ((tile / ntw) % nth) * th, b = tile / (ntw * nth);
+      const int m = 32 * q + lane;  // this thread's accumulator lane: pixel m of the tile
+      const int hh = h0 + m / tw, ww = w0 + m % tw;
+      const bool inside = hh < H && ww < W;
+      const long long p = ((long long)b * H + hh) * W + ww;
+      uint4 mk[MASK ? COUT / 8 : 1];
+      if (MASK && inside) {
+#pragma unroll
+        for (int j = 0; j < COUT / 8; j++) mk[j] = __ldg(reinterpret_cast<const uint4*>(mask + p * COUT) + j);
+      }
       if (!mbar_wait_bounded(&accfull[buf], (it / 2) & 1)) {
         if (lane == 0) atomicOr(err, 1);
         break;
@@ -279,16 +296,18 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&accempty[buf]);  // the accumulator may take the tile after next
-      const int w0 = (tile % ntw) * tw, h0 = ((tile / ntw) % nth) * th, b = tile / (ntw * nth);
-      const int m = 32 * q + lane;  // this thread's accumulator lane: pixel m of the tile
-      const int hh = h0 + m / tw, ww = w0 + m % tw;
-      if (hh >= H || ww >= W) continue;
-      const long long p = ((long long)b * H + hh) * W + ww;
+      if (!inside) continue;
       float v[COUT];
 #pragma unroll
       for (int j = 0; j < COUT; j++) {
         v[j] = __uint_as_float(r[j]) + bv[j];
         if (RELU) v[j] = fmaxf(v[j], 0.f);
+        if (MASK) {
+          const uint4 u = mk[j / 8];
+          const uint32_t w = (j / 2) % 4 == 0 ? u.x : (j / 2) % 4 == 1 ? u.y : (j / 2) % 4 == 2 ? u.z : u.w;
+          // the BF16 value as FP32: its bits are the upper half
+          if (!(__uint_as_float(j & 1 ? w & 0xffff0000u : w << 16) > 0.f)) v[j] = 0.f;
+        }
       }
       if (OUT_F32) {
         float4* yp = reinterpret_cast<float4*>(static_cast<float*>(y) + p * COUT);
@@ -464,12 +483,6 @@ __global__ void bias_grad_kernel(const bf16* __restrict__ dy, float* __restrict_
     atomicAdd(&sh[e % COUT], __bfloat162float(dy[e]));
   __syncthreads();
   for (int n = threadIdx.x; n < COUT; n += blockDim.x) atomicAdd(&db[n], sh[n]);
-}
-
-// d[e] = (y[e] > 0) ? d[e] : 0   (ReLU backward through the post-activation output y)
-__global__ void relu_back_kernel(bf16* __restrict__ d, const bf16* __restrict__ y, long long n) {
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
-    if (!(__bfloat162float(y[e]) > 0.f)) d[e] = __float2bfloat16(0.f);
 }
 
 // wT[c][tap][n] = w[n][8 - tap][c]: the weights of the input-gradient convolution.
@@ -734,23 +747,23 @@ cudaError_t encode_conv_maps(const sbp_cnn* c, const bf16* x, const bf16* w, int
   return cudaSuccess;
 }
 
-template <int CIN, int COUT, bool RELU, bool OUT_F32>
+template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 cudaError_t configure_tc() {
-  return cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              TcConv<CIN, COUT>::SMEM);
+  return cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, TcConv<CIN, COUT>::SMEM);
 }
 
-template <int CIN, int COUT, bool RELU, bool OUT_F32>
-cudaError_t launch_tc(const bf16* x, const bf16* w, const float* bias, void* y, const sbp_cnn* c, int batch,
-                      cudaStream_t s) {
+template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
+cudaError_t launch_tc(const bf16* x, const bf16* w, const float* bias, const bf16* mask, void* y, const sbp_cnn* c,
+                      int batch, cudaStream_t s) {
   CUtensorMap xm, wm;
   cudaError_t e = encode_conv_maps(c, x, w, CIN, COUT, batch, &xm, &wm);
   if (e != cudaSuccess) return e;
   const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
   const long long slots = (long long)TcConv<CIN, COUT>::CTAS * c->nsm;  // persistent: every CTA resident
   const unsigned grid = (unsigned)(tiles < slots ? tiles : slots);
-  conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32><<<grid, TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::SMEM, s>>>(
-      xm, wm, bias, y, batch, c->H, c->W, c->tw, c->th, c->err);
+  conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK><<<grid, TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::SMEM, s>>>(
+      xm, wm, bias, mask, y, batch, c->H, c->W, c->tw, c->th, c->err);
   return cudaGetLastError();
 }
 
@@ -763,23 +776,24 @@ cudaError_t configure_wgrad_tc() {
 // Shared-memory opt-in of the tensor-core convolutions (outside stream capture).
 cudaError_t configure_convs() {
   cudaError_t e;
-  if ((e = configure_tc<32, 32, true, false>()) != cudaSuccess) return e;
-  if ((e = configure_tc<32, 16, false, true>()) != cudaSuccess) return e;
-  if ((e = configure_tc<32, 32, false, false>()) != cudaSuccess) return e;
-  if ((e = configure_tc<16, 32, false, false>()) != cudaSuccess) return e;
+  if ((e = configure_tc<32, 32, true, false, false>()) != cudaSuccess) return e;
+  if ((e = configure_tc<32, 16, false, true, false>()) != cudaSuccess) return e;
+  if ((e = configure_tc<32, 32, false, false, true>()) != cudaSuccess) return e;
+  if ((e = configure_tc<16, 32, false, false, true>()) != cudaSuccess) return e;
   if ((e = configure_wgrad_tc<32>()) != cudaSuccess) return e;
   return configure_wgrad_tc<16>();
 }
 
-// Launch one conv of layer l (forward) or its input-gradient conv.
+// Launch one conv of layer l (forward), or its input-gradient conv with the ReLU
+// backward pass through the layer's input.
 cudaError_t conv_fwd(int l, const bf16* x, void* y, const sbp_cnn* c, int batch, cudaStream_t s) {
-  if (l < kLayers - 1) return launch_tc<32, 32, true, false>(x, c->wb[l], c->bias[l], y, c, batch, s);
-  return launch_tc<32, 16, false, true>(x, c->wb[l], c->bias[l], y, c, batch, s);
+  if (l < kLayers - 1) return launch_tc<32, 32, true, false, false>(x, c->wb[l], c->bias[l], nullptr, y, c, batch, s);
+  return launch_tc<32, 16, false, true, false>(x, c->wb[l], c->bias[l], nullptr, y, c, batch, s);
 }
 
 cudaError_t conv_dgrad(int l, const bf16* dy, bf16* dx, const sbp_cnn* c, int batch, cudaStream_t s) {
-  if (l == kLayers - 1) return launch_tc<16, 32, false, false>(dy, c->wT[l], nullptr, dx, c, batch, s);
-  return launch_tc<32, 32, false, false>(dy, c->wT[l], nullptr, dx, c, batch, s);
+  if (l == kLayers - 1) return launch_tc<16, 32, false, false, true>(dy, c->wT[l], nullptr, c->act[l], dx, c, batch, s);
+  return launch_tc<32, 32, false, false, true>(dy, c->wT[l], nullptr, c->act[l], dx, c, batch, s);
 }
 
 // dw += the weight gradient of layer l (x: its input, 32 channels; dy: its output gradient).
@@ -1039,8 +1053,7 @@ static int backward(sbp_cnn* c, const float* x, const float* target, int batch, 
     }
     if (l == 0) break;
     CCK(conv_dgrad(l, dcur, dnext, c, batch, c->stream));
-    relu_back_kernel<<<blocks_for(P * kCin[l], 256), 256, 0, c->stream>>>(dnext, c->act[l], P * kCin[l]);
-    c->launches += 2;
+    c->launches++;
     bf16* tmp = dcur;
     dcur = dnext;
     dnext = tmp;
