@@ -20,6 +20,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -341,8 +342,8 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
 // and 5-8 (whose last quarter, tap 8, is the one kept) -- cover the nine taps with
 // M = 128, N = COUT, eight K steps of 16 pixels each. The accumulators (3 x COUT
 // tensor-memory columns) sum over every tile the CTA takes; at the end the four
-// epilogue warps write them to the CTA's slice of dw_part, which wgrad_reduce_kernel
-// then adds to dw in CTA order (the same bits on every run).
+// epilogue warps write them to the CTA's slice of the layer's part of dw_part, which
+// weight_step_kernel adds up in CTA order (the same bits on every run).
 template <int COUT>
 struct TcWgrad {
   static_assert(COUT == 16 || COUT == 32, "output channels: the MMA's N");
@@ -465,15 +466,6 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
   }
 }
 
-// dw[e] += sum over the weight-gradient CTAs of their partial sums, in CTA order.
-__global__ void wgrad_reduce_kernel(const float* __restrict__ part, float* __restrict__ dw, int n, int ctas) {
-  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int c = 0; c < ctas; c++) s += part[(long long)c * n + e];
-    dw[e] += s;
-  }
-}
-
 template <int COUT>
 __global__ void bias_grad_kernel(const bf16* __restrict__ dy, float* __restrict__ db, long long P) {
   __shared__ float sh[COUT];
@@ -536,20 +528,66 @@ __global__ void mse_kernel(const float* __restrict__ out16, const float* __restr
   if (threadIdx.x == 0) atomicAdd(loss, sh[0]);
 }
 
-// Adam on FP32 master parameters; writes the BF16 copy used by the kernels.
-__global__ void adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                            const float* __restrict__ g, bf16* __restrict__ p16, int n, float lr, float b1, float b2,
-                            float eps, float c1, float c2) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const float gg = g[e];
-  const float mm = b1 * m[e] + (1.f - b1) * gg;
-  const float vv = b2 * v[e] + (1.f - b2) * gg * gg;
-  m[e] = mm;
-  v[e] = vv;
+// One layer's weights and what the training step keeps beside them.
+struct LayerWeights {
+  const float* part;  // the weight-gradient CTAs' partial sums [ctas][n]
+  float *g, *p, *m, *v;
+  bf16 *p16, *pT;     // the BF16 copy and the flipped, transposed one
+  int n, cin, cout;
+};
+
+struct AllWeights {
+  LayerWeights layer[kLayers];
+};
+
+// Volatile, so that a run of them stays ahead of the additions that use them.
+__device__ __forceinline__ float ld_early(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Every layer's weight gradient g[e] = sum over the weight-gradient CTAs of their partial
+// sums, in CTA order (the same bits on every run), and with ADAM the step on the FP32
+// master weights and their two BF16 copies, which the kernels read. With ADAM nothing is
+// changed if a tensor-core kernel set *err.
+// Bound by the latency of the loads: a thread's chain is `ctas` additions, so the loads
+// are issued UN at a time ahead of them. One launch for the four layers: blockIdx.y.
+// (One B x H x W = 8 x 258 x 257 step, 152 CTAs: a reduction per layer with one load per
+// addition took 4 x 17.5 us, the Adam, copy and transpose launches 4 x 9.3 us.)
+template <bool ADAM>
+__global__ void __launch_bounds__(128) weight_step_kernel(const __grid_constant__ AllWeights a, int ctas, float lr,
+                                                          float b1, float b2, float eps, float c1, float c2,
+                                                          const int* __restrict__ err) {
+  constexpr int UN = 38;
+  const LayerWeights& w = a.layer[blockIdx.y];
+  const int e = blockIdx.x * blockDim.x + threadIdx.x, n = w.n;
+  if (e >= n || (ADAM && *err)) return;
+  float s = 0.f;
+  const float* part = w.part + e;
+  int c = 0;
+  for (; c + UN <= ctas; c += UN) {
+    float t[UN];
+#pragma unroll
+    for (int k = 0; k < UN; k++) t[k] = ld_early(part + (long long)(c + k) * n);
+#pragma unroll
+    for (int k = 0; k < UN; k++) s += t[k];
+  }
+  for (; c < ctas; c++) s += part[(long long)c * n];
+  const float gg = 0.f + s;
+  w.g[e] = gg;
+  if (!ADAM) return;
+  const float mm = b1 * w.m[e] + (1.f - b1) * gg;
+  const float vv = b2 * w.v[e] + (1.f - b2) * gg * gg;
+  w.m[e] = mm;
+  w.v[e] = vv;
   const float upd = lr * (mm / c1) / (sqrtf(vv / c2) + eps);
-  p[e] -= upd;
-  if (p16) p16[e] = __float2bfloat16(p[e]);
+  const float p = w.p[e] - upd;
+  w.p[e] = p;
+  const bf16 h = __float2bfloat16(p);
+  w.p16[e] = h;
+  const int ci = e % w.cin, tap = (e / w.cin) % 9, co = e / (9 * w.cin);
+  w.pT[((long long)ci * 9 + (8 - tap)) * w.cout + co] = h;
 }
 
 __global__ void f32_to_bf16_kernel(const float* __restrict__ a, bf16* __restrict__ b, int n) {
@@ -670,7 +708,7 @@ struct sbp_cnn {
   int* err = nullptr;        // the tensor-core convolutions' error word (a bounded wait ran out)
   int tw = 0, th = 0;        // their pixel tile: th rows of tw pixels, th * tw = 128
   int nsm = 1;               // SMs: the persistent convolutions' grid
-  float* dw_part = nullptr;  // the weight gradient's per-CTA sums ([nsm][32 * 9 * 32])
+  float* dw_part[kLayers] = {};  // the weight gradients' per-CTA sums ([nsm][wcount(l)])
   long long launches = 0;
   std::string msg;
 };
@@ -697,11 +735,11 @@ long long wcount(int l) { return (long long)kCout[l] * 9 * kCin[l]; }
 void cnn_release(sbp_cnn* c) {
   for (int l = 0; l < kLayers; l++) {
     void* ps[] = {c->wm[l], c->wb[l], c->wT[l], c->bias[l], c->mw[l], c->vw[l], c->mbias[l], c->vbias[l],
-                  c->gw[l], c->gb[l], c->act[l]};
+                  c->gw[l], c->gb[l], c->act[l], c->dw_part[l]};
     for (void* p : ps)
       if (p) cudaFree(p);
   }
-  void* ps[] = {c->dact, c->dact2, c->out16, c->loss, c->err, c->dw_part};
+  void* ps[] = {c->dact, c->dact2, c->out16, c->loss, c->err};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -796,8 +834,14 @@ cudaError_t conv_dgrad(int l, const bf16* dy, bf16* dx, const sbp_cnn* c, int ba
   return launch_tc<32, 32, false, false, true>(dy, c->wT[l], nullptr, c->act[l], dx, c, batch, s);
 }
 
-// dw += the weight gradient of layer l (x: its input, 32 channels; dy: its output gradient).
-cudaError_t conv_wgrad(int l, const bf16* x, const bf16* dy, float* dw, const sbp_cnn* c, int batch, cudaStream_t s) {
+// CTAs of the weight gradients: each leaves one partial sum.
+unsigned wgrad_ctas(const sbp_cnn* c, int batch) {
+  const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
+  return (unsigned)(tiles < c->nsm ? tiles : c->nsm);
+}
+
+// Partial sums of the weight gradient of layer l (x: its input, 32 channels; dy: its output gradient).
+cudaError_t conv_wgrad(int l, const bf16* x, const bf16* dy, const sbp_cnn* c, int batch, cudaStream_t s) {
   CUtensorMap xm, dym, unused;
   const int cout = kCout[l];
   // x: 32-channel tap tiles; dy: one unshifted tile of cout channels (its map from the same
@@ -805,17 +849,28 @@ cudaError_t conv_wgrad(int l, const bf16* x, const bf16* dy, float* dw, const sb
   cudaError_t e = encode_conv_maps(c, x, c->wb[l], 32, cout, batch, &xm, &unused);
   if (e == cudaSuccess) e = encode_conv_maps(c, dy, c->wb[l], cout, cout, batch, &dym, &unused);
   if (e != cudaSuccess) return e;
-  const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
-  const unsigned grid = (unsigned)(tiles < c->nsm ? tiles : c->nsm);
+  const unsigned grid = wgrad_ctas(c, batch);
   if (cout == 32)
     conv3x3_wgrad_tc_kernel<32><<<grid, TcWgrad<32>::THREADS, TcWgrad<32>::SMEM, s>>>(
-        xm, dym, c->dw_part, batch, c->H, c->W, c->tw, c->th, c->err);
+        xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th, c->err);
   else
     conv3x3_wgrad_tc_kernel<16><<<grid, TcWgrad<16>::THREADS, TcWgrad<16>::SMEM, s>>>(
-        xm, dym, c->dw_part, batch, c->H, c->W, c->tw, c->th, c->err);
-  const int n = (int)wcount(l);
-  wgrad_reduce_kernel<<<(n + 255) / 256, 256, 0, s>>>(c->dw_part, dw, n, (int)grid);
+        xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th, c->err);
   return cudaGetLastError();
+}
+
+AllWeights all_weights(const sbp_cnn* c) {
+  AllWeights a;
+  for (int l = 0; l < kLayers; l++)
+    a.layer[l] = LayerWeights{c->dw_part[l], c->gw[l], c->wm[l], c->mw[l], c->vw[l], c->wb[l], c->wT[l],
+                              (int)wcount(l), kCin[l], kCout[l]};
+  return a;
+}
+
+inline dim3 weight_step_grid() {
+  long long n = 0;
+  for (int l = 0; l < kLayers; l++) n = std::max(n, wcount(l));
+  return dim3((unsigned)((n + 127) / 128), kLayers);
 }
 
 cudaError_t bias_grad(int l, const bf16* dy, float* db, int batch, const sbp_cnn* c, cudaStream_t s) {
@@ -918,8 +973,9 @@ int sbp_cnn_create(int height, int width, int max_batch, int device, void* strea
   if (configure_convs() != cudaSuccess) return bad("cudaFuncSetAttribute(convolutions)");
   if (cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || c->nsm < 1)
     return bad("cudaDeviceGetAttribute(SMs)");
-  if (cudaMalloc(&c->dw_part, (size_t)c->nsm * 32 * 9 * 32 * sizeof(float)) != cudaSuccess)
-    return bad("cudaMalloc(weight-gradient partial sums)");
+  for (int l = 0; l < kLayers; l++)
+    if (cudaMalloc(&c->dw_part[l], (size_t)c->nsm * wcount(l) * sizeof(float)) != cudaSuccess)
+      return bad("cudaMalloc(weight-gradient sums)");
   if (!encode_fn()) return bad("cuTensorMapEncodeTiled is not available from the driver");
   // a network that failed its initialisation is released, not handed out
   const int rc = sbp_cnn_init(c, 1234);
@@ -1030,24 +1086,23 @@ int sbp_cnn_forward(sbp_cnn* c, const float* x, int batch, float* out) {
 // Gradients of the mean squared error of network(x) against target (both device, NHWC FP32,
 // 4 and 3 channels), without updating the parameters; written as one FP32 vector in the
 // layout of sbp_cnn_get_params (host `grad`, may be NULL). Returns the loss in *loss.
-// bias_grads: also the biases' gradients (the training step leaves biases untrained and skips them).
-static int backward(sbp_cnn* c, const float* x, const float* target, int batch, float* loss, bool bias_grads) {
+// lr > 0: the training step, which updates the weights (biases stay untrained, their gradients are skipped).
+static int backward(sbp_cnn* c, const float* x, const float* target, int batch, float* loss, float lr) {
+  const bool train = lr > 0;
   const long long P = (long long)batch * c->H * c->W;
   int rc = run_forward(c, x, batch);
   if (rc) return rc;
   CCK(cudaMemsetAsync(c->loss, 0, 4, c->stream));
   mse_kernel<<<blocks_for(P * 16, 256), 256, 0, c->stream>>>(c->out16, target, c->dact, c->loss, P);
   c->launches++;
-  for (int l = 0; l < kLayers; l++) {
-    CCK(cudaMemsetAsync(c->gw[l], 0, wcount(l) * 4, c->stream));
-    CCK(cudaMemsetAsync(c->gb[l], 0, kCout[l] * 4, c->stream));
-  }
+  if (!train)
+    for (int l = 0; l < kLayers; l++) CCK(cudaMemsetAsync(c->gb[l], 0, kCout[l] * 4, c->stream));
   bf16* dcur = c->dact;   // gradient w.r.t. the output of layer l (pre-activation once masked)
   bf16* dnext = c->dact2;
   for (int l = kLayers - 1; l >= 0; l--) {
-    CCK(conv_wgrad(l, c->act[l], dcur, c->gw[l], c, batch, c->stream));
-    c->launches += 2;  // weight gradient and its reduction
-    if (bias_grads) {
+    CCK(conv_wgrad(l, c->act[l], dcur, c, batch, c->stream));
+    c->launches++;
+    if (!train) {
       CCK(bias_grad(l, dcur, c->gb[l], batch, c, c->stream));
       c->launches++;
     }
@@ -1058,6 +1113,19 @@ static int backward(sbp_cnn* c, const float* x, const float* target, int batch, 
     dcur = dnext;
     dnext = tmp;
   }
+  const AllWeights a = all_weights(c);
+  const int ctas = (int)wgrad_ctas(c, batch);
+  if (train) {
+    const float b1 = 0.9f, b2 = 0.999f, t = (float)(c->step + 1);
+    const float c1 = 1.f - std::pow(b1, t), c2 = 1.f - std::pow(b2, t);
+    // padded channels stay zero: their gradients are zero (zero inputs / zero targets) and
+    // Adam leaves zero-gradient entries unchanged.
+    weight_step_kernel<true><<<weight_step_grid(), 128, 0, c->stream>>>(a, ctas, lr, b1, b2, 1e-8f, c1, c2, c->err);
+  } else {
+    weight_step_kernel<false><<<weight_step_grid(), 128, 0, c->stream>>>(a, ctas, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, c->err);
+  }
+  CCK(cudaGetLastError());
+  c->launches++;
   float h = 0;
   int e = 0;
   CCK(cudaMemcpyAsync(&h, c->loss, 4, cudaMemcpyDeviceToHost, c->stream));
@@ -1067,6 +1135,7 @@ static int backward(sbp_cnn* c, const float* x, const float* target, int batch, 
     CCK(cudaMemsetAsync(c->err, 0, 4, c->stream));
     return cfail(c, SBP_ERR_DEVICE, "a tensor-core convolution's wait for its tiles ran out");
   }
+  if (train) c->step++;
   if (loss) *loss = h / (float)(P * kOutReal);
   return SBP_OK;
 }
@@ -1076,7 +1145,7 @@ int sbp_cnn_gradients(sbp_cnn* c, const float* x, const float* target, int batch
   if (!c || !x || !target || batch < 1 || batch > c->maxB) return SBP_ERR_INVALID;
   if (grad && n != sbp_cnn_param_count()) return SBP_ERR_INVALID;
   CCK(cudaSetDevice(c->device));
-  int rc = backward(c, x, target, batch, loss, true);
+  int rc = backward(c, x, target, batch, loss, 0.f);
   if (rc || !grad) return rc;
   long long o = 0;
   for (int l = 0; l < kLayers; l++) {
@@ -1095,23 +1164,7 @@ int sbp_cnn_gradients(sbp_cnn* c, const float* x, const float* target, int batch
 int sbp_cnn_train_step(sbp_cnn* c, const float* x, const float* target, int batch, float lr, float* loss) {
   if (!c || !x || !target || batch < 1 || batch > c->maxB || !(lr > 0)) return SBP_ERR_INVALID;
   CCK(cudaSetDevice(c->device));
-  int rc = backward(c, x, target, batch, loss, false);
-  if (rc) return rc;
-  c->step++;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = 1.f - std::pow(b1, (float)c->step), c2 = 1.f - std::pow(b2, (float)c->step);
-  for (int l = 0; l < kLayers; l++) {
-    const int n = (int)wcount(l);
-    adam_kernel<<<(n + 255) / 256, 256, 0, c->stream>>>(c->wm[l], c->mw[l], c->vw[l], c->gw[l], nullptr, n, lr, b1, b2,
-                                                        1e-8f, c1, c2);
-    c->launches += 1;
-  }
-  // padded channels stay zero: their gradients are zero (zero inputs / zero targets) and
-  // Adam leaves zero-gradient entries unchanged.
-  rc = refresh_weights(c);
-  if (rc) return rc;
-  CCK(cudaStreamSynchronize(c->stream));
-  return SBP_OK;
+  return backward(c, x, target, batch, loss, lr);
 }
 
 int sbp_cnn_features(const double* state, const double* rho, const double* K, int nx, int ny, int block_rows,

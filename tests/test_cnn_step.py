@@ -1,0 +1,59 @@
+"""The training step's one launch for every layer (sums of the weight-gradient CTAs,
+Adam, the two BF16 copies)."""
+import numpy as np
+import pytest
+
+import cnn_oracle as N
+from test_cnn import _small_params
+
+LR = 1e-3
+
+
+def _batch(shape, seed):
+    import torch
+
+    rng = np.random.default_rng(seed)
+    x = torch.from_numpy(rng.standard_normal(shape + (N.IN_REAL,)).astype(np.float32)).cuda()
+    t = torch.from_numpy(rng.standard_normal(shape + (3,)).astype(np.float32)).cuda()
+    return x, t
+
+
+def _weights():
+    """Mask of the vector's weights (the biases are not trained)."""
+    out = []
+    for ci, co, _ in N.LAYERS:
+        out += [np.ones(co * 9 * ci, bool), np.zeros(co, bool)]
+    return np.concatenate(out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 8, 16), (1, 304, 16), (3, 104, 16), (2, 130, 257)],
+                         ids=["1-tile", "38-tiles", "39-tiles", "every-sm"])
+def test_gpu_step_is_adam_on_the_gradients(sbp, shape):
+    """One partial sum, the 38 loaded at a time, one more, and as many as the chip has SMs.
+    Two steps against FP64 Adam on the gradients that `gradients` returns for the same weights.
+    Tolerance: an update is at most lr in size and takes fewer than 16 FP32 roundings from the
+    gradient; the weight itself is rounded once more."""
+    B, H, W = shape
+    x, t = _batch(shape, 11)
+    mask = _weights()
+    with sbp.Cnn(H, W, B) as net, sbp.Cnn(H, W, B) as fresh:
+        net.set_params(_small_params(5).astype(np.float32))
+        m = v = 0.0
+        for k in (1, 2):
+            p = net.get_params().astype(np.float64)
+            loss, g = net.gradients(x.data_ptr(), t.data_ptr(), B)
+            assert np.any(g[mask])
+            assert net.train_step(x.data_ptr(), t.data_ptr(), B, LR) == pytest.approx(loss, rel=1e-5)
+            g = np.where(mask, g.astype(np.float64), 0.0)
+            b1, b2 = float(np.float32(0.9)), float(np.float32(0.999))
+            m, v = b1 * m + (1 - b1) * g, b2 * v + (1 - b2) * g * g
+            want = p - LR * (m / (1 - b1**k)) / (np.sqrt(v / (1 - b2**k)) + 1e-8)
+            got = net.get_params().astype(np.float64)
+            # 1 - b2^k is itself a difference of FP32 values near one: relative error 2^-24 / (k 1e-3)
+            tol = 2 * LR * (16 * 2.0**-24 + 2.0**-23 / 1e-3) + np.abs(p) * 2.0**-23
+            assert np.all(np.abs(got - want) <= tol), k
+        # the copies the kernels read are those of the new weights: same bits as when they are set
+        fresh.set_params(net.get_params())
+        assert np.array_equal(net.gradients(x.data_ptr(), t.data_ptr(), B)[1][mask],
+                              fresh.gradients(x.data_ptr(), t.data_ptr(), B)[1][mask])
