@@ -485,13 +485,30 @@ __global__ void flip_weights_kernel(const bf16* __restrict__ w, bf16* __restrict
   wT[e] = w[((long long)n * 9 + (8 - tap)) * cin + c];
 }
 
-// x16[p][c] = c < 24 ? bf16(x[p][c]) : 0, c < 32
-__global__ void pack_input_kernel(const float* __restrict__ x, bf16* __restrict__ x16, long long P) {
-  constexpr int CP = kCin[0];
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < P * CP; e += (long long)gridDim.x * blockDim.x) {
-    const long long p = e / CP;
-    const int c = (int)(e % CP);
-    x16[e] = __float2bfloat16(c < kInReal ? x[p * kInReal + c] : 0.f);
+// x16[p][c] = c < 24 ? bf16(x[p][c]) : 0, c < 32. Bound by memory: a thread takes eight
+// channels, one 16-byte store and, where x starts on a 16-byte boundary (VEC: rows are 96
+// bytes, so every eight channels then do), two 16-byte loads; else eight single ones.
+// (8 x 258 x 257, 85 MB: one channel per thread took 19.8 us.)
+template <bool VEC>
+__global__ void __launch_bounds__(256) pack_input_kernel(const float* __restrict__ x, bf16* __restrict__ x16, long long P) {
+  static_assert(kCin[0] == 32 && kInReal == 24, "three groups of eight channels and one of zeros");
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < P * 4; e += (long long)gridDim.x * blockDim.x) {
+    const int g = (int)(e & 3);
+    float v[8] = {};
+    if (g < 3) {
+      const float* src = x + (e >> 2) * kInReal + 8 * g;
+      if (VEC) {
+        const float4 lo = __ldg(reinterpret_cast<const float4*>(src)), hi = __ldg(reinterpret_cast<const float4*>(src) + 1);
+        v[0] = lo.x, v[1] = lo.y, v[2] = lo.z, v[3] = lo.w, v[4] = hi.x, v[5] = hi.y, v[6] = hi.z, v[7] = hi.w;
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k] = __ldg(src + k);
+      }
+    }
+    reinterpret_cast<uint4*>(x16)[e] = make_uint4(pack_pair(__float2bfloat16(v[0]), __float2bfloat16(v[1])),
+                                                  pack_pair(__float2bfloat16(v[2]), __float2bfloat16(v[3])),
+                                                  pack_pair(__float2bfloat16(v[4]), __float2bfloat16(v[5])),
+                                                  pack_pair(__float2bfloat16(v[6]), __float2bfloat16(v[7])));
   }
 }
 
@@ -503,21 +520,24 @@ __global__ void unpack_output_kernel(const float* __restrict__ out16, float* __r
 }
 
 // Mean squared error over the 3 real channels; gradient (bf16, 16 channels) and the loss sum.
+// Bound by memory: a thread takes a pixel, whose other 13 output channels it does not
+// read (8 x 258 x 257: 40 MB moved instead of 57; one channel per thread took 17.0 us).
 __global__ void mse_kernel(const float* __restrict__ out16, const float* __restrict__ target, bf16* __restrict__ d16,
                            float* __restrict__ loss, long long P) {
+  static_assert(kOutReal == 3, "the first three channels");
   __shared__ float sh[256];
   float s = 0.f;
   const float scale = 2.f / (float)(P * kOutReal);
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < P * 16; e += (long long)gridDim.x * blockDim.x) {
-    const long long p = e / 16;
-    const int c = (int)(e % 16);
-    float g = 0.f;
-    if (c < kOutReal) {
-      const float r = out16[e] - target[p * kOutReal + c];
-      s += r * r;
-      g = scale * r;
-    }
-    d16[e] = __float2bfloat16(g);
+  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
+    const float4 o = __ldg(reinterpret_cast<const float4*>(out16 + p * 16));
+    const float r0 = o.x - target[3 * p], r1 = o.y - target[3 * p + 1], r2 = o.z - target[3 * p + 2];
+    s += r0 * r0;
+    s += r1 * r1;
+    s += r2 * r2;
+    uint4* d = reinterpret_cast<uint4*>(d16 + p * 16);
+    d[0] = make_uint4(pack_pair(__float2bfloat16(scale * r0), __float2bfloat16(scale * r1)),
+                      pack_pair(__float2bfloat16(scale * r2), __float2bfloat16(0.f)), 0u, 0u);
+    d[1] = make_uint4(0u, 0u, 0u, 0u);
   }
   sh[threadIdx.x] = s;
   __syncthreads();
@@ -895,7 +915,10 @@ int refresh_weights(sbp_cnn* c) {
 
 int run_forward(sbp_cnn* c, const float* x, int batch) {
   const long long P = (long long)batch * c->H * c->W;
-  pack_input_kernel<<<blocks_for(P * kCin[0], 256), 256, 0, c->stream>>>(x, c->act[0], P);
+  if (reinterpret_cast<uintptr_t>(x) % 16 == 0)
+    pack_input_kernel<true><<<blocks_for(P * 4, 256), 256, 0, c->stream>>>(x, c->act[0], P);
+  else
+    pack_input_kernel<false><<<blocks_for(P * 4, 256), 256, 0, c->stream>>>(x, c->act[0], P);
   c->launches++;
   for (int l = 0; l < kLayers; l++) {
     void* y = (l == kLayers - 1) ? (void*)c->out16 : (void*)c->act[l + 1];
@@ -1093,7 +1116,7 @@ static int backward(sbp_cnn* c, const float* x, const float* target, int batch, 
   int rc = run_forward(c, x, batch);
   if (rc) return rc;
   CCK(cudaMemsetAsync(c->loss, 0, 4, c->stream));
-  mse_kernel<<<blocks_for(P * 16, 256), 256, 0, c->stream>>>(c->out16, target, c->dact, c->loss, P);
+  mse_kernel<<<blocks_for(P, 256), 256, 0, c->stream>>>(c->out16, target, c->dact, c->loss, P);
   c->launches++;
   if (!train)
     for (int l = 0; l < kLayers; l++) CCK(cudaMemsetAsync(c->gb[l], 0, kCout[l] * 4, c->stream));

@@ -1,5 +1,5 @@
 """The training step's one launch for every layer (sums of the weight-gradient CTAs,
-Adam, the two BF16 copies)."""
+Adam, the two BF16 copies) and the input packing where x starts off a 16-byte boundary."""
 import numpy as np
 import pytest
 
@@ -57,3 +57,20 @@ def test_gpu_step_is_adam_on_the_gradients(sbp, shape):
         fresh.set_params(net.get_params())
         assert np.array_equal(net.gradients(x.data_ptr(), t.data_ptr(), B)[1][mask],
                               fresh.gradients(x.data_ptr(), t.data_ptr(), B)[1][mask])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_gpu_unaligned_input_gives_the_same_bits(sbp, offset):
+    import torch
+
+    B, H, W = 2, 7, 19
+    x, t = _batch((B, H, W), 4)
+    shifted = torch.zeros(x.numel() + 4, dtype=torch.float32, device="cuda")
+    shifted[offset:offset + x.numel()] = x.reshape(-1)
+    out = torch.empty((2, B, H, W, 3), dtype=torch.float32, device="cuda")
+    with sbp.Cnn(H, W, B) as net:
+        net.set_params(_small_params(3).astype(np.float32))
+        net.forward(x.data_ptr(), B, out[0].data_ptr())
+        net.forward(shifted.data_ptr() + 4 * offset, B, out[1].data_ptr())
+    assert torch.any(out[0] != 0) and torch.equal(out[0], out[1])
