@@ -12,10 +12,10 @@
 //                         K = 9 taps x input channels; also computes the input
 //                         gradient (dgrad) with the spatially flipped,
 //                         transposed weights.
-//   conv3x3_wgrad_tc_kernel  weight gradient on tcgen05, K = pixels: four taps'
-//                         shifted input tiles stacked along M (MN-major operands),
+//   conv3x3_wgrad_tc_kernel  weight gradient on tcgen05, K = pixels: a column's three
+//                         vertical taps stacked along M (MN-major operands),
 //                         accumulated over all of a CTA's pixel tiles in tensor
-//                         memory; wgrad_reduce_kernel adds the CTAs' sums to dw in
+//                         memory; weight_step_kernel adds the CTAs' sums up in
 //                         CTA order (repeatable bits).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -46,17 +46,24 @@ __device__ __forceinline__ uint32_t pack_pair(bf16 lo, bf16 hi) {
   return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
+// The widest pixel tile: 32 x 4 pixels.
+constexpr int kConvMaxTw = 32;
+// A column box: 128 / tw + 2 rows of tw pixels, rounded up to whole 1024-byte units.
+__host__ __device__ constexpr int conv_box_bytes(int tw, int rowb) {
+  return ((128 / tw + 2) * tw * rowb + 1023) / 1024 * 1024;
+}
 
 // ---------------------------------------------------------------- tcgen05 convolution
 // The forward and input-gradient 3x3 convolutions on the 5th-generation tensor cores:
 // an implicit GEMM per 128-pixel tile (th x tw pixels of one image), M = 128 pixels,
-// N = COUT, K = 9 taps x CIN. TMA loads each tap's shifted input tile (a 4D box
-// {CIN, tw, th, 1} of the NHWC activations: the image border comes back as zeros)
-// and each tap's weight tile into shared memory, rows of CIN BF16 values swizzled
-// by the TMA (64-byte swizzle for 32 channels, 32-byte for 16) -- the K-major
-// layout the MMA's shared-memory descriptors describe. One thread issues
+// N = COUT, K = 9 taps x CIN. TMA loads the tile's three column boxes, one per horizontal
+// tap offset and with a row above and below the tile (a 4D box {CIN, tw, th + 2, 1} of the
+// NHWC activations: the image border comes back as zeros), and each tap's weight tile into
+// shared memory, rows of CIN BF16 values swizzled by the TMA (64-byte swizzle for 32
+// channels, 32-byte for 16) -- the K-major
+// layout the MMA's shared-memory descriptors describe. One lane issues
 // tcgen05.mma (kind::f16, BF16 inputs, FP32 accumulator in tensor memory) tap by
-// tap as the tiles land, K = 16 per instruction; tcgen05.commit signals the
+// tap once the boxes have landed, K = 16 per instruction; tcgen05.commit signals the
 // epilogue, where each warp reads its 32 accumulator lanes (pixels) with
 // tcgen05.ld, adds the bias, applies ReLU and stores. Every wait is bounded.
 
@@ -89,19 +96,34 @@ constexpr uint32_t umma_idesc_bf16(int M, int N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+// One MMA, issued by the lanes with `leader` set: one lane of a converged warp. Predicated
+// rather than branched around, so that the descriptors stay in uniform registers, which the
+// instruction reads.
+__device__ __forceinline__ void umma_bf16(uint32_t leader, uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc,
+                                          uint32_t accum) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
       "}\n" ::"r"(tmem_d),
-      "l"(a), "l"(b), "r"(idesc), "r"(accum)
+      "l"(a), "l"(b), "r"(idesc), "r"(accum), "r"(leader)
       : "memory");
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
-               : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t leader, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}\n" ::"r"(smem_addr(bar)),
+      "r"(leader)
+      : "memory");
+}
+
+// A wait of a whole converged warp: true if it ended in time for every lane.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity));
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* slot, uint32_t ncols) {
@@ -137,9 +159,9 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-// Shared-memory layout of conv3x3_tc_kernel: a ring of NS tap tiles (128 pixel rows
-// of CIN BF16), the nine taps' weight tiles (COUT rows of CIN), barriers and the
-// tensor-memory address; tiles 1024-byte aligned (whole swizzle atoms).
+// Shared-memory layout of conv3x3_tc_kernel: a ring of NS column boxes (th + 2 rows of tw
+// pixels of CIN BF16), the nine taps' weight tiles (COUT rows of CIN), barriers and the
+// tensor-memory address; boxes and tiles 1024-byte aligned (whole swizzle atoms).
 template <int CIN, int COUT>
 struct TcConv {
   static_assert(CIN == 16 || CIN == 32, "input channels: one or two K steps of 16 per tap");
@@ -147,30 +169,71 @@ struct TcConv {
   static constexpr int ROWB = CIN * 2;  // bytes per row: the swizzle span
   static constexpr uint32_t LAYOUT = CIN == 32 ? 4u : 6u;  // 64-byte / 32-byte swizzle
   static constexpr uint32_t ATOM = 8 * ROWB;
-  static constexpr int NS = 9;  // tap tiles in flight: one pixel tile per CTA, two CTAs per SM
-  static constexpr int CTAS = 2;  // resident CTAs per SM (measured at 8 x 258 x 257, forward pass:
-                                  // 0.198 ms; one CTA with 18 slots 0.310 ms, one tile per CTA
-                                  // 0.271 ms, the mma.sync form 0.471 ms)
-  static constexpr int A_BYTES = 128 * ROWB, B_BYTES = COUT * ROWB;
-  static constexpr int OFF_B = NS * A_BYTES;
-  static constexpr int OFF_BAR = OFF_B + ((9 * B_BYTES + 1023) / 1024) * 1024;
-  // full[NS], empty[NS], wbar, accfull[2], accempty[2], done; then the tensor-memory address
-  static constexpr int NBAR = 2 * NS + 6;
-  static constexpr int SMEM = OFF_BAR + 8 * NBAR + 16 + 1024;  // + alignment slack of the dynamic base
+  static constexpr int NS = 6;    // column boxes in flight: two pixel tiles per CTA
+  static constexpr int CTAS = 2;  // resident CTAs per SM (forward pass at 8 x 258 x 257: 0.138 ms; three
+                                  // CTAs with 4 boxes 0.138 ms, four with 3 boxes 0.146 ms)
+  static constexpr int B_BYTES = COUT * ROWB;
+  static constexpr int box_bytes(int tw) { return conv_box_bytes(tw, ROWB); }
+  static constexpr int off_bar() { return ((9 * B_BYTES + 1023) / 1024) * 1024; }  // after the weights
+  static constexpr int NACC = 2;  // accumulators of 32 columns (four: the same time)
+  // full[NS], empty[NS], wbar, accfull[NACC], accempty[NACC], done; then the tensor-memory address
+  static constexpr int NBAR = 2 * NS + 2 * NACC + 2;
+  static constexpr int HEAD = (off_bar() + 8 * NBAR + 16 + 1023) / 1024 * 1024;  // weights, barriers
+  static constexpr int smem(int tw) { return HEAD + NS * box_bytes(tw) + 1024; }  // + the dynamic base's slack
   static constexpr uint32_t IDESC = umma_idesc_bf16(128, COUT);
   static constexpr int THREADS = 192;  // producer, MMA issuer, four epilogue warps
-  static_assert(A_BYTES % 1024 == 0 && B_BYTES % 256 == 0, "tiles start on swizzle atoms");
-  static_assert(CTAS * (SMEM + 1024) <= 228 * 1024, "shared memory");
+  static_assert(B_BYTES % 256 == 0, "tiles start on swizzle atoms");
+  static_assert(CTAS * (smem(kConvMaxTw) + 1024) <= 228 * 1024, "shared memory");
+};
+
+// The pixel tiles of a persistent CTA: every gridDim.x-th, as tile column, tile row and
+// image, stepped by carries instead of divided out of a tile number.
+struct TileWalk {
+  int w, h, b, dw, dh, db, ntw, nth;
+
+  __device__ __forceinline__ TileWalk(int ntw_, int nth_) : ntw(ntw_), nth(nth_) {
+    w = blockIdx.x % ntw;
+    h = (blockIdx.x / ntw) % nth;
+    b = blockIdx.x / (ntw * nth);
+    dw = gridDim.x % ntw;
+    dh = (gridDim.x / ntw) % nth;
+    db = gridDim.x / (ntw * nth);
+  }
+
+  __device__ __forceinline__ void next() {
+    w += dw;
+    h += dh;
+    b += db;
+    if (w >= ntw) {
+      w -= ntw;
+      h++;
+    }
+    if (h >= nth) {
+      h -= nth;
+      b++;
+    }
+  }
 };
 
 // y[p][n] = act(bias[n] + sum_{tap,c} x[p + off(tap)][c] * w[n][tap][c]); x through xmap
-// ({CIN, W, H, B}), w through wmap ({CIN, 9, COUT}). Persistent, two CTAs per SM: a CTA
-// takes every gridDim.x-th 128-pixel tile (th rows of tw pixels). Warp roles: warp 0 loads the weights
-// once, then each tile's nine shifted tap tiles into a ring of NS slots; warp 1 (which owns
-// the tensor memory) issues each tap's MMAs as its tile lands, frees the slot with
-// tcgen05.commit, and commits each pixel tile into one of two accumulators (32 columns
-// each); warps 2-5 read an accumulator (warp w: lanes 32 (w % 4) ..), release it, and add
-// bias, apply ReLU and store while the next tile accumulates in the other. Bounded waits.
+// ({CIN, W, H, B}, box {CIN, tw, th + 2, 1}), w through wmap ({CIN, 9, COUT}). Persistent: a
+// CTA takes every gridDim.x-th 128-pixel tile (th rows of tw pixels). Warp roles: warp 0 loads
+// the weights once, then for each tile three boxes, one per horizontal tap offset, with a row
+// above and below the tile, into a ring of NS slots; warp 1 (which owns the tensor memory)
+// issues the nine taps' MMAs in tap order -- the vertical offsets are start addresses tw pixel
+// rows apart in a box, whole 8-row swizzle atoms since tw is a multiple of 8 -- frees each box
+// after its last tap with tcgen05.commit, and commits each pixel tile into one of two
+// accumulators (32 columns each); warps 2-5 read an accumulator (warp w: lanes 32 (w % 4) ..),
+// release it, and add bias, apply ReLU and store while the next tile accumulates in the other.
+// Bounded waits.
+//
+// What bounded it was the MMA warp's instructions: with the loads, the stores and eight of
+// nine MMAs left out the forward pass (8 x 258 x 257) still took 0.161 of its 0.197 ms.
+// Issued from one lane's branch, each MMA builds its two descriptors in that lane and moves
+// them to uniform registers; now the whole warp runs the loop, descriptors are a base plus
+// constants, and only the MMAs and the commits are predicated on one lane: 0.138 ms. Three
+// column boxes instead of nine shifted tiles (2.4 x fewer bytes through L2) made no
+// difference before that.
 //
 // MASK (input gradients): the ReLU backward pass through `mask`, the post-activation
 // values the output is the gradient of -- y is zero where the mask is not above zero.
@@ -185,14 +248,16 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
   static_assert(!MASK || (!RELU && !OUT_F32), "the mask is the input gradient's, in BF16");
   using L = TcConv<CIN, COUT>;
   constexpr int NS = L::NS;
+  const int box = L::box_bytes(tw), box_tx = (th + 2) * tw * L::ROWB;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  unsigned char* boxes = smem + L::HEAD;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::off_bar());
   uint64_t* empty = full + NS;
   uint64_t* wbar = empty + NS;
   uint64_t* accfull = wbar + 1;
-  uint64_t* accempty = accfull + 2;
-  uint64_t* done = accempty + 2;
+  uint64_t* accempty = accfull + L::NACC;
+  uint64_t* done = accempty + L::NACC;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int ntw = (W + tw - 1) / tw, nth = (H + th - 1) / th;
@@ -203,14 +268,14 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
       mbar_init(&empty[s], 1);
     }
     mbar_init(wbar, 1);
-    for (int s = 0; s < 2; s++) {
+    for (int s = 0; s < L::NACC; s++) {
       mbar_init(&accfull[s], 1);
       mbar_init(&accempty[s], 4);
     }
     mbar_init(done, 1);
     fence_barrier_init();
   }
-  if (warp == 1) tmem_alloc(tslot, 64);
+  if (warp == 1) tmem_alloc(tslot, 32 * L::NACC);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -219,20 +284,20 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
   if (warp == 0) {  // ---- loads
     if (lane == 0) {
       mbar_arrive_expect_tx(wbar, 9 * L::B_BYTES);
-      for (int t = 0; t < 9; t++) tma_load_3d(smem + L::OFF_B + t * L::B_BYTES, &wmap, 0, t, 0, wbar);
+      for (int t = 0; t < 9; t++) tma_load_3d(smem + t * L::B_BYTES, &wmap, 0, t, 0, wbar);
       int k = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x) {
-        const int w0 = (tile % ntw) * tw, h0 = ((tile / ntw) % nth) * th, b = tile / (ntw * nth);
-        for (int t = 0; t < 9; t++, k++) {
+      for (TileWalk t(ntw, nth); ok && t.b < B; t.next()) {
+        const int w0 = t.w * tw, h0 = t.h * th, b = t.b;
+        for (int dx = 0; dx < 3; dx++, k++) {
           const int s = k % NS;
           if (k >= NS && !mbar_wait_bounded(&empty[s], ((k / NS) - 1) & 1)) {
             atomicOr(err, 1);
             ok = false;
             break;
           }
-          mbar_arrive_expect_tx(&full[s], L::A_BYTES);
-          tma_load_4d(smem + s * L::A_BYTES, &xmap, 0, w0 + t % 3 - 1, h0 + t / 3 - 1, b, &full[s]);
+          mbar_arrive_expect_tx(&full[s], box_tx);
+          tma_load_4d(boxes + s * box, &xmap, 0, w0 + dx - 1, h0 - 1, b, &full[s]);
         }
       }
       // no copy may be in flight when the CTA exits
@@ -240,43 +305,56 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
       for (int kk = (k >= NS ? k - NS : 0); kk < k; kk++) mbar_wait_bounded(&full[kk % NS], (kk / NS) & 1);
     }
   } else if (warp == 1) {  // ---- MMAs
-    if (lane == 0) {
-      bool ok = mbar_wait_bounded(wbar, 0);
-      int k = 0, it = 0;
-      for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, it++) {
-        const int buf = it & 1;
-        if (it >= 2 && !(ok = mbar_wait_bounded(&accempty[buf], ((it / 2) - 1) & 1))) break;
-        tc_fence_after();
-        const uint32_t d = tmem + (uint32_t)(32 * buf);
-        for (int t = 0; t < 9; t++, k++) {
-          const int s = k % NS;
-          if (!(ok = mbar_wait_bounded(&full[s], (k / NS) & 1))) break;
-          tc_fence_after();
-          const uint32_t a0 = smem_addr(smem + s * L::A_BYTES), b0 = smem_addr(smem + L::OFF_B + t * L::B_BYTES);
+    const uint32_t leader = lane == 0;
+    bool ok = mbar_wait_warp(wbar, 0);
+    const uint64_t a0 = umma_smem_desc(smem_addr(boxes), L::ATOM, L::LAYOUT);
+    const uint64_t b0 = umma_smem_desc(smem_addr(smem), L::ATOM, L::LAYOUT);
+    const uint32_t box16 = (uint32_t)box >> 4, row16 = (uint32_t)(tw * L::ROWB) >> 4;  // as in descriptors
+    int slot = 0, phase = 0, it = 0;
+    for (int tile = blockIdx.x; ok && tile < ntiles; tile += gridDim.x, it++) {
+      const int buf = it % L::NACC;
+      if (it >= L::NACC && !(ok = mbar_wait_warp(&accempty[buf], ((it / L::NACC) - 1) & 1))) break;
+      tc_fence_after();
+      const uint32_t d = tmem + (uint32_t)(32 * buf);
+      int sl[3];
+      uint64_t a[3];
 #pragma unroll
-          for (int kk = 0; kk < CIN / 16; kk++)
-            umma_bf16(d, umma_smem_desc(a0 + 32 * kk, L::ATOM, L::LAYOUT),
-                      umma_smem_desc(b0 + 32 * kk, L::ATOM, L::LAYOUT), L::IDESC, (t | kk) != 0);
-          umma_commit(&empty[s]);  // the slot is free once these MMAs have read it
+      for (int dx = 0; dx < 3; dx++) {
+        sl[dx] = slot;
+        a[dx] = a0 + (uint64_t)(slot * box16);
+        if (ok) ok = mbar_wait_warp(&full[slot], phase);
+        if (++slot == NS) {
+          slot = 0;
+          phase ^= 1;
         }
-        if (!ok) break;
-        umma_commit(&accfull[buf]);
       }
-      if (!ok) atomicOr(err, 1);
-      umma_commit(done);  // every MMA issued has completed once this arrives
-      mbar_wait_bounded(done, 0);
+      if (!ok) break;
+      tc_fence_after();
+#pragma unroll
+      for (int t = 0; t < 9; t++) {
+        const int dy = t / 3, dx = t % 3;
+#pragma unroll
+        for (int kk = 0; kk < CIN / 16; kk++)  // 16 channels are 32 bytes
+          umma_bf16(leader, d, a[dx] + dy * row16 + 2 * kk, b0 + (t * L::B_BYTES >> 4) + 2 * kk, L::IDESC,
+                    (t | kk) != 0);
+        if (dy == 2) umma_commit(leader, &empty[sl[dx]]);  // the box is free once the MMAs so far have read it
+      }
+      umma_commit(leader, &accfull[buf]);
     }
+    if (!ok && leader) atomicOr(err, 1);
+    umma_commit(leader, done);  // every MMA issued has completed once this arrives
+    mbar_wait_warp(done, 0);
   } else {  // ---- epilogue: warps 2-5
     const int q = warp & 3;  // the lane quarter this warp may read
     float bv[COUT];
 #pragma unroll
-    for (int j = 0; j < COUT; j++) bv[j] = bias ? bias[j] : 0.f;
+    for (int j = 0; j < COUT; j++) bv[j] = MASK ? 0.f : bias[j];  // input gradients have no bias
     int it = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
-      const int buf = it & 1;
-      const int w0 = (tile % ntw) * tw, h0 = ((tile / ntw) % nth) * th, b = tile / (ntw * nth);
-      const int m = 32 * q + lane;  // this thread's accumulator lane: pixel m of the tile
-      const int hh = h0 + m / tw, ww = w0 + m % tw;
+    const int m = 32 * q + lane;  // this thread's accumulator lane: pixel m of the tile
+    const int hm = m / tw, wm = m % tw;
+    for (TileWalk t(ntw, nth); t.b < B; t.next(), it++) {
+      const int buf = it % L::NACC, b = t.b;
+      const int hh = t.h * th + hm, ww = t.w * tw + wm;
       const bool inside = hh < H && ww < W;
       const long long p = ((long long)b * H + hh) * W + ww;
       uint4 mk[MASK ? COUT / 8 : 1];
@@ -284,7 +362,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
 #pragma unroll
         for (int j = 0; j < COUT / 8; j++) mk[j] = __ldg(reinterpret_cast<const uint4*>(mask + p * COUT) + j);
       }
-      if (!mbar_wait_bounded(&accfull[buf], (it / 2) & 1)) {
+      if (!mbar_wait_bounded(&accfull[buf], (it / L::NACC) & 1)) {
         if (lane == 0) atomicOr(err, 1);
         break;
       }
@@ -296,7 +374,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
       tmem_wait_ld();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&accempty[buf]);  // the accumulator may take the tile after next
+      if (lane == 0) mbar_arrive(&accempty[buf]);  // the accumulator may take a later tile
       if (!inside) continue;
       float v[COUT];
 #pragma unroll
@@ -329,41 +407,39 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, 64);
+    tmem_dealloc(tmem, 32 * L::NACC);
   }
 }
 
 // ---------------------------------------------------------------- tcgen05 weight gradient
 // dw[n][tap][c] += sum_p dy[p][n] * x[p + off(tap)][c] as tcgen05 MMAs with K = pixels:
-// per 128-pixel tile, TMA loads the nine shifted x tiles (as in the forward pass) and the
-// dy tile into one stage. Both operands are MN-major there (channels contiguous per
-// pixel row). Four taps' x tiles, 8 KB apart, form one 128-row A operand (rows (tap, c):
-// the spacing is the descriptor's leading offset), so three MMA groups -- taps 0-3, 4-7
-// and 5-8 (whose last quarter, tap 8, is the one kept) -- cover the nine taps with
-// M = 128, N = COUT, eight K steps of 16 pixels each. The accumulators (3 x COUT
-// tensor-memory columns) sum over every tile the CTA takes; at the end the four
-// epilogue warps write them to the CTA's slice of the layer's part of dw_part, which
-// weight_step_kernel adds up in CTA order (the same bits on every run).
+// per 128-pixel tile, TMA loads the three column boxes of x (as in the forward pass) and
+// the dy tile into one stage. Both operands are MN-major there (channels contiguous per
+// pixel row). A column's three taps start one row of tw pixels apart in its box; with a
+// fourth row offset, whose results are not used, they form one 128-row A operand (rows
+// (dy, c): the spacing is the descriptor's leading offset), so three MMA groups -- one per
+// column -- cover the nine taps with M = 128, N = COUT, eight K steps of 16 pixels each.
+// The accumulators (3 x COUT tensor-memory columns) sum over every tile the CTA takes; at
+// the end the four epilogue warps write them to the CTA's slice of the layer's part of
+// dw_part, which weight_step_kernel adds up in CTA order (the same bits on every run).
 template <int COUT>
 struct TcWgrad {
   static_assert(COUT == 16 || COUT == 32, "output channels: the MMA's N");
-  static constexpr int CIN = 32;
-  static constexpr int A_BYTES = 128 * CIN * 2;  // one tap's x tile
+  static constexpr int CIN = 32, A_ROWB = CIN * 2;
   static constexpr int B_ROWB = COUT * 2;
   static constexpr int B_BYTES = 128 * B_ROWB;   // the dy tile
   static constexpr uint32_t A_LAYOUT = 4u, B_LAYOUT = COUT == 32 ? 4u : 6u;  // 64-byte / 32-byte swizzle
-  static constexpr uint32_t A_SBO = 8 * CIN * 2, B_SBO = 8 * B_ROWB;
-  static constexpr int STAGE = 9 * A_BYTES + B_BYTES;
-  static constexpr int NST = 2;  // stages: the next tile loads while this one's MMAs run
-  static constexpr int OFF_BAR = NST * STAGE;
-  static constexpr int SMEM = OFF_BAR + 64 + 1024;
+  static constexpr uint32_t A_SBO = 8 * A_ROWB, B_SBO = 8 * B_ROWB;
+  static constexpr int NST = 5;  // stages: the next tiles load while this one's MMAs run (8 x 258 x 257, with
+                                 // the descriptors in uniform registers: 41 -> 31 us per layer)
+  static constexpr int stage(int tw) { return 3 * conv_box_bytes(tw, A_ROWB) + B_BYTES; }
+  static constexpr int HEAD = 1024;  // barriers, tensor-memory address
+  static constexpr int smem(int tw) { return HEAD + NST * stage(tw) + 1024; }
   static constexpr uint32_t IDESC = umma_idesc_bf16(128, COUT) | (1u << 15) | (1u << 16);  // A, B MN-major
   static constexpr int THREADS = 192;
-  static_assert(STAGE % 1024 == 0 && SMEM <= 227 * 1024, "shared memory");
-  // one instruction reads two 8-row K groups of four M spans of A (at most 8 KB + 2 KB past
-  // its start, the last group starting at tap 5 plus seven K steps) and of one span of dy:
-  // inside its stage
-  static_assert(5 * A_BYTES + 14 * A_SBO + A_BYTES + 4 * A_SBO <= 9 * A_BYTES, "operand reads stay in the stage");
+  static_assert(smem(kConvMaxTw) <= 227 * 1024, "shared memory");
+  // the fourth row offset of the last column reads one row of pixels past its box: the dy tile
+  static_assert(B_BYTES >= kConvMaxTw * A_ROWB, "operand reads stay in the stage");
 };
 
 template <int COUT>
@@ -373,8 +449,10 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
   using L = TcWgrad<COUT>;
   constexpr int NST = L::NST, CIN = L::CIN;
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::OFF_BAR);
+  unsigned char* head = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
+  unsigned char* smem = head + L::HEAD;
+  const int box = conv_box_bytes(tw, L::A_ROWB), stage = L::stage(tw);
+  uint64_t* full = reinterpret_cast<uint64_t*>(head);
   uint64_t* empty = full + NST;
   uint64_t* accfull = empty + NST;
   uint32_t* tslot = reinterpret_cast<uint32_t*>(accfull + 1);
@@ -399,52 +477,53 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
   if (warp == 0) {  // ---- loads
     if (lane == 0) {
       int it = 0;
-      for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+      for (TileWalk t(ntw, nth); t.b < B; t.next(), it++) {
         const int s = it % NST;
         if (it >= NST && !mbar_wait_bounded(&empty[s], ((it / NST) - 1) & 1)) {
           atomicOr(err, 1);
           break;
         }
-        const int w0 = (tile % ntw) * tw, h0 = ((tile / ntw) % nth) * th, b = tile / (ntw * nth);
-        unsigned char* st = smem + s * L::STAGE;
-        mbar_arrive_expect_tx(&full[s], L::STAGE);
-        for (int t = 0; t < 9; t++) tma_load_4d(st + t * L::A_BYTES, &xmap, 0, w0 + t % 3 - 1, h0 + t / 3 - 1, b, &full[s]);
-        tma_load_4d(st + 9 * L::A_BYTES, &dymap, 0, w0, h0, b, &full[s]);
+        const int w0 = t.w * tw, h0 = t.h * th, b = t.b;
+        unsigned char* st = smem + s * stage;
+        mbar_arrive_expect_tx(&full[s], 3 * (th + 2) * tw * L::A_ROWB + L::B_BYTES);
+        for (int dx = 0; dx < 3; dx++) tma_load_4d(st + dx * box, &xmap, 0, w0 + dx - 1, h0 - 1, b, &full[s]);
+        tma_load_4d(st + 3 * box, &dymap, 0, w0, h0, b, &full[s]);
       }
       for (int kk = (it >= NST ? it - NST : 0); kk < it; kk++) mbar_wait_bounded(&full[kk % NST], (kk / NST) & 1);
     }
   } else if (warp == 1) {  // ---- MMAs
-    if (lane == 0) {
-      bool ok = true;
-      int it = 0;
-      for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
-        const int s = it % NST;
-        if (!(ok = mbar_wait_bounded(&full[s], (it / NST) & 1))) break;
-        tc_fence_after();
-        const uint32_t st = smem_addr(smem + s * L::STAGE), dy0 = st + 9 * L::A_BYTES;
+    const uint32_t leader = lane == 0;
+    bool ok = true;
+    const uint64_t a0 = umma_smem_desc_mn(smem_addr(smem), tw * L::A_ROWB, L::A_SBO, L::A_LAYOUT);
+    const uint64_t b0 = umma_smem_desc_mn(smem_addr(smem) + 3 * box, L::B_SBO, L::B_SBO, L::B_LAYOUT);
+    const uint32_t stage16 = (uint32_t)stage >> 4, box16 = (uint32_t)box >> 4;  // as in descriptors
+    int s = 0, phase = 0, it = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
+      if (!(ok = mbar_wait_warp(&full[s], phase))) break;
+      tc_fence_after();
+      const uint64_t a = a0 + (uint64_t)(s * stage16), b = b0 + (uint64_t)(s * stage16);
 #pragma unroll
-        for (int g = 0; g < 3; g++) {
-          const uint32_t a0 = st + (g == 0 ? 0 : (g == 1 ? 4 : 5)) * L::A_BYTES;
+      for (int k = 0; k < 8; k++)  // 16 pixels = two 8-row groups per K step
 #pragma unroll
-          for (int k = 0; k < 8; k++)  // 16 pixels = two 8-row groups per K step
-            umma_bf16(tmem + (uint32_t)(g * COUT),
-                      umma_smem_desc_mn(a0 + 2 * k * L::A_SBO, L::A_BYTES, L::A_SBO, L::A_LAYOUT),
-                      umma_smem_desc_mn(dy0 + 2 * k * L::B_SBO, L::B_SBO, L::B_SBO, L::B_LAYOUT), L::IDESC,
-                      (it | k) != 0);
-        }
-        umma_commit(&empty[s]);
+        for (int g = 0; g < 3; g++)
+          umma_bf16(leader, tmem + (uint32_t)(g * COUT), a + g * box16 + (2 * k * L::A_SBO >> 4),
+                    b + (2 * k * L::B_SBO >> 4), L::IDESC, (it | k) != 0);
+      umma_commit(leader, &empty[s]);
+      if (++s == NST) {
+        s = 0;
+        phase ^= 1;
       }
-      if (!ok) atomicOr(err, 1);
-      umma_commit(accfull);  // every MMA issued has completed once this arrives
     }
+    if (!ok && leader) atomicOr(err, 1);
+    umma_commit(leader, accfull);  // every MMA issued has completed once this arrives
   } else {  // ---- epilogue: warps 2-5, once per CTA
-    const int q = warp & 3;  // lane quarter: row (tap offset q within a group, c = lane)
+    const int q = warp & 3;  // lane quarter: row (vertical tap offset q, c = lane)
     if (mbar_wait_bounded(accfull, 0)) {
       tc_fence_after();
 #pragma unroll
       for (int g = 0; g < 3; g++) {
-        if (g == 2 && q != 3) continue;  // taps 5-7 again: kept from the second group
-        const int tap = (g == 0 ? 0 : (g == 1 ? 4 : 5)) + q;
+        if (q == 3) continue;
+        const int tap = 3 * q + g;
 #pragma unroll
         for (int n0 = 0; n0 < COUT; n0 += 16) {
           uint32_t r[16];
@@ -726,9 +805,9 @@ struct sbp_cnn {
   float* out16 = nullptr;    // last layer output (FP32, 16 channels)
   float* loss = nullptr;
   int* err = nullptr;        // the tensor-core convolutions' error word (a bounded wait ran out)
-  int tw = 0, th = 0;        // their pixel tile: th rows of tw pixels, th * tw = 128
+  int tw = 0, th = 0;        // the tensor-core kernels' pixel tile: th rows of tw pixels, th * tw = 128
   int nsm = 1;               // SMs: the persistent convolutions' grid
-  float* dw_part[kLayers] = {};  // the weight gradients' per-CTA sums ([nsm][wcount(l)])
+  float* dw_part[kLayers] = {};  // the weight gradients' per-CTA sums ([nsm][wcount(l)] each, one block)
   long long launches = 0;
   std::string msg;
 };
@@ -755,11 +834,11 @@ long long wcount(int l) { return (long long)kCout[l] * 9 * kCin[l]; }
 void cnn_release(sbp_cnn* c) {
   for (int l = 0; l < kLayers; l++) {
     void* ps[] = {c->wm[l], c->wb[l], c->wT[l], c->bias[l], c->mw[l], c->vw[l], c->mbias[l], c->vbias[l],
-                  c->gw[l], c->gb[l], c->act[l], c->dw_part[l]};
+                  c->gw[l], c->gb[l], c->act[l]};
     for (void* p : ps)
       if (p) cudaFree(p);
   }
-  void* ps[] = {c->dact, c->dact2, c->out16, c->loss, c->err};
+  void* ps[] = {c->dact, c->dact2, c->out16, c->loss, c->err, c->dw_part[0]};
   for (void* p : ps)
     if (p) cudaFree(p);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
@@ -781,17 +860,17 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// The tensor maps of one convolution: the NHWC BF16 input ({ch, W, H, B}, box {ch, tw,
-// th, 1}) and the weights ([cout][9][ch]: {ch, 9, cout}, box {ch, 1, cout}), rows
+// The tensor maps of one convolution: the NHWC BF16 input ({ch, W, H, B}, box {ch, bw,
+// bh, 1}) and the weights ([cout][9][ch]: {ch, 9, cout}, box {ch, 1, cout}), rows
 // swizzled over their ch * 2 bytes. Out-of-range boxes read zeros (the image border).
-cudaError_t encode_conv_maps(const sbp_cnn* c, const bf16* x, const bf16* w, int ch, int cout, int batch,
-                             CUtensorMap* xm, CUtensorMap* wm) {
+cudaError_t encode_conv_maps(const sbp_cnn* c, const bf16* x, const bf16* w, int ch, int cout, int batch, int bw,
+                             int bh, CUtensorMap* xm, CUtensorMap* wm) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
   const CUtensorMapSwizzle sw = ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
   const cuuint64_t xd[4] = {(cuuint64_t)ch, (cuuint64_t)c->W, (cuuint64_t)c->H, (cuuint64_t)batch};
   const cuuint64_t xs[3] = {(cuuint64_t)ch * 2, (cuuint64_t)c->W * ch * 2, (cuuint64_t)c->H * c->W * ch * 2};
-  const cuuint32_t xb[4] = {(cuuint32_t)ch, (cuuint32_t)c->tw, (cuuint32_t)c->th, 1};
+  const cuuint32_t xb[4] = {(cuuint32_t)ch, (cuuint32_t)bw, (cuuint32_t)bh, 1};
   const cuuint32_t e[4] = {1, 1, 1, 1};
   if (enc(xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), xd, xs, xb, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
           sw, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -808,19 +887,19 @@ cudaError_t encode_conv_maps(const sbp_cnn* c, const bf16* x, const bf16* w, int
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 cudaError_t configure_tc() {
   return cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, TcConv<CIN, COUT>::SMEM);
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, TcConv<CIN, COUT>::smem(kConvMaxTw));
 }
 
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 cudaError_t launch_tc(const bf16* x, const bf16* w, const float* bias, const bf16* mask, void* y, const sbp_cnn* c,
                       int batch, cudaStream_t s) {
   CUtensorMap xm, wm;
-  cudaError_t e = encode_conv_maps(c, x, w, CIN, COUT, batch, &xm, &wm);
+  cudaError_t e = encode_conv_maps(c, x, w, CIN, COUT, batch, c->tw, c->th + 2, &xm, &wm);
   if (e != cudaSuccess) return e;
   const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
   const long long slots = (long long)TcConv<CIN, COUT>::CTAS * c->nsm;  // persistent: every CTA resident
   const unsigned grid = (unsigned)(tiles < slots ? tiles : slots);
-  conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK><<<grid, TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::SMEM, s>>>(
+  conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK><<<grid, TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::smem(c->tw), s>>>(
       xm, wm, bias, mask, y, batch, c->H, c->W, c->tw, c->th, c->err);
   return cudaGetLastError();
 }
@@ -828,7 +907,7 @@ cudaError_t launch_tc(const bf16* x, const bf16* w, const float* bias, const bf1
 template <int COUT>
 cudaError_t configure_wgrad_tc() {
   return cudaFuncSetAttribute(conv3x3_wgrad_tc_kernel<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              TcWgrad<COUT>::SMEM);
+                              TcWgrad<COUT>::smem(kConvMaxTw));
 }
 
 // Shared-memory opt-in of the tensor-core convolutions (outside stream capture).
@@ -866,15 +945,15 @@ cudaError_t conv_wgrad(int l, const bf16* x, const bf16* dy, const sbp_cnn* c, i
   const int cout = kCout[l];
   // x: 32-channel tap tiles; dy: one unshifted tile of cout channels (its map from the same
   // encoder, with dy as the "input" and the weights map unused)
-  cudaError_t e = encode_conv_maps(c, x, c->wb[l], 32, cout, batch, &xm, &unused);
-  if (e == cudaSuccess) e = encode_conv_maps(c, dy, c->wb[l], cout, cout, batch, &dym, &unused);
+  cudaError_t e = encode_conv_maps(c, x, c->wb[l], 32, cout, batch, c->tw, c->th + 2, &xm, &unused);
+  if (e == cudaSuccess) e = encode_conv_maps(c, dy, c->wb[l], cout, cout, batch, c->tw, c->th, &dym, &unused);
   if (e != cudaSuccess) return e;
   const unsigned grid = wgrad_ctas(c, batch);
   if (cout == 32)
-    conv3x3_wgrad_tc_kernel<32><<<grid, TcWgrad<32>::THREADS, TcWgrad<32>::SMEM, s>>>(
+    conv3x3_wgrad_tc_kernel<32><<<grid, TcWgrad<32>::THREADS, TcWgrad<32>::smem(c->tw), s>>>(
         xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th, c->err);
   else
-    conv3x3_wgrad_tc_kernel<16><<<grid, TcWgrad<16>::THREADS, TcWgrad<16>::SMEM, s>>>(
+    conv3x3_wgrad_tc_kernel<16><<<grid, TcWgrad<16>::THREADS, TcWgrad<16>::smem(c->tw), s>>>(
         xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th, c->err);
   return cudaGetLastError();
 }
@@ -981,10 +1060,12 @@ int sbp_cnn_create(int height, int width, int max_batch, int device, void* strea
       cudaMalloc(&c->out16, (size_t)P * 16 * 4) || cudaMalloc(&c->loss, 4) || cudaMalloc(&c->err, 4))
     return bad("cudaMalloc(activations)");
   cudaMemset(c->err, 0, 4);
-  // the tensor-core convolutions' tile: 128 pixels, th rows of tw (a power of two), the
-  // shape whose tiles cover the image with the fewest padding pixels (ties: wider rows)
+  // the tensor-core kernels' tile: 128 pixels, th rows of tw, the shape whose tiles cover the
+  // image with the fewest padding pixels (ties: wider rows). tw >= 8: a row of pixels is whole
+  // swizzle atoms, so that the vertical taps can start at any row of a box; tw <= 32: wider
+  // tiles' boxes are mostly halo (64: 4 rows for 2) and five of them overfill shared memory
   long long best = -1;
-  for (int tw = 128; tw >= 1; tw /= 2) {
+  for (int tw = kConvMaxTw; tw >= 8; tw /= 2) {
     const int th = 128 / tw;
     const long long area = (long long)((width + tw - 1) / tw) * tw * ((height + th - 1) / th) * th;
     if (best < 0 || area < best) {
@@ -996,9 +1077,11 @@ int sbp_cnn_create(int height, int width, int max_batch, int device, void* strea
   if (configure_convs() != cudaSuccess) return bad("cudaFuncSetAttribute(convolutions)");
   if (cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || c->nsm < 1)
     return bad("cudaDeviceGetAttribute(SMs)");
-  for (int l = 0; l < kLayers; l++)
-    if (cudaMalloc(&c->dw_part[l], (size_t)c->nsm * wcount(l) * sizeof(float)) != cudaSuccess)
-      return bad("cudaMalloc(weight-gradient sums)");
+  long long sums = 0;
+  for (int l = 0; l < kLayers; l++) sums += wcount(l);
+  if (cudaMalloc(&c->dw_part[0], (size_t)(c->nsm * sums) * sizeof(float)) != cudaSuccess)
+    return bad("cudaMalloc(weight-gradient partial sums)");
+  for (int l = 1; l < kLayers; l++) c->dw_part[l] = c->dw_part[l - 1] + c->nsm * wcount(l - 1);
   if (!encode_fn()) return bad("cuTensorMapEncodeTiled is not available from the driver");
   // a network that failed its initialisation is released, not handed out
   const int rc = sbp_cnn_init(c, 1234);

@@ -1,10 +1,11 @@
-"""The training step's one launch for every layer (sums of the weight-gradient CTAs,
-Adam, the two BF16 copies) and the input packing where x starts off a 16-byte boundary."""
+"""The tensor-core kernels' tile widths, the training step's one launch for every layer
+(sums of the weight-gradient CTAs, Adam, the two BF16 copies) and the input packing where x
+starts off a 16-byte boundary."""
 import numpy as np
 import pytest
 
 import cnn_oracle as N
-from test_cnn import _small_params
+import test_cnn
 
 LR = 1e-3
 
@@ -38,7 +39,7 @@ def test_gpu_step_is_adam_on_the_gradients(sbp, shape):
     x, t = _batch(shape, 11)
     mask = _weights()
     with sbp.Cnn(H, W, B) as net, sbp.Cnn(H, W, B) as fresh:
-        net.set_params(_small_params(5).astype(np.float32))
+        net.set_params(test_cnn._small_params(5).astype(np.float32))
         m = v = 0.0
         for k in (1, 2):
             p = net.get_params().astype(np.float64)
@@ -70,7 +71,16 @@ def test_gpu_unaligned_input_gives_the_same_bits(sbp, offset):
     shifted[offset:offset + x.numel()] = x.reshape(-1)
     out = torch.empty((2, B, H, W, 3), dtype=torch.float32, device="cuda")
     with sbp.Cnn(H, W, B) as net:
-        net.set_params(_small_params(3).astype(np.float32))
+        net.set_params(test_cnn._small_params(3).astype(np.float32))
         net.forward(x.data_ptr(), B, out[0].data_ptr())
         net.forward(shifted.data_ptr() + 4 * offset, B, out[1].data_ptr())
     assert torch.any(out[0] != 0) and torch.equal(out[0], out[1])
+
+
+# 8, 16 and 32 pixels wide; every SM's weight-gradient CTA with a second tile at width 16;
+# an image smaller than a tile
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(2, 10, 8), (1, 8, 48), (1, 4, 33), (9, 8, 272), (1, 1, 1)],
+                         ids=["8-wide", "16-wide", "32-wide", "153-tiles", "1-pixel"])
+def test_gpu_tile_widths_match_oracle(sbp, shape):
+    test_cnn.test_gpu_forward_and_gradients_match_oracle(sbp, shape)
