@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "../../include/sbpgpu.h"
+#include "launch.h"
 #include "sbp_device.cuh"
 
 namespace sbp {
@@ -159,6 +160,14 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
+// Eight mask values. Volatile: not before the kernel's wait for the ones that wrote them.
+// Through L1, since a thread's four loads share two sectors.
+__device__ __forceinline__ uint4 ld_mask(const bf16* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 // Shared-memory layout of conv3x3_tc_kernel: a ring of NS column boxes (th + 2 rows of tw
 // pixels of CIN BF16), the nine taps' weight tiles (COUT rows of CIN), barriers and the
 // tensor-memory address; boxes and tiles 1024-byte aligned (whole swizzle atoms).
@@ -185,6 +194,15 @@ struct TcConv {
   static_assert(B_BYTES % 256 == 0, "tiles start on swizzle atoms");
   static_assert(CTAS * (smem(kConvMaxTw) + 1024) <= 228 * 1024, "shared memory");
 };
+
+// The two halves of grid_dependency_wait. A kernel whose CTAs take several tiles does not
+// let the next kernel's CTAs in before it ends: they would take the places that free up
+// first, two kernels' persistent CTAs sharing the SMs unevenly (training step at 8 x 258 x 257
+// 366 us when let in at the start, 358 after the last loads, 344 at the end, 371 without
+// overlap). With a tile per CTA (2 x 40 x 33) it does, after its loads: 75 us, 86 at the end,
+// 112 without overlap.
+__device__ __forceinline__ void grid_inputs_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // The pixel tiles of a persistent CTA: every gridDim.x-th, as tile column, tile row and
 // image, stepped by carries instead of divided out of a tile number.
@@ -280,6 +298,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tslot;
+  grid_inputs_wait();  // nothing of the kernels before this one is read or overwritten above
 
   if (warp == 0) {  // ---- loads
     if (lane == 0) {
@@ -300,6 +319,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
           tma_load_4d(boxes + s * box, &xmap, 0, w0 + dx - 1, h0 - 1, b, &full[s]);
         }
       }
+      if (ntiles <= (int)gridDim.x) grid_let_next();
       // no copy may be in flight when the CTA exits
       mbar_wait_bounded(wbar, 0);
       for (int kk = (k >= NS ? k - NS : 0); kk < k; kk++) mbar_wait_bounded(&full[kk % NS], (kk / NS) & 1);
@@ -360,7 +380,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
       uint4 mk[MASK ? COUT / 8 : 1];
       if (MASK && inside) {
 #pragma unroll
-        for (int j = 0; j < COUT / 8; j++) mk[j] = __ldg(reinterpret_cast<const uint4*>(mask + p * COUT) + j);
+        for (int j = 0; j < COUT / 8; j++) mk[j] = ld_mask(mask + p * COUT + 8 * j);
       }
       if (!mbar_wait_bounded(&accfull[buf], (it / L::NACC) & 1)) {
         if (lane == 0) atomicOr(err, 1);
@@ -473,6 +493,7 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tslot;
+  grid_inputs_wait();  // nothing of the kernels before this one is read or overwritten above
 
   if (warp == 0) {  // ---- loads
     if (lane == 0) {
@@ -489,6 +510,7 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
         for (int dx = 0; dx < 3; dx++) tma_load_4d(st + dx * box, &xmap, 0, w0 + dx - 1, h0 - 1, b, &full[s]);
         tma_load_4d(st + 3 * box, &dymap, 0, w0, h0, b, &full[s]);
       }
+      if (ntiles <= (int)gridDim.x) grid_let_next();
       for (int kk = (it >= NST ? it - NST : 0); kk < it; kk++) mbar_wait_bounded(&full[kk % NST], (kk / NST) & 1);
     }
   } else if (warp == 1) {  // ---- MMAs
@@ -604,11 +626,12 @@ __global__ void unpack_output_kernel(const float* __restrict__ out16, float* __r
 __global__ void mse_kernel(const float* __restrict__ out16, const float* __restrict__ target, bf16* __restrict__ d16,
                            float* __restrict__ loss, long long P) {
   static_assert(kOutReal == 3, "the first three channels");
+  grid_dependency_wait();
   __shared__ float sh[256];
   float s = 0.f;
   const float scale = 2.f / (float)(P * kOutReal);
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < P; p += (long long)gridDim.x * blockDim.x) {
-    const float4 o = __ldg(reinterpret_cast<const float4*>(out16 + p * 16));
+    const float4 o = __ldcg(reinterpret_cast<const float4*>(out16 + p * 16));
     const float r0 = o.x - target[3 * p], r1 = o.y - target[3 * p + 1], r2 = o.z - target[3 * p + 2];
     s += r0 * r0;
     s += r1 * r1;
@@ -642,7 +665,7 @@ struct AllWeights {
 // Volatile, so that a run of them stays ahead of the additions that use them.
 __device__ __forceinline__ float ld_early(const float* p) {
   float v;
-  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
   return v;
 }
 
@@ -659,9 +682,10 @@ __global__ void __launch_bounds__(128) weight_step_kernel(const __grid_constant_
                                                           float b1, float b2, float eps, float c1, float c2,
                                                           const int* __restrict__ err) {
   constexpr int UN = 38;
+  grid_dependency_wait();
   const LayerWeights& w = a.layer[blockIdx.y];
   const int e = blockIdx.x * blockDim.x + threadIdx.x, n = w.n;
-  if (e >= n || (ADAM && *err)) return;
+  if (e >= n || (ADAM && __ldcg(err))) return;
   float s = 0.f;
   const float* part = w.part + e;
   int c = 0;
@@ -899,9 +923,9 @@ cudaError_t launch_tc(const bf16* x, const bf16* w, const float* bias, const bf1
   const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
   const long long slots = (long long)TcConv<CIN, COUT>::CTAS * c->nsm;  // persistent: every CTA resident
   const unsigned grid = (unsigned)(tiles < slots ? tiles : slots);
-  conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK><<<grid, TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::smem(c->tw), s>>>(
-      xm, wm, bias, mask, y, batch, c->H, c->W, c->tw, c->th, c->err);
-  return cudaGetLastError();
+  return sbp::launch_overlapped(conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK>, dim3(grid),
+                           dim3(TcConv<CIN, COUT>::THREADS), TcConv<CIN, COUT>::smem(c->tw), s, xm, wm, bias, mask, y,
+                           batch, c->H, c->W, c->tw, c->th, c->err);
 }
 
 template <int COUT>
@@ -950,12 +974,12 @@ cudaError_t conv_wgrad(int l, const bf16* x, const bf16* dy, const sbp_cnn* c, i
   if (e != cudaSuccess) return e;
   const unsigned grid = wgrad_ctas(c, batch);
   if (cout == 32)
-    conv3x3_wgrad_tc_kernel<32><<<grid, TcWgrad<32>::THREADS, TcWgrad<32>::smem(c->tw), s>>>(
-        xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th, c->err);
-  else
-    conv3x3_wgrad_tc_kernel<16><<<grid, TcWgrad<16>::THREADS, TcWgrad<16>::smem(c->tw), s>>>(
-        xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th, c->err);
-  return cudaGetLastError();
+    return sbp::launch_overlapped(conv3x3_wgrad_tc_kernel<32>, dim3(grid), dim3(TcWgrad<32>::THREADS),
+                             TcWgrad<32>::smem(c->tw), s, xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th,
+                             c->err);
+  return sbp::launch_overlapped(conv3x3_wgrad_tc_kernel<16>, dim3(grid), dim3(TcWgrad<16>::THREADS),
+                           TcWgrad<16>::smem(c->tw), s, xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th,
+                           c->err);
 }
 
 AllWeights all_weights(const sbp_cnn* c) {
@@ -1196,10 +1220,11 @@ int sbp_cnn_forward(sbp_cnn* c, const float* x, int batch, float* out) {
 static int backward(sbp_cnn* c, const float* x, const float* target, int batch, float* loss, float lr) {
   const bool train = lr > 0;
   const long long P = (long long)batch * c->H * c->W;
+  CCK(cudaMemsetAsync(c->loss, 0, 4, c->stream));
   int rc = run_forward(c, x, batch);
   if (rc) return rc;
-  CCK(cudaMemsetAsync(c->loss, 0, 4, c->stream));
-  mse_kernel<<<blocks_for(P, 256), 256, 0, c->stream>>>(c->out16, target, c->dact, c->loss, P);
+  CCK(sbp::launch_overlapped(mse_kernel, dim3(blocks_for(P, 256)), dim3(256), 0, c->stream, c->out16, target, c->dact,
+                        c->loss, P));
   c->launches++;
   if (!train)
     for (int l = 0; l < kLayers; l++) CCK(cudaMemsetAsync(c->gb[l], 0, kCout[l] * 4, c->stream));
@@ -1226,11 +1251,12 @@ static int backward(sbp_cnn* c, const float* x, const float* target, int batch, 
     const float c1 = 1.f - std::pow(b1, t), c2 = 1.f - std::pow(b2, t);
     // padded channels stay zero: their gradients are zero (zero inputs / zero targets) and
     // Adam leaves zero-gradient entries unchanged.
-    weight_step_kernel<true><<<weight_step_grid(), 128, 0, c->stream>>>(a, ctas, lr, b1, b2, 1e-8f, c1, c2, c->err);
+    CCK(sbp::launch_overlapped(weight_step_kernel<true>, weight_step_grid(), dim3(128), 0, c->stream, a, ctas, lr, b1, b2,
+                          1e-8f, c1, c2, c->err));
   } else {
-    weight_step_kernel<false><<<weight_step_grid(), 128, 0, c->stream>>>(a, ctas, 0.f, 0.f, 0.f, 0.f, 1.f, 1.f, c->err);
+    CCK(sbp::launch_overlapped(weight_step_kernel<false>, weight_step_grid(), dim3(128), 0, c->stream, a, ctas, 0.f, 0.f,
+                          0.f, 0.f, 1.f, 1.f, c->err));
   }
-  CCK(cudaGetLastError());
   c->launches++;
   float h = 0;
   int e = 0;
