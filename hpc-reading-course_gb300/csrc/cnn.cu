@@ -179,7 +179,7 @@ struct TcConv {
   static constexpr uint32_t LAYOUT = CIN == 32 ? 4u : 6u;  // 64-byte / 32-byte swizzle
   static constexpr uint32_t ATOM = 8 * ROWB;
   static constexpr int NS = 6;    // column boxes in flight: two pixel tiles per CTA
-  static constexpr int CTAS = 2;  // resident CTAs per SM (forward pass at 8 x 258 x 257: 0.138 ms; three
+  static constexpr int CTAS = 2;  // resident CTAs per SM (forward pass at 8 x 258 x 257, launches not overlapped: 0.138 ms; three
                                   // CTAs with 4 boxes 0.138 ms, four with 3 boxes 0.146 ms)
   static constexpr int B_BYTES = COUT * ROWB;
   static constexpr int box_bytes(int tw) { return conv_box_bytes(tw, ROWB); }
@@ -249,7 +249,8 @@ struct TileWalk {
 // nine MMAs left out the forward pass (8 x 258 x 257) still took 0.161 of its 0.197 ms.
 // Issued from one lane's branch, each MMA builds its two descriptors in that lane and moves
 // them to uniform registers; now the whole warp runs the loop, descriptors are a base plus
-// constants, and only the MMAs and the commits are predicated on one lane: 0.138 ms. Three
+// constants, and only the MMAs and the commits are predicated on one lane: 0.138 ms (0.126
+// with the kernels' launches overlapped). Three
 // column boxes instead of nine shifted tiles (2.4 x fewer bytes through L2) made no
 // difference before that.
 //
@@ -451,7 +452,7 @@ struct TcWgrad {
   static constexpr uint32_t A_LAYOUT = 4u, B_LAYOUT = COUT == 32 ? 4u : 6u;  // 64-byte / 32-byte swizzle
   static constexpr uint32_t A_SBO = 8 * A_ROWB, B_SBO = 8 * B_ROWB;
   static constexpr int NST = 5;  // stages: the next tiles load while this one's MMAs run (8 x 258 x 257, with
-                                 // the descriptors in uniform registers: 41 -> 31 us per layer)
+                                 // the descriptors in uniform registers: 41 -> 32 us per layer)
   static constexpr int stage(int tw) { return 3 * conv_box_bytes(tw, A_ROWB) + B_BYTES; }
   static constexpr int HEAD = 1024;  // barriers, tensor-memory address
   static constexpr int smem(int tw) { return HEAD + NST * stage(tw) + 1024; }
