@@ -133,9 +133,11 @@ int wave_kind(const sbp_ctx* ctx) {
 //   FP32 rho=K=1   4.7 / 7.9    6.5 / 10.4  10.2 / 13.4  15.2 / 15.8  23.0 / 20.6  36.0 / 28.6
 //   FP32 var.      5.7 / 8.6    7.7 / 12.8  12.1 / 15.1  18.6 / 19.5  30.7 / 26.0  46.2 / 37.5
 // (Fehlberg stages at 1024^2: 0.2 ms per attempt in either form.)
+// A grid of cells has at most 65535 rows of them (a narrow grid can have more).
+bool cells_fit(const sbp_ctx* ctx) { return ctx->ny <= 65535LL * kCellTY; }
 bool use_cell(const sbp_ctx* ctx) {
   const bool early = ctx->fp32 || wave_kind(ctx) == WK_HOM;
-  return ctx->npts <= (early ? 1150000 : 1600000);
+  return cells_fit(ctx) && ctx->npts <= (early ? 1150000 : 1600000);
 }
 
 // Encodes one 3D tensor map (x, y, component) over a state buffer of the context.
@@ -653,7 +655,7 @@ int launch_rhs_aos(sbp_ctx* ctx, double t, const double* src, double* dst, int b
 bool rhs_takes_aos(const sbp_ctx* ctx, const double* src, const double* dst, int where) {
   const double *se = src + ctx->nscalar, *de = dst + ctx->nscalar;
   return where == SBP_DEVICE && ctx->wave && !ctx->ysplit && !ctx->drop_tile && (se <= dst || de <= src) &&
-         ctx->ny <= 65535LL * kCellTY;  // the rows a grid of cells can have
+         cells_fit(ctx);
 }
 
 int rhs_impl(sbp_ctx* ctx, double t, const double* src, double* dst, int where, int bc_on) {
