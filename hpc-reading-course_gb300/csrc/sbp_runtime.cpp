@@ -88,6 +88,7 @@ struct sbp_ctx {
   long long launches = 0;
   unsigned long long wait_ns = 0;  // limit of the wave stage kernels' bounded waits (0: the kernel default)
   int drop_tile = 0;               // test aid: tile + 1 whose load the next RHS evaluation skips
+  int form = SBP_FORM_BY_SIZE;     // test aid: the 2D wave kernels to run
   std::string msg;
 };
 
@@ -136,6 +137,7 @@ int wave_kind(const sbp_ctx* ctx) {
 // A grid of cells has at most 65535 rows of them (a narrow grid can have more).
 bool cells_fit(const sbp_ctx* ctx) { return ctx->ny <= 65535LL * kCellTY; }
 bool use_cell(const sbp_ctx* ctx) {
+  if (ctx->form != SBP_FORM_BY_SIZE) return cells_fit(ctx) && ctx->form == SBP_FORM_CELLS;
   const bool early = ctx->fp32 || wave_kind(ctx) == WK_HOM;
   return cells_fit(ctx) && ctx->npts <= (early ? 1150000 : 1600000);
 }
@@ -446,7 +448,7 @@ int enqueue_step(sbp_ctx* ctx, double t, double dt, const double* ct = nullptr) 
 
 // Whether a context's RK4 steps run as one launch each (wave_step.cuh).
 bool use_step(const sbp_ctx* ctx) {
-  return ctx->wave && !ctx->fp32 && step_takes(ctx->d.order, ctx->nx, ctx->ny);
+  return ctx->form == SBP_FORM_BY_SIZE && ctx->wave && !ctx->fp32 && step_takes(ctx->d.order, ctx->nx, ctx->ny);
 }
 
 // One RK4 step from `in` to `out` in one launch; ct as for enqueue_step.
@@ -655,7 +657,7 @@ int launch_rhs_aos(sbp_ctx* ctx, double t, const double* src, double* dst, int b
 bool rhs_takes_aos(const sbp_ctx* ctx, const double* src, const double* dst, int where) {
   const double *se = src + ctx->nscalar, *de = dst + ctx->nscalar;
   return where == SBP_DEVICE && ctx->wave && !ctx->ysplit && !ctx->drop_tile && (se <= dst || de <= src) &&
-         cells_fit(ctx);
+         cells_fit(ctx) && ctx->form != SBP_FORM_PERSISTENT;
 }
 
 int rhs_impl(sbp_ctx* ctx, double t, const double* src, double* dst, int where, int bc_on) {
@@ -708,14 +710,23 @@ int wave_grid(const sbp_ctx* ctx) {
   return (int)(ntiles < nsm ? ntiles : nsm);
 }
 
+// Room for the error partial sums of the form that runs.
+int rk45_partials(sbp_ctx* ctx) {
+  const int parts = ctx->wave ? wave_grid(ctx) : 0;
+  if (ctx->rk_partial) CK(cudaFree(ctx->rk_partial));
+  ctx->rk_partial = nullptr;
+  CK(cudaMalloc((void**)&ctx->rk_partial, sizeof(double) * (parts > kReduceBlocks ? parts : kReduceBlocks)));
+  return SBP_OK;
+}
+
 int rk45_prepare(sbp_ctx* ctx) {
   if (ctx->rk_ctrl) return SBP_OK;
   const size_t bytes = (size_t)ctx->dofs * ctx->plane * sizeof(double);
   for (int s = 0; s < 6; s++) CK(cudaMalloc((void**)&ctx->rk_k[s], bytes));
   CK(cudaMalloc((void**)&ctx->rk_unew, bytes));
   CK(cudaMemsetAsync(ctx->rk_unew, 0, bytes, ctx->stream));  // row padding stays zero
-  const int parts = ctx->wave ? wave_grid(ctx) : 0;
-  CK(cudaMalloc((void**)&ctx->rk_partial, sizeof(double) * (parts > kReduceBlocks ? parts : kReduceBlocks)));
+  int rc;
+  if ((rc = rk45_partials(ctx))) return rc;
   CK(cudaMalloc((void**)&ctx->rk_ctrl, sizeof(Rk45Ctrl)));
   return SBP_OK;
 }
@@ -1273,18 +1284,34 @@ int sbp_ts_rk45(sbp_ctx* ctx, double t_end, double dt, double* v, int where) {
   return sbp_get_state(ctx, v, where);
 }
 
+// Drops the captured graphs, whose launches carry the settings they were captured with.
+static void drop_captured(sbp_ctx* ctx) {
+  drop_graphs(ctx);
+  if (ctx->rk_graph) {
+    cudaGraphExecDestroy(ctx->rk_graph);
+    ctx->rk_graph = nullptr;
+  }
+}
+
 int sbp_set_wait_limit(sbp_ctx* ctx, long long ns) {
   if (!ctx) return SBP_ERR_INVALID;
   if (ns < 0 || ns > 60LL * 1000 * 1000 * 1000) return fail(ctx, SBP_ERR_INVALID, "wait limit must be in [0, 60 s]");
   CK(cudaSetDevice(ctx->d.device));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->wait_ns = (unsigned long long)ns;
-  drop_graphs(ctx);  // captured launches carry the old limit
-  if (ctx->rk_graph) {
-    cudaGraphExecDestroy(ctx->rk_graph);
-    ctx->rk_graph = nullptr;
-  }
+  drop_captured(ctx);
   return SBP_OK;
+}
+
+int sbp_test_wave_form(sbp_ctx* ctx, int form) {
+  if (!ctx) return SBP_ERR_INVALID;
+  if (!ctx->wave) return fail(ctx, SBP_ERR_UNSUPPORTED, "the kernel-form test aid exists for the 2D wave kernels");
+  if (form < SBP_FORM_BY_SIZE || form > SBP_FORM_CELLS) return fail(ctx, SBP_ERR_INVALID, "unknown kernel form");
+  CK(cudaSetDevice(ctx->d.device));
+  CK(cudaStreamSynchronize(ctx->stream));
+  ctx->form = form;
+  drop_captured(ctx);
+  return ctx->rk_partial ? rk45_partials(ctx) : SBP_OK;
 }
 
 int sbp_test_drop_tile(sbp_ctx* ctx, long long tile) {

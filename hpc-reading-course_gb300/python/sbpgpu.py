@@ -27,6 +27,7 @@ WAVE_3D = 8
 BC_REFERENCE, BC_CHARACTERISTIC = 0, 1
 FP64, FP32 = 0, 1
 HOST, DEVICE = 0, 1
+FORM_BY_SIZE, FORM_PERSISTENT, FORM_CELLS = 0, 1, 2
 TWO_D = {WAVE_HOM_2D, WAVE_MMS_2D, WAVE_VAR_2D, ADVECTION_2D, WAVE_2BLOCK_2D}
 DOFS = {WAVE_HOM_2D: 3, WAVE_MMS_2D: 3, WAVE_VAR_2D: 3, ADVECTION_1D: 1, ADVECTION_2D: 1, REFLECTION_1D: 2,
         WAVE_2BLOCK_2D: 3, WAVE_3D: 4}
@@ -35,7 +36,7 @@ DOFS = {WAVE_HOM_2D: 3, WAVE_MMS_2D: 3, WAVE_VAR_2D: 3, ADVECTION_1D: 1, ADVECTI
 EXPORTS = ("sbp_create", "sbp_destroy", "sbp_last_error", "sbp_dofs", "sbp_size", "sbp_rhs", "sbp_apply", "sbp_rk4_nsteps",
            "sbp_ts_rk4", "sbp_rk4", "sbp_set_state", "sbp_get_state", "sbp_rk4_resident", "sbp_synchronize",
            "sbp_error_norms", "sbp_hnorm", "sbp_get_stream", "sbp_launch_count", "sbp_probe_dfma_rate",
-           "sbp_set_wait_limit", "sbp_test_drop_tile",
+           "sbp_set_wait_limit", "sbp_test_drop_tile", "sbp_test_wave_form",
            "sbp_wave_rhs_noalloc", "sbp_write_petsc_vec", "sbp_read_petsc_vec",
            "sbp_batch_create", "sbp_batch_destroy", "sbp_batch_last_error", "sbp_batch_set_state",
            "sbp_batch_get_state", "sbp_batch_rk4_resident", "sbp_batch_synchronize", "sbp_batch_autotune",
@@ -130,6 +131,7 @@ def load(path: str = LIB_PATH) -> C.CDLL:
     L.sbp_probe_dfma_rate.argtypes = [C.c_int, _dp]
     L.sbp_set_wait_limit.argtypes = [P, C.c_longlong]
     L.sbp_test_drop_tile.argtypes = [P, C.c_longlong]
+    L.sbp_test_wave_form.argtypes = [P, C.c_int]
     L.sbp_wave_rhs_noalloc.argtypes = [C.POINTER(Desc), C.c_double, C.c_void_p, C.c_void_p]
     L.sbp_batch_create.argtypes = [C.POINTER(Instance), C.c_int, C.c_int, C.c_int, C.c_void_p, C.POINTER(P)]
     L.sbp_batch_destroy.argtypes = [P]
@@ -331,6 +333,10 @@ class Context:
         """Test aid: the next rhs()/apply() issues no load for this tile, so its
         bounded wait runs out and the call raises SbpError(ERR_DEVICE)."""
         self._check(self._L.sbp_test_drop_tile(self._h, tile))
+
+    def test_wave_form(self, form: int):
+        """Test aid: the 2D wave kernels to run (FORM_BY_SIZE, FORM_PERSISTENT, FORM_CELLS)."""
+        self._check(self._L.sbp_test_wave_form(self._h, form))
 
     def rhs_ptr(self, t: float, src_ptr: int, dst_ptr: int, where: int):
         self._check(self._L.sbp_rhs(self._h, t, src_ptr, dst_ptr, where))

@@ -213,6 +213,13 @@ long long sbp_launch_count(const sbp_ctx* ctx);
 int sbp_set_wait_limit(sbp_ctx* ctx, long long ns);
 int sbp_test_drop_tile(sbp_ctx* ctx, long long tile);
 
+/* Test aid: which kernels a 2D wave context runs from now on. A context picks them
+ * by its grid's size (SBP_FORM_BY_SIZE): whole RK4 steps, one cell of the grid per
+ * short CTA, or persistent tiles. The other two values hold it to one of the latter
+ * (a grid with more rows than cells can cover stays on tiles). */
+enum { SBP_FORM_BY_SIZE = 0, SBP_FORM_PERSISTENT = 1, SBP_FORM_CELLS = 2 };
+int sbp_test_wave_form(sbp_ctx* ctx, int form);
+
 /* Measured FP64 FMA throughput of the current device in DFMA/s (a
  * 1-second-scale probe). No counterpart in the reference; used to state the
  * FP64 ALU roof beside the HBM roof. */
