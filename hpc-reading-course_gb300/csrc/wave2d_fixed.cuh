@@ -10,19 +10,23 @@
 //     order 2: (1/2)  (v1 - v-1)
 //     order 4: (1/12) (8 (v1 - v-1) - (v2 - v-2))
 //     order 6: (1/60) (45 (v1 - v-1) - 9 (v2 - v-2) + (v3 - v-3))
-// so den * sum is an integer combination of the point values. Each tile's
-// stencil boxes are converted once, in place, to 64-bit integers in units of
-// 2^(Emax - 1075), where Emax is the largest biased exponent among the box
-// values of the group (p; u and v together): a double +-M 2^(E-1075) with its
-// 53-bit mantissa M becomes +-trunc(M / 2^(Emax - E)), |V| < 2^53. The sums
-// are then exact in int64 (|S| < 110 * 2^54 < 2^61 at order 6, and the sum of
-// the u and v terms below 2^62), and one conversion back to a double carries the only
-// other rounding of the stencil: the result is as accurate as the reference's FP64
-// evaluation (the conversion to fixed point cuts each value at 2^-52 of the box's largest
-// magnitude, the FP64 sum rounds each partial sum to 2^-53 of its own). Stages with
-// per-point coefficients and the Fehlberg stages (fx_fine) keep two more bits, units of
-// 2^(Emax - 1077), sums below 2^63, and round the conversion back to nearest: the
-// adaptive integrator's steps follow small differences of the state.
+// so den * sum is an integer combination of the point values, exact in int64.
+//
+// Constant coefficients, RHS and RK4 stages: each tile's stencil boxes are converted once, in
+// place, to 64-bit integers in units of 2^(Emax - 1075), where Emax is the largest biased
+// exponent among the box values of the group (p; u and v together): a double +-M 2^(E-1075)
+// with its 53-bit mantissa M becomes +-trunc(M / 2^(Emax - E)), |V| < 2^53. The sums stay
+// below 2^62 (|S| < 110 * 2^54 < 2^61 at order 6, and the u and v terms together), and one
+// conversion back to a double carries the only other rounding: an error of a few 2^-52 of the
+// box's largest magnitude, whatever the point's own.
+//
+// Every other stage (fx_fine) keeps each value whole: the boxes are converted to words that
+// hold the signed mantissa above its exponent (fx_pack), and a stencil brings the words it
+// reads to its own largest exponent. Its values are then in units of 2^-54 of the largest one
+// it reads and its result is rounded to nearest: at every point the accuracy of FP64 taps,
+// also for small values beside large ones. One value's conversion takes about 12 integer
+// instructions and its use in a stencil seven, against about 20 and one in box units (variable
+// coefficients at 2049^2, order 4: 139 us a stage, 123 in box units, 225 with FP64 taps).
 // The integer work runs on the INT pipe; the
 // FP64 pipe is left with the RK4 stage update, 1-2 FMAs per component, into
 // which the scale sigma = -hi/den is folded (fx_ca, fx_cw).
@@ -42,9 +46,8 @@ template <> struct FixDen<2> { static constexpr int value = 2; };
 template <> struct FixDen<4> { static constexpr int value = 12; };
 template <> struct FixDen<6> { static constexpr int value = 60; };
 
-// Which stages take the finer unit and round the stencil sums to nearest. The RK4 and
-// RHS stages of constant coefficients do not: it cost them 1.3 % at 4096^2 and 1024^2, and
-// their error against 64-bit arithmetic was the same with and without it.
+// Which stages give each stencil its own exponent and round its sum to nearest. The RK4 and
+// RHS stages of constant coefficients take their box's.
 template <int KIND, int STAGE> constexpr bool fx_fine() {
   return is_rkf_stage(STAGE) || KIND == WK_VAR || KIND == WK_MMS;
 }
@@ -100,6 +103,73 @@ __device__ __forceinline__ long long fx_stencil(const long long* c, int st) {
   } else {
     return 45 * (c[st] - c[-st]) - 9 * (c[2 * st] - c[-2 * st]) + (c[3 * st] - c[-3 * st]);
   }
+}
+
+// Whole values: a word is the signed mantissa, 53 bits and sign, above a 10-bit field r. The
+// value's biased exponent is kFxTop - r; zero is a zero mantissa with r = kFxNone.
+constexpr int kFxTop = 1087, kFxNone = 1023;
+
+// The word of a double. Sets `out` if it has none: from 2^65 (3.7e19), Inf, NaN, or nonzero
+// and below 2^-958.
+__device__ __forceinline__ long long fx_pack(double v, bool& out) {
+  const unsigned lo = (unsigned)__double2loint(v), hi = (unsigned)__double2hiint(v);
+  const unsigned r = (unsigned)kFxTop - ((hi >> 20) & 0x7FFu);
+  const bool zero = ((hi << 1) | lo) == 0;
+  out |= !zero && r >= (unsigned)kFxNone;
+  const unsigned mh = (hi & 0x000FFFFFu) | 0x00100000u;
+  const long long m = (long long)(((unsigned long long)__funnelshift_l(lo, mh, 10) << 32) | (lo << 10));
+  const long long sg = (long long)((int)hi >> 31);  // 0 or -1
+  return zero ? (long long)kFxNone : (((m ^ sg) - sg) | (long long)(r & 1023u));
+}
+
+// The double of a word, exactly.
+__device__ __forceinline__ double fx_unpack(long long w) {
+  const unsigned r = (unsigned)w & 1023u;
+  const long long m = w & ~1023ll, sg = w >> 63;
+  const unsigned long long a = (unsigned long long)((m ^ sg) - sg);  // leading one at bit 62
+  const unsigned hw = (((unsigned)kFxTop - r - 1) << 20) + (unsigned)(a >> 42);  // it adds the last 1 to the exponent
+  const double v = __hiloint2double((int)(hw | ((unsigned)sg & 0x80000000u)), (int)(a >> 10));
+  return a == 0 ? 0.0 : v;
+}
+
+// The largest exponent (smallest r) among the words that the stencil at c reads, and r.
+template <int ORD>
+__device__ __forceinline__ int fx_least(const long long* c, int st, int r = kFxNone) {
+#pragma unroll
+  for (int k = 1; k <= ORD / 2; k++) r = min(r, min((int)c[k * st] & 1023, (int)c[-k * st] & 1023));
+  return r;
+}
+
+// den * (interior stencil sum) at c in units of 2^(kFxTop - r - 1077): a word is shifted down by
+// 8 bits and its exponent's distance to r (shr.s64 takes any count: 64 and more give 0 or -1).
+// 110 * 2 * 2^55 < 2^63: the sums at order 6, the u and v terms together, stay in range.
+template <int ORD>
+__device__ __forceinline__ long long fx_sum(const long long* c, int st, int r) {
+  const auto at = [&](int k) {
+    const long long w = c[k * st];
+    long long t;
+    asm("shr.s64 %0, %1, %2;" : "=l"(t) : "l"(w & ~1023ll), "r"(((int)w & 1023) - r + 8));
+    return t;
+  };
+  if constexpr (ORD == 2) {
+    return at(1) - at(-1);
+  } else if constexpr (ORD == 4) {
+    return 8 * (at(1) - at(-1)) - (at(2) - at(-2));
+  } else {
+    return 45 * (at(1) - at(-1)) - 9 * (at(2) - at(-2)) + (at(3) - at(-3));
+  }
+}
+
+// den * (interior stencil sum) on words, as a double; and the sum of two such.
+template <int ORD>
+__device__ __forceinline__ double fx_d1(const long long* c, int st) {
+  const int r = fx_least<ORD>(c, st);
+  return fx_to<true>(fx_sum<ORD>(c, st, r), fx_base<true>(kFxTop - r));
+}
+template <int ORD>
+__device__ __forceinline__ double fx_d1_sum(const long long* a, int sa, const long long* b, int sb) {
+  const int r = fx_least<ORD>(b, sb, fx_least<ORD>(a, sa));
+  return fx_to<true>(fx_sum<ORD>(a, sa, r) + fx_sum<ORD>(b, sb, r), fx_base<true>(kFxTop - r));
 }
 
 // The interior stencil at the point c of an FP64 line in global memory (scaled taps, the
@@ -407,7 +477,6 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
                                                 double* errsq = nullptr) {
   constexpr int RKS = is_rkf_stage(STAGE) ? STAGE - ST_RKF1 + 1 : 1;
   constexpr bool FINE = fx_fine<KIND, STAGE>();
-  constexpr int CW = OpShape<ORD>::CW;
   constexpr int TY = Tile::TY, CS = OpShape<ORD>::CS;
   constexpr int HX = Tile::HX, HY = Tile::HY, PW = Tile::PW;
   constexpr int ROWS = TY / Tile::WARPS;
@@ -427,7 +496,13 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
   const bool xfaces = dbar != nullptr && prm.bc != BC_NONE &&
                       ((iw >= i0 && iw < i0 + kWaveTX) || (ie >= i0 && ie < i0 + kWaveTX && ie < g.nx));
   const double sg[3] = {prm.fx_sig[0], prm.fx_sig[1], prm.fx_sigp};
-  const int ebp = fx_base<FINE>(ep), ebuv = fx_base<FINE>(euv);
+  const int ebp = fx_base<false>(ep), ebuv = fx_base<false>(euv);
+  const auto d1 = [&](const long long* c, int st, int eb) {
+    if constexpr (FINE) return fx_d1<ORD>(c, st);
+    else return fx_to<false>(fx_stencil<ORD>(c, st), eb);
+  };
+  (void)ebp;
+  (void)ebuv;
   (void)sN;
   (void)sA;
   (void)sK;
@@ -467,7 +542,7 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
       }
       (void)pre;
       // RHS in units of sigma per component: F_u = sx ku, F_v = sy kv, F_p = sx kp
-      // (tiles outside the fixed-point range, finer unit only: FP64 taps for the interior)
+      // (fx_fine, tiles with values that have no word: FP64 taps for the interior)
       const bool taps = FINE && bad, xfx = xint && !taps, yfx = yint && !taps;
       const auto other_x = [&](const double* line) {
         if (FINE && xint) return fx_taps_global<ORD>(line + I, 1, prm.dx.taps) * prm.fx_isig[0];
@@ -479,20 +554,21 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
       };
       double ku, kv, kp;
       if (xfx) {
-        ku = fx_to<FINE>(fx_stencil<ORD>(cP, 1), ebp);
+        ku = d1(cP, 1, ebp);
       } else {
         ku = other_x(xline + 2 * plane);
       }
       if (yfx) {
-        kv = fx_to<FINE>(fx_stencil<ORD>(cP, PW), ebp);
+        kv = d1(cP, PW, ebp);
       } else {
         kv = other_y(yline + 2 * plane);
       }
       if (xfx && yfx && prm.fx_square) {
-        kp = fx_to<FINE>(fx_stencil<ORD>(cU, 1) + fx_stencil<ORD>(cV, kWaveTX), ebuv);
+        if constexpr (FINE) kp = fx_d1_sum<ORD>(cU, 1, cV, kWaveTX);
+        else kp = fx_to<false>(fx_stencil<ORD>(cU, 1) + fx_stencil<ORD>(cV, kWaveTX), ebuv);
       } else {
-        const double ax = xfx ? fx_to<FINE>(fx_stencil<ORD>(cU, 1), ebuv) : other_x(xline);
-        const double ay = yfx ? fx_to<FINE>(fx_stencil<ORD>(cV, kWaveTX), ebuv) : other_y(yline + plane);
+        const double ax = xfx ? d1(cU, 1, ebuv) : other_x(xline);
+        const double ay = yfx ? d1(cV, kWaveTX, ebuv) : other_y(yline + plane);
         kp = fma(prm.fx_rho, ay, ax);
       }
       if (!FINE && bad) ku = kv = kp = __longlong_as_double(0x7FF8000000000000ll);
@@ -589,23 +665,12 @@ __device__ __forceinline__ void wave_tile_fixed(const WaveParams<double>& prm, c
   }
 }
 
-// Converter warps: the p, u and v boxes of one ring stage to int64 in place.
-// t is the thread's index among the converter threads. The exponent maxima go
-// through one barrier among the converters (fxa, bounded wait): each converter
-// warp writes its own p and u/v maxima to wmax[warp][0..1], every converter then
-// takes the maximum over them, and so does every compute warp later (fx_tile_emax),
-// so nothing has to be reset between tiles. Returns false if the wait ran out.
-template <typename Tile, bool FINE>
-__device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fxa, int* wmax, uint32_t parity,
-                                                 unsigned long long wait_ns, int t);
-
-// The p and u/v exponent maxima of a converted stage from its converter warps'
-// pairs, with the tile guard applied: a box whose maximum is below 64 (values
-// under 2^-959) converts to zeros, and one at 2031 or more (values from 2^1008,
-// Inf, NaN) marks the tile bad. A bad tile is NaN throughout in the stages that do
-// not take the finer unit; those that do evaluate it with FP64 taps from global memory,
-// and tiles whose largest value is nonzero but below 2^-959 as well.
-template <int CONV, bool FINE>
+// What the converter warps leave beside a converted stage, a pair per warp: the exponent maxima
+// of p and of u and v, for stages that take their box's exponent. A box whose maximum is below
+// 64 (values under 2^-959) converts to zeros, and one at 2031 or more (values from 2^1008, Inf,
+// NaN) marks the tile bad: it is NaN throughout. Kernels that evaluate a bad tile with FP64 taps
+// instead (TAPS) want one whose largest value is nonzero but below 2^-959 marked as well.
+template <int CONV, bool TAPS>
 __device__ __forceinline__ void fx_tile_emax(const int* wmax, int& ep, int& euv, bool& bad) {
   ep = 0;
   euv = 0;
@@ -615,54 +680,84 @@ __device__ __forceinline__ void fx_tile_emax(const int* wmax, int& ep, int& euv,
     euv = max(euv, wmax[2 * c + 1]);
   }
   bad = ep >= 2031 || euv >= 2031;
-  if (FINE) bad = bad || (ep > 0 && ep < 64) || (euv > 0 && euv < 64);
+  if (TAPS) bad = bad || (ep > 0 && ep < 64) || (euv > 0 && euv < 64);
   if (ep < 64) ep = 2111;  // every value converts to 0
   if (euv < 64) euv = 2111;
 }
 
+// Of stages on whole values: whether the warp met one without a word. FP64 taps from global
+// memory then evaluate the tile.
+template <int CONV>
+__device__ __forceinline__ bool fx_tile_out(const int* wmax) {
+  int o = 0;
+#pragma unroll
+  for (int c = 0; c < CONV; c++) o |= wmax[2 * c];
+  return o != 0;
+}
+
+// Converter warps: the p, u and v boxes of one ring stage to words (FINE) or to int64 in units
+// of the box's largest exponent, in place. t is the thread's index among the converter
+// threads. Box units: the exponent maxima go through one barrier among the converters (fxa,
+// bounded wait), each of which then takes the maximum over all, and so does every compute warp
+// later, so nothing has to be reset between tiles. Returns false if the wait ran out.
 template <typename Tile, bool FINE>
 __device__ __forceinline__ bool fx_convert_stage(unsigned char* st, uint64_t* fxa, int* wmax, uint32_t parity,
                                                  unsigned long long wait_ns, int t) {
   constexpr int NT = 32 * Tile::CONV;
   constexpr int NP = Tile::PH * Tile::PW, NU = Tile::TY * Tile::PW, NV = Tile::PH * kWaveTX;
-  uint2* wP = reinterpret_cast<uint2*>(st);
-  uint2* wU = reinterpret_cast<uint2*>(st + Tile::OFF_U);
-  uint2* wV = reinterpret_cast<uint2*>(st + Tile::OFF_V);
   const int lane = t & 31, cw = t >> 5;
-  unsigned mp = 0, muv = 0;
-  for (int e = t; e < NP; e += NT) mp = max(mp, wP[e].y & 0x7FF00000u);
-  for (int e = t; e < NU; e += NT) muv = max(muv, wU[e].y & 0x7FF00000u);
-  for (int e = t; e < NV; e += NT) muv = max(muv, wV[e].y & 0x7FF00000u);
-  mp = __reduce_max_sync(0xffffffffu, mp);
-  muv = __reduce_max_sync(0xffffffffu, muv);
-  if (lane == 0) {
-    wmax[2 * cw] = (int)(mp >> 20);
-    wmax[2 * cw + 1] = (int)(muv >> 20);
-  }
-  __syncwarp();
-  if (lane == 0) mbar_arrive(fxa);
-  if (!mbar_wait_bounded(fxa, parity, wait_ns)) return false;
-  int ep, euv;
-  bool bad;
-  fx_tile_emax<Tile::CONV, FINE>(wmax, ep, euv, bad);
-  (void)bad;
-  long long* iP = reinterpret_cast<long long*>(wP);
-  long long* iU = reinterpret_cast<long long*>(wU);
-  long long* iV = reinterpret_cast<long long*>(wV);
+  if constexpr (FINE) {
+    bool out = false;
+    const auto pack = [&](unsigned char* box, int n) {
+      double* d = reinterpret_cast<double*>(box);
+      long long* q = reinterpret_cast<long long*>(box);
 #pragma unroll 4
-  for (int e = t; e < NP; e += NT) {
-    const uint2 w = wP[e];
-    iP[e] = fx_from<FINE>(w.x, w.y, ep);
-  }
+      for (int e = t; e < n; e += NT) q[e] = fx_pack(d[e], out);
+    };
+    pack(st, NP);
+    pack(st + Tile::OFF_U, NU);
+    pack(st + Tile::OFF_V, NV);
+    out = __any_sync(0xffffffffu, out);
+    if (lane == 0) wmax[2 * cw] = out;
+  } else {
+    uint2* wP = reinterpret_cast<uint2*>(st);
+    uint2* wU = reinterpret_cast<uint2*>(st + Tile::OFF_U);
+    uint2* wV = reinterpret_cast<uint2*>(st + Tile::OFF_V);
+    unsigned mp = 0, muv = 0;
+    for (int e = t; e < NP; e += NT) mp = max(mp, wP[e].y & 0x7FF00000u);
+    for (int e = t; e < NU; e += NT) muv = max(muv, wU[e].y & 0x7FF00000u);
+    for (int e = t; e < NV; e += NT) muv = max(muv, wV[e].y & 0x7FF00000u);
+    mp = __reduce_max_sync(0xffffffffu, mp);
+    muv = __reduce_max_sync(0xffffffffu, muv);
+    if (lane == 0) {
+      wmax[2 * cw] = (int)(mp >> 20);
+      wmax[2 * cw + 1] = (int)(muv >> 20);
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(fxa);
+    if (!mbar_wait_bounded(fxa, parity, wait_ns)) return false;
+    int ep, euv;
+    bool bad;
+    fx_tile_emax<Tile::CONV, false>(wmax, ep, euv, bad);
+    (void)bad;
+    long long* iP = reinterpret_cast<long long*>(wP);
+    long long* iU = reinterpret_cast<long long*>(wU);
+    long long* iV = reinterpret_cast<long long*>(wV);
 #pragma unroll 4
-  for (int e = t; e < NU; e += NT) {
-    const uint2 w = wU[e];
-    iU[e] = fx_from<FINE>(w.x, w.y, euv);
-  }
+    for (int e = t; e < NP; e += NT) {
+      const uint2 w = wP[e];
+      iP[e] = fx_from<false>(w.x, w.y, ep);
+    }
 #pragma unroll 4
-  for (int e = t; e < NV; e += NT) {
-    const uint2 w = wV[e];
-    iV[e] = fx_from<FINE>(w.x, w.y, euv);
+    for (int e = t; e < NU; e += NT) {
+      const uint2 w = wU[e];
+      iU[e] = fx_from<false>(w.x, w.y, euv);
+    }
+#pragma unroll 4
+    for (int e = t; e < NV; e += NT) {
+      const uint2 w = wV[e];
+      iV[e] = fx_from<false>(w.x, w.y, euv);
+    }
   }
   // the converted boxes were written through the generic proxy; order those writes
   // before the TMA (async proxy) refills the stage
@@ -755,8 +850,8 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, K
         break;
       }
       const int tile = tslot[b];
-      if (tile >= 0 && !fx_convert_stage<Tile, fx_fine<KIND, STAGE>()>(smem + b * Tile::STAGE_BYTES, &fxa[b], wmax + 16 * b, (k / NST) & 1,
-                                                prm.wait_ns, t)) {
+      if (tile >= 0 && !fx_convert_stage<Tile, fx_fine<KIND, STAGE>()>(smem + b * Tile::STAGE_BYTES, &fxa[b],
+                                                                       wmax + 16 * b, (k / NST) & 1, prm.wait_ns, t)) {
         if (lane == 0) atomicOr(prm.err, ERR_TMA_TIMEOUT);
         break;
       }
@@ -790,9 +885,10 @@ __global__ void __launch_bounds__(fx_kernel_threads<WaveStageTile<double, ORD, K
       j0 = (tile / ntx) * TY;
       g = FxGeom{prm.nx, prm.ny, 0, 0, 0, 0, prm.pitch, prm.plane, 0};
     }
-    int ep, euv;
+    int ep = 0, euv = 0;
     bool bad;
-    fx_tile_emax<CONV, fx_fine<KIND, STAGE>()>(wmax + 16 * b, ep, euv, bad);
+    if constexpr (fx_fine<KIND, STAGE>()) bad = fx_tile_out<CONV>(wmax + 16 * b);
+    else fx_tile_emax<CONV, false>(wmax + 16 * b, ep, euv, bad);
     wave_tile_fixed<ORD, STAGE, Tile, KIND>(prm, g, prm.in, prm.wout, prm.c_acc, prm.c_w, prm.fx_ca, prm.fx_cw,
                                             smem + b * Tile::STAGE_BYTES, i0, j0, warp, lane, ep, euv, bad, &dbar[b],
                                             &dphase, b, k, ct, &errsq);

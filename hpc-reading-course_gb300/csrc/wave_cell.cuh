@@ -8,7 +8,7 @@
 // 32 x 8 points: all its loads are in flight at once, every thread converts
 // the values it loaded, and several CTAs per SM overlap their phases. The same operations
 // in the same order as the persistent kernels in FP32 (bit for bit); in FP64 the same
-// fixed-point stencils, with the exponent maxima of this cell.
+// fixed-point stencils, box units being those of this cell.
 //
 // A CTA:
 //   1. loads p (x and y halo), u (x halo), v (y halo) into registers, and the operands of
@@ -18,7 +18,8 @@
 //      FP64 pipe for the whole sequence), kept in shared memory. Their lines come from L2
 //      (from a copy of the box in shared memory instead: nothing gained at 65^2, 17 %
 //      slower at 1025^2, where the copy and its registers cost CTAs per SM);
-//   3. FP64: exponent maxima over the CTA, conversion to int64; the boxes to shared memory;
+//   3. FP64: conversion to words, or to int64 in units of the cell's largest exponent
+//      (fx_fine); the boxes to shared memory;
 //   4. stencils, SAT and update per point; points on an x face only leave their RHS in
 //      shared memory, and the first warp finishes them, one point per lane.
 // Launched with programmatic stream serialization: the next stage's CTAs may start while
@@ -182,11 +183,20 @@ __global__ void __launch_bounds__(kCellThreads, wave_cell_ctas<STAGE>())
     s_cls[d][yr][col] = s;
   }
 
-  // ---- 3. boxes to shared memory (FP64: as int64 in units of the cell's largest exponent)
+  // ---- 3. boxes to shared memory
   constexpr bool FINE = fx_fine<KIND, STAGE>();
   int ebp = 0, ebuv = 0;
   bool taps = false;  // the cell's values leave the fixed-point range: FP64 taps
-  if constexpr (FIX) {
+  if constexpr (FIX && FINE) {
+    bool out = false;
+#pragma unroll
+    for (int c = 0; c < PER; c++) {
+      const int e = tid + c * kCellThreads;
+      const long long w = fx_pack((double)val[c], out);
+      if (e < C::N) box.i[e] = w;
+    }
+    taps = __syncthreads_or(out);
+  } else if constexpr (FIX) {
     unsigned mp = 0, muv = 0;
 #pragma unroll
     for (int c = 0; c < PER; c++) {
@@ -203,23 +213,24 @@ __global__ void __launch_bounds__(kCellThreads, wave_cell_ctas<STAGE>())
     __syncthreads();
     int ep, euv;
     fx_tile_emax<C::WARPS, true>(&s_max[0][0], ep, euv, taps);
-    ebp = fx_base<FINE>(ep);
-    ebuv = fx_base<FINE>(euv);
+    ebp = fx_base<false>(ep);
+    ebuv = fx_base<false>(euv);
 #pragma unroll
     for (int c = 0; c < PER; c++) {
       const int e = tid + c * kCellThreads;
       const double v = (double)val[c];
       if (e < C::N)
-        box.i[e] = fx_from<FINE>((unsigned)__double2loint(v), (unsigned)__double2hiint(v), e < C::NP ? ep : euv);
+        box.i[e] = fx_from<false>((unsigned)__double2loint(v), (unsigned)__double2hiint(v), e < C::NP ? ep : euv);
     }
+    __syncthreads();
   } else {
 #pragma unroll
     for (int c = 0; c < PER; c++) {
       const int e = tid + c * kCellThreads;
       if (e < C::N) box.f[e] = val[c];
     }
+    __syncthreads();
   }
-  __syncthreads();
 
   // ---- 4. points
   const bool xfaces = prm.bc != BC_NONE && (i0 == 0 || (nx - 1 >= i0 && nx - 1 < i0 + TX));
@@ -303,13 +314,18 @@ __global__ void __launch_bounds__(kCellThreads, wave_cell_ctas<STAGE>())
         if (!yint) return y_closure(comp) * prm.fx_isig[1];
         return taps_by<T, ORD>([&](int q) { return in_at(comp, q, i); }, j, prm.dy.taps) * prm.fx_isig[1];
       };
-      k[0] = xfx ? fx_to<FINE>(fx_stencil<ORD>(box.i + cp, 1), ebp) : other_x(0, 2);
-      k[1] = yfx ? fx_to<FINE>(fx_stencil<ORD>(box.i + cp, PW), ebp) : other_y(2);
+      const auto d1 = [&](int at, int st, int eb) {
+        if constexpr (FINE) return fx_d1<ORD>(box.i + at, st);
+        else return fx_to<false>(fx_stencil<ORD>(box.i + at, st), eb);
+      };
+      k[0] = xfx ? d1(cp, 1, ebp) : other_x(0, 2);
+      k[1] = yfx ? d1(cp, PW, ebp) : other_y(2);
       if (xfx && yfx && prm.fx_square) {
-        k[2] = fx_to<FINE>(fx_stencil<ORD>(box.i + cu, 1) + fx_stencil<ORD>(box.i + cv, TX), ebuv);
+        if constexpr (FINE) k[2] = fx_d1_sum<ORD>(box.i + cu, 1, box.i + cv, TX);
+        else k[2] = fx_to<false>(fx_stencil<ORD>(box.i + cu, 1) + fx_stencil<ORD>(box.i + cv, TX), ebuv);
       } else {
-        const double ax = xfx ? fx_to<FINE>(fx_stencil<ORD>(box.i + cu, 1), ebuv) : other_x(1, 0);
-        const double ay = yfx ? fx_to<FINE>(fx_stencil<ORD>(box.i + cv, TX), ebuv) : other_y(1);
+        const double ax = xfx ? d1(cu, 1, ebuv) : other_x(1, 0);
+        const double ay = yfx ? d1(cv, TX, ebuv) : other_y(1);
         k[2] = fma(prm.fx_rho, ay, ax);
       }
       if constexpr (KIND == WK_VAR) {
