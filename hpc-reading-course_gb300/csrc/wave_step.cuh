@@ -9,18 +9,18 @@
 // halo points (16 x 16 at order 4: 2016 point-stages for 1024), and the FP64 pipe bounds a
 // CTA, so the form pays while every SM has at most one. u^{n+1} goes to another buffer, since
 // neighbours read u^n; two buffers alternate.
-// Measured, us per stage (a step's quarter), cells -> this: order 4 161^2 rho=K=1 6.5 -> 4.5,
-// variable 7.6 -> 5.1, forced 7.5 -> 4.9, 257^2 7.2 -> 6.2, 8.1 -> 7.2, 7.9 -> 7.1; order 2 161^2 5.7
-// -> 3.1, 257^2 6.2 -> 4.8; order 6 161^2 7.3 -> 6.1, 193^2 7.5 -> 6.9. With more cells than SMs it
-// loses (order 4 289^2 9.6 against 7.2).
+// Measured, us per stage (a step's quarter), cells / this: rho=K=1 129^2 6.0 / 3.1, 6.9 / 4.1 and
+// 7.8 / 5.9 at orders 2, 4 and 6, 257^2 6.8 / 4.9 and 7.9 / 6.3 (order 6: 217^2 8.6 / 7.0); variable
+// 129^2 6.6 / 3.9, 7.8 / 4.9, 8.4 / 6.7; forced 6.5 / 3.6, 7.4 / 4.6, 7.8 / 6.6; grids of 20:1 and
+// 1:9 the same gains. With more cells than SMs it loses: some SM then takes two, one after the
+// other (order 4 289^2 9.6 against 7.2).
 //
 // Per stage: the closure sums and the SAT of face points, one per thread (a row of the cell
 // has one to six such points; in the point loop each would hold its warp's FP64 pipe); the
-// points of the stage's rectangle (fixed-point stencils, wave2d_fixed.cuh, the finer unit),
-// their next stage input in registers; the exponent maxima; conversion in place. Closure rows
-// and SAT take the stage input's values back from the integers (exact to 2^-54 of the
-// rectangle's largest value). A rectangle whose values leave the fixed-point range is kept
-// as doubles, and its stencils are FP64 taps.
+// points of the stage's rectangle (fixed-point stencils on words, wave2d_fixed.cuh), their next
+// stage input in registers; conversion to words in place, which hold the values whole: closure
+// rows and SAT take them back. A rectangle with a value that has no word is kept as doubles,
+// and its stencils are FP64 taps.
 #pragma once
 
 #include "wave_cell.cuh"
@@ -43,7 +43,7 @@ template <int ORD, int TC> struct WaveStep {
   static constexpr int P = TC + GROW, N = P * P;  // box side, points
   static constexpr int CR = 4 * CS;               // closure rows a rectangle can have
   static constexpr int PER = (N + kStepThreads - 1) / kStepThreads;
-  // u^n, the stage input (int64), coefficient planes, acc, y-closure sums
+  // u^n, the stage input (words), coefficient planes, acc, y-closure sums
   static constexpr int smem(int planes) { return ((6 + planes) * N + 3 * TC * TC + 2 * CR * P) * 8; }
 };
 
@@ -115,19 +115,18 @@ template <int ORD, int KIND, int TC>
 __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid_constant__ WaveParams<double> prm,
                                                                     const __grid_constant__ WaveStepCoef cf) {
   using S = WaveStep<ORD, TC>;
-  constexpr int CS = S::CS, P = S::P, N = S::N, PER = S::PER, NT = kStepThreads, WARPS = NT / 32;
+  constexpr int CS = S::CS, P = S::P, N = S::N, PER = S::PER, NT = kStepThreads;
   constexpr int NK = KIND == WK_VAR ? 2 : (KIND == WK_MMS ? 3 : 0);
   extern __shared__ __align__(16) unsigned char step_smem[];
   double* const su = reinterpret_cast<double*>(step_smem);         // u^n: [3][N]
-  long long* const si = reinterpret_cast<long long*>(su + 3 * N);  // stage input: [3][N]
+  long long* const si = reinterpret_cast<long long*>(su + 3 * N);  // stage input, as words: [3][N]
   double* const sk = reinterpret_cast<double*>(si + 3 * N);        // coefficients: [NK][N]
   double* const sacc = sk + NK * N;                                // acc: [3][TC * TC]
   double* const scy = sacc + 3 * TC * TC;                          // y-closure sums of p and v: [2][CR][P]
   __shared__ double s_cls[2][P][2 * CS];  // x-closure sums of p and u, units of sigma: [.][row][column]
   __shared__ double s_sat[2][P][2];       // x-face SAT of u and p, units of sigma: [west, east][row]
   __shared__ double s_saty[4][P][2];      // SAT of v and p on rows 0, ny - 1, ys - 1, ys
-  __shared__ int s_max[2][WARPS][2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
   const int nx = prm.nx, ny = prm.ny, ys = KIND == WK_VAR ? prm.ysplit : 0;
   const long long pitch = prm.pitch, plane = prm.plane;
   const int ci = blockIdx.x * TC, cj = blockIdx.y * TC;
@@ -159,7 +158,6 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
 
   // u^n and the coefficients on the box
   double v[PER][3];  // this thread's values of the next stage input
-  unsigned mp = 0, muv = 0;
 #pragma unroll
   for (int c = 0; c < PER; c++) {
     const int e = tid + c * NT;
@@ -173,9 +171,6 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
       }
 #pragma unroll
       for (int m = 0; m < NK; m++) sk[m * N + at(i, j)] = __ldg(prm.rinv + m * plane + q);
-      muv = max(muv, (unsigned)__double2hiint(v[c][0]) & 0x7FF00000u);
-      muv = max(muv, (unsigned)__double2hiint(v[c][1]) & 0x7FF00000u);
-      mp = max(mp, (unsigned)__double2hiint(v[c][2]) & 0x7FF00000u);
     }
   }
   double ct[3] = {0, 0, 0};
@@ -188,37 +183,30 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
 #pragma unroll 1
   for (int s = 0; s < 4; s++) {
     // ---- the stage input to shared memory
-    mp = __reduce_max_sync(0xffffffffu, mp);
-    muv = __reduce_max_sync(0xffffffffu, muv);
-    if (lane == 0) {
-      s_max[s & 1][warp][0] = (int)(mp >> 20);
-      s_max[s & 1][warp][1] = (int)(muv >> 20);
-    }
-    __syncthreads();  // maxima known; every thread has read the previous stage input
-    int ep, euv;
-    bool taps;
-    fx_tile_emax<WARPS, true>(&s_max[s & 1][0][0], ep, euv, taps);
-    const int ebp = fx_base<true>(ep), ebuv = fx_base<true>(euv);
-    {
-      const int w = px1 - px0, n = s == 0 ? bn : (x1[s - 1] - x0[s - 1]) * (y1[s - 1] - y0[s - 1]);
+    const int pw = px1 - px0, pn = s == 0 ? bn : (x1[s - 1] - x0[s - 1]) * (y1[s - 1] - y0[s - 1]);
+    long long word[PER][3];
+    bool out = false;
 #pragma unroll
-      for (int c = 0; c < PER; c++) {
-        const int e = tid + c * NT;
-        if (e < n) {
-          const int r = div(e, w), o = at(px0 + e - r * w, py0 + r);
+    for (int c = 0; c < PER; c++)
+      if (tid + c * NT < pn) {
 #pragma unroll
-          for (int m = 0; m < 3; m++)
-            si[m * N + o] = taps ? __double_as_longlong(v[c][m])
-                                 : fx_from<true>((unsigned)__double2loint(v[c][m]), (unsigned)__double2hiint(v[c][m]),
-                                                 m == 2 ? ep : euv);
-        }
+        for (int m = 0; m < 3; m++) word[c][m] = fx_pack(v[c][m], out);
+      }
+    const bool taps = __syncthreads_or(out);  // and every thread has read the previous stage input
+#pragma unroll
+    for (int c = 0; c < PER; c++) {
+      const int e = tid + c * NT;
+      if (e < pn) {
+        const int r = div(e, pw), o = at(px0 + e - r * pw, py0 + r);
+#pragma unroll
+        for (int m = 0; m < 3; m++) si[m * N + o] = taps ? __double_as_longlong(v[c][m]) : word[c][m];
       }
     }
     __syncthreads();
     // a value of the stage input
     const auto val = [&](int m, int i, int j) {
       const long long q = si[m * N + at(i, j)];
-      return taps ? __longlong_as_double(q) : fx_to<true>(q, m == 2 ? ebp : ebuv);
+      return taps ? __longlong_as_double(q) : fx_unpack(q);
     };
     // ---- x-closure sums and x-face SAT, one per thread
     const int ax0 = x0[s], ax1 = x1[s], ay0 = y0[s], ay1 = y1[s], rows = ay1 - ay0;
@@ -277,7 +265,6 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
     }
     // ---- points
     const int n = w * rows;
-    mp = muv = 0;
 #pragma unroll
     for (int c = 0; c < PER; c++) {
       const int e = tid + c * NT;
@@ -299,15 +286,15 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
       };
       double k[3];
       const bool xfx = xint && !taps, yfx = yint && !taps;
-      if (xfx) k[0] = fx_to<true>(fx_stencil<ORD>(cp, 1), ebp);
+      if (xfx) k[0] = fx_d1<ORD>(cp, 1);
       else k[0] = xint ? x_taps(2) : s_cls[0][r][col];
-      if (yfx) k[1] = fx_to<true>(fx_stencil<ORD>(cp, P), ebp);
+      if (yfx) k[1] = fx_d1<ORD>(cp, P);
       else k[1] = d_y(2);
       if (xfx && yfx && prm.fx_square) {
-        k[2] = fx_to<true>(fx_stencil<ORD>(cu, 1) + fx_stencil<ORD>(cv, P), ebuv);
+        k[2] = fx_d1_sum<ORD>(cu, 1, cv, P);
       } else {
-        const double ax = xfx ? fx_to<true>(fx_stencil<ORD>(cu, 1), ebuv) : (xint ? x_taps(0) : s_cls[1][r][col]);
-        const double ay = yfx ? fx_to<true>(fx_stencil<ORD>(cv, P), ebuv) : d_y(1);
+        const double ax = xfx ? fx_d1<ORD>(cu, 1) : (xint ? x_taps(0) : s_cls[1][r][col]);
+        const double ay = yfx ? fx_d1<ORD>(cv, P) : d_y(1);
         k[2] = fma(prm.fx_rho, ay, ax);
       }
       if constexpr (KIND == WK_VAR) {
@@ -346,11 +333,6 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
         } else {
           prm.wout[m * plane + (long long)j * pitch + i] = fma(cf.ca[0][m], k[m], sacc[m * TC * TC + oa]);
         }
-      }
-      if (s < 3) {
-        muv = max(muv, (unsigned)__double2hiint(v[c][0]) & 0x7FF00000u);
-        muv = max(muv, (unsigned)__double2hiint(v[c][1]) & 0x7FF00000u);
-        mp = max(mp, (unsigned)__double2hiint(v[c][2]) & 0x7FF00000u);
       }
     }
     px0 = ax0, px1 = ax1, py0 = ay0;
