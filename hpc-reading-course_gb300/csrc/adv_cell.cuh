@@ -3,12 +3,14 @@
 //
 // line_stage_kernel's form (one thread per point, every tap a global load) issues eight FP64
 // FMAs of taps per point at order 4 on a pipe that takes 19 clocks per warp instruction and SM:
-// 5.8 clocks per point. Here the cell's box of u is loaded once and converted to int64
-// (wave2d_fixed.cuh, the finer unit), the interior stencils are integer sums, and the FP64
-// pipe keeps the two scalings and the update. A thread takes ROWS rows of a column, whose
-// values it reads from shared memory once. x-closure sums: one per thread, as in
-// wave_cell.cuh, whose notes on overlapped launches and ld.cg apply here. The FP64 pipe still
-// bounds it (four instructions per point: 2.4 of 3.4 clocks at 2049^2).
+// 5.8 clocks per point. Here the cell's box of u is loaded once and converted to words
+// (wave2d_fixed.cuh), the interior stencils are integer sums, and the FP64 pipe keeps the two
+// scalings and the update. A thread takes ROWS rows of a column. x-closure sums: one per thread,
+// as in wave_cell.cuh, whose notes on overlapped launches and ld.cg apply here. Measured, us per
+// stage, line form -> this: 2049^2 70 -> 44, 103 -> 50 and 137 -> 59 at orders 2, 4 and 6, with
+// velocity fields 89 -> 68, 122 -> 73, 154 -> 77; 801^2 order 4 19.9 -> 10.4. The FP64 pipe (four
+// instructions per point: 2.4 of 3.5 clocks at 2049^2 order 4) and the integer instructions
+// bound it together.
 #pragma once
 
 #include "line_kernels.cuh"
@@ -19,13 +21,11 @@ namespace sbp {
 // FIELDS: a velocity at every point (one kernel for both would execute both forms' FP64
 // instructions, seven per point instead of four).
 template <int ORD, int STAGE, bool FIELDS, int ROWS>
-__global__ void __launch_bounds__(kCellThreads, ROWS > 2 ? 3 : 4) adv_cell_kernel(const __grid_constant__ LineParams<double> prm) {
+__global__ void __launch_bounds__(kCellThreads, 4) adv_cell_kernel(const __grid_constant__ LineParams<double> prm) {
   constexpr int R = OpShape<ORD>::W / 2, CS = OpShape<ORD>::CS, TX = kCellTX, TY = kCellThreads / 32 * ROWS;
   constexpr int PW = TX + 2 * R, N = (TY + 2 * R) * PW, PER = (N + kCellThreads - 1) / kCellThreads;
-  constexpr int WARPS = kCellThreads / 32;
   __shared__ long long box[N];
   __shared__ double s_cls[TY][2 * CS];
-  __shared__ int s_max[WARPS][2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nx = prm.nx, ny = prm.ny, i0 = blockIdx.x * TX, j0 = blockIdx.y * TY, i = i0 + lane;
   const int y0 = warp * ROWS;  // this thread's points: column i, rows j0 + y0 ..
@@ -60,45 +60,34 @@ __global__ void __launch_bounds__(kCellThreads, ROWS > 2 ? 3 : 4) adv_cell_kerne
     const int I = col < wcols ? col : e0 + col - wcols;
     if (jr < ny) s_cls[yr][col] = closure_by<double, ORD>([&](int k) { return in_at(jr, k); }, nx, I, prm.dx.cls);
   }
-  unsigned m = 0;
-#pragma unroll
-  for (int c = 0; c < PER; c++) m = max(m, (unsigned)__double2hiint(val[c]) & 0x7FF00000u);
-  m = __reduce_max_sync(0xffffffffu, m);
-  if (lane == 0) s_max[warp][0] = s_max[warp][1] = (int)(m >> 20);
-  __syncthreads();
-  int ep, same;
-  bool taps;  // the cell's values leave the fixed-point range: FP64 taps
-  fx_tile_emax<WARPS, true>(&s_max[0][0], ep, same, taps);
-  const int eb = fx_base<true>(ep);
+  bool out = false;
 #pragma unroll
   for (int c = 0; c < PER; c++) {
     const int e = tid + c * kCellThreads;
-    if (e < N)
-      box[e] = fx_from<true>((unsigned)__double2loint(val[c]), (unsigned)__double2hiint(val[c]), ep);
+    const long long w = fx_pack(val[c], out);
+    if (e < N) box[e] = w;
   }
-  __syncthreads();
+  const bool taps = __syncthreads_or(out);  // a value without a word: FP64 taps
   if (i >= nx) return;
   const bool xint = i >= CS && i < nx - CS;
   const int ccol = i < CS ? i : wcols + (i - e0);
-  long long col[ROWS + 2 * R];  // the column's values around this thread's rows
-#pragma unroll
-  for (int r = 0; r < ROWS + 2 * R; r++) col[r] = box[(y0 + r) * PW + lane + R];
 #pragma unroll
   for (int r = 0; r < ROWS; r++) {
     const int y = y0 + r, j = j0 + y;
     if (j >= ny) break;
     const long long q = (long long)j * pitch + i;
+    const long long* at = box + (y + R) * PW + lane + R;
     // derivative = factor * value per direction: a stencil sum in units of sigma, or a
     // closure or tap sum already scaled
     double dx, dy, fx = 1.0, fy = 1.0;
     if (xint && !taps) {
-      dx = fx_to<true>(fx_stencil<ORD>(box + (y + R) * PW + lane + R, 1), eb);
+      dx = fx_d1<ORD>(at, 1);
       fx = prm.fx_sig[0];
     } else {
       dx = xint ? taps_by<double, ORD>([&](int p) { return in_at(j, p); }, i, prm.dx.taps) : s_cls[y][ccol];
     }
     if (j >= CS && j < ny - CS && !taps) {
-      dy = fx_to<true>(fx_stencil<ORD>(col + r + R, 1), eb);
+      dy = fx_d1<ORD>(at, PW);
       fy = prm.fx_sig[1];
     } else if (j >= CS && j < ny - CS) {
       dy = taps_by<double, ORD>([&](int p) { return in_at(p, i); }, j, prm.dy.taps);

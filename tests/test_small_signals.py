@@ -160,3 +160,22 @@ def test_wave_2d(sbp, port, kind, nx, ny, order, form):
             assert st["accepted"] == 1
             ref = port.rk45(pb, v.ravel(), t, t + dt, dt, atol=1e30, rtol=0.0)[0]
             within(ctx.get_state(), ref, step_bound(bar, RKF, v, fmax, dt), shape)
+
+
+@pytest.mark.parametrize("field", [False, True], ids=["constant", "field"])
+@pytest.mark.parametrize("order", [2, 4, 6])
+def test_advection_2d(sbp, port, order, field):
+    for nx, ny in ((205, 203), (703, 651)):  # one and two rows per thread
+        kw = {"a": 1.5, "b": -1.0}
+        if field:
+            rng = np.random.default_rng(nx)
+            kw.update(a_field=rng.uniform(-1, 1, nx * ny), b_field=rng.uniform(-1, 1, nx * ny))
+        pb = O.Problem(O.ADVECTION_2D, order, nx, ny, **kw)
+        shape = (ny, nx, 1)
+        v = steep(shape, order, fall=(300 / nx, 200 / ny), top=0)
+        v *= 2.0 ** -(8.0 * (np.arange(nx) % 32))[None, :, None]  # and within every cell
+        bar, dt = Bar(port, pb), 0.05 / nx
+        with sbp.Context(sbp.ADVECTION_2D, order, nx, ny, **kw) as ctx:
+            within(ctx.rhs(v.ravel()), port.rhs(pb, v.ravel()), 64 * EPS * bar(np.abs(v)), shape)
+            within(ctx.rk4(v.ravel(), 0.0, dt, 1), port.rk4(pb, v.ravel(), 0.0, dt, 1),
+                   step_bound(bar, RK4, v, 0.0, dt), shape)
