@@ -418,9 +418,10 @@ inline bool w3_force_column() {
 // z planes per CTA of the fixed-point kernel. A CTA converts 2R planes more than it computes,
 // but CTAs on a face take longer than inner ones, so a grid wants several waves of them: 12
 // planes where that leaves four waves of two CTAs per SM, fewer (down to 4) on smaller grids.
-// us per stage at order 4 with 4 / 6 / 8 / 12 / 24 / 48 planes: 49^3 38 / 36 / 45 / 65 / 122 / 239,
-// 97^3 111 / 116 / 115 / 143 / 174 / 240, 201 x 193 x 161 406 / 394 / 389 / 382 / 406 / 471,
-// 256^3 896 / 851 / 841 / 817 / 824 / 891.
+// us per stage with 4 / 6 planes at least: 49^3 24.0 / 26.2, 38.3 / 36.1, 46.1 / 45.4 at orders 2,
+// 4 and 6, 220 x 40 x 40 29.9 / 36.1, 44.6 / 49.6, 53.9 / 60.4; with 8 / 12 / 16 / 24 at most:
+// 201 x 193 x 161 291 / 291 / 304 / 323, 396 / 388 / 407 / 428, 460 / 446 / 467 / 491, 256^3 638 /
+// 626 / 641 / 637, 859 / 831 / 850 / 837, 994 / 955 / 973 / 954.
 inline int fixed3_chunk(long long columns, int nz) {
   const long long z = columns * nz / (4 * 2 * device_sm_count());
   return (int)(z < 4 ? 4 : (z > 12 ? 12 : z));

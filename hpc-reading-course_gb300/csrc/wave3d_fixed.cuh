@@ -5,24 +5,21 @@
 // copies; at 12 warps per SM it took 700 clocks per warp and plane. Here a CTA of 256 threads
 // owns a 32 x 8 column of points and marches along z: one thread issues the next planes' TMA
 // boxes, all threads convert an arriving plane's p, w and the current plane's u, v boxes to
-// int64 in place (wave2d_fixed.cuh, the finer unit), and the stencils are integer sums; the
-// FP64 pipe keeps the update and, for p, the two spacing ratios: nine instructions.
-// Measured, us per stage, plane ring -> this: order 4 49^3 50 -> 38, 97^3 138 -> 111,
-// 201 x 193 x 161 552 -> 382, 256^3 1273 -> 817; order 2 256^3 838 -> 681; order 6 1764 -> 926.
-// What bounds it now: the instructions (about 750 per warp and plane, a quarter conversions,
-// IPC 2.2) and the FP64 pipe (half busy). Closure sums of the x columns shared out one per
-// thread and x-face SAT on one warp, as in the 2D cells, measured slower here (two more
-// barriers per plane: 201 x 193 x 161 401).
+// words in place (wave2d_fixed.cuh), and the stencils are integer sums; the FP64 pipe keeps the
+// update and, for p, the two spacing ratios: nine instructions.
+// Measured, us per stage, plane ring -> this: order 4 49^3 50 -> 38, 97^3 138 -> 112,
+// 201 x 193 x 161 552 -> 388, 256^3 1273 -> 831; order 2 256^3 838 -> 626; order 6 1764 -> 955.
+// What bounds it now: the integer instructions and the FP64 pipe. Closure sums of the x columns
+// shared out one per thread and x-face SAT on one warp, as in the 2D cells, measured slower here
+// (two more barriers per plane).
 //
 // Rings, by plane: A holds p (x halo HX, y halo R) and w of planes k .. k + R and those in
-// flight (a thread keeps its column's p and w along z in registers), B holds u (x halo), v (y halo) and the point boxes the stage update reads. Each
-// group of boxes (plane m in A, plane m - R in B) completes one mbarrier; waits are bounded.
-// Per plane two block barriers: "maxima known" (before it every thread has left the previous
-// plane, so the slots that plane read may be refilled) and "converted".
-// The exponent maximum is per plane and box group, so along z the window's values are brought
-// to the largest exponent of their planes by shifts; they are seldom needed.
-// Closure rows and planes whose values leave the fixed-point range take FP64 taps from global
-// memory; SAT in true units.
+// flight (a thread keeps its column's p and w along z in registers), B holds u (x halo), v (y
+// halo) and the point boxes the stage update reads. Each group of boxes (plane m in A, plane m - R in B) completes one mbarrier; waits are bounded.
+// Per plane one block barrier, "converted": past it every thread has left the previous plane, so
+// that the slots that plane read may be refilled.
+// Closure rows and planes with a value that has no word take FP64 taps from global memory; SAT
+// in true units.
 #pragma once
 
 #include "line_kernels.cuh"
@@ -115,21 +112,18 @@ __device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
-__device__ __forceinline__ bool fx_in_range(int e) { return e == 0 || (e >= 64 && e < 2031); }
-
 template <int ORD, int STAGE>
 __global__ void __launch_bounds__(kF3Threads, 2)
     wave3d_fixed_kernel(const __grid_constant__ Wave3Maps maps, const __grid_constant__ Wave3Params<double> prm,
                         const int zchunk) {
   using G = Fixed3<ORD, STAGE>;
   constexpr int R = G::R, W = G::W, CS = OpShape<ORD>::CS, TX = G::TX, TY = G::TY, PX = G::PX, D = G::D;
-  constexpr int SA = G::SA, SB = G::SB, WARPS = kF3Threads / 32;
+  constexpr int SA = G::SA, SB = G::SB;
   extern __shared__ __align__(128) unsigned char f3_smem[];
   double* const sA = reinterpret_cast<double*>(f3_smem);
   double* const sB = sA + SA * G::A_SZ;
   __shared__ uint64_t full[SA];
-  __shared__ __align__(16) int s_max[2][WARPS][4];  // exponent maxima of p, w, u and v (u, v: one group), by plane parity
-  __shared__ int s_stop;
+  __shared__ int s_out[3][2];  // by group modulo 3: its p or w, its u or v boxes hold a value without a word
   if (prm.skip && *prm.skip) return;
   const int nx = prm.nx, ny = prm.ny, nz = prm.nz;
   const int pitch = (int)prm.pitch, slab = (int)prm.slab, plane = (int)prm.plane;  // 4 * plane < 2^31 (host)
@@ -143,9 +137,9 @@ __global__ void __launch_bounds__(kF3Threads, 2)
   const int k0 = blockIdx.z * zchunk, k1 = k0 + zchunk < nz ? k0 + zchunk : nz;
   if (tid == 0) {
     for (int s = 0; s < SA; s++) mbar_init(&full[s], 1);
-    s_stop = 0;
     fence_barrier_init();
   }
+  if (tid < 6) s_out[tid / 2][tid % 2] = 0;
   __syncthreads();
 
   // Group g (0, 1, ...): plane k0 - R + g of p and w into A's slot g % SA; from g = 2R on, while
@@ -174,17 +168,11 @@ __global__ void __launch_bounds__(kF3Threads, 2)
   if (tid == 0)
     for (; issued < D + 1; issued++) issue(issued);
 
-  // register windows along z of this thread's column, planes k - R .. k + R, and the planes'
-  // exponent maxima (0: a plane of zeros)
+  // register windows along z of this thread's column, planes k - R .. k + R
   long long zp[W], zw[W];
-  int ezp[W], ezw[W];
 #pragma unroll
-  for (int s = 0; s < W; s++) {
-    zp[s] = zw[s] = 0;
-    ezp[s] = ezw[s] = -1;
-  }
-  int same = 0;          // latest planes in a row with equal exponents (p and w each)
-  unsigned usable = ~0u;  // bit s: the plane s before the latest is within the fixed-point range
+  for (int s = 0; s < W; s++) zp[s] = zw[s] = kFxNone;
+  unsigned usable = ~0u;  // bit s: every value of the plane s before the latest has a word
   const int pc = (ty + R) * PX + tx + G::HX, wc = ty * TX + tx, uc = ty * PX + tx + G::HX, vc = (ty + R) * TX + tx;
 
 #pragma unroll 1
@@ -193,37 +181,29 @@ __global__ void __launch_bounds__(kF3Threads, 2)
     const bool own = kb >= k0;
     double* a = sA + sa * G::A_SZ;
     double* b = sB + (own ? (kb - k0) % SB : 0) * G::B_SZ;
-    if (!mbar_wait_bounded(&full[sa], (g / SA) & 1)) s_stop = 1;  // the copy will not complete
-    // exponent maxima of the arriving boxes
-    double va[G::PER_A], vb[G::PER_B];
-    unsigned mp = 0, mw = 0, muv = 0;
+    long long* ia = reinterpret_cast<long long*>(a);
+    long long* ib = reinterpret_cast<long long*>(b);
+    const bool late = !mbar_wait_bounded(&full[sa], (g / SA) & 1);  // the copy will not complete
+    bool outa = false, outb = false;
 #pragma unroll
     for (int c = 0; c < G::PER_A; c++) {
       const int e = tid + c * kF3Threads;
-      va[c] = e < G::NP ? a[e] : (e < G::NP + G::NW ? a[G::A_W + e - G::NP] : 0.0);
-      const unsigned h = (unsigned)__double2hiint(va[c]) & 0x7FF00000u;
-      if (e < G::NP) mp = max(mp, h);
-      else mw = max(mw, h);
+      if (e < G::NP) ia[e] = fx_pack(a[e], outa);
+      else if (e < G::NP + G::NW) ia[G::A_W + e - G::NP] = fx_pack(a[G::A_W + e - G::NP], outa);
     }
     if (own) {
 #pragma unroll
       for (int c = 0; c < G::PER_B; c++) {
         const int e = tid + c * kF3Threads;
-        vb[c] = e < G::NU ? b[e] : (e < G::NU + G::NV ? b[G::B_V + e - G::NU] : 0.0);
-        muv = max(muv, (unsigned)__double2hiint(vb[c]) & 0x7FF00000u);
+        if (e < G::NU) ib[e] = fx_pack(b[e], outb);
+        else if (e < G::NU + G::NV) ib[G::B_V + e - G::NU] = fx_pack(b[G::B_V + e - G::NU], outb);
       }
     }
-    mp = __reduce_max_sync(0xffffffffu, mp);
-    mw = __reduce_max_sync(0xffffffffu, mw);
-    muv = __reduce_max_sync(0xffffffffu, muv);
-    int(*mx)[4] = s_max[g & 1];
-    if (tx == 0) {
-      mx[ty][0] = (int)(mp >> 20);
-      mx[ty][1] = (int)(mw >> 20);
-      mx[ty][2] = (int)(muv >> 20);
-    }
-    __syncthreads();  // maxima known; every thread has left the previous plane
-    if (s_stop) {     // uniform: written before the barrier, read after it
+    if (outa) s_out[g % 3][0] = 1;
+    if (outb) s_out[g % 3][1] = 1;
+    // order the generic writes before the TMA that refills these slots
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    if (__syncthreads_or(late)) {  // converted; every thread has left the previous plane
       if (tid == 0) {
         atomicOr(prm.err, ERR_TMA_TIMEOUT);
         // let the copies in flight land (bounded) before the CTA's shared memory goes
@@ -232,87 +212,37 @@ __global__ void __launch_bounds__(kF3Threads, 2)
       return;
     }
     if (tid == 0 && issued < groups) issue(issued++);  // into slots the previous planes have left
-    int ep, ew, euv;
-    {  // lane l of every warp reads warp l & 7's maxima
-      const int4 m4 = *reinterpret_cast<const int4*>(mx[tx & (WARPS - 1)]);
-      ep = __reduce_max_sync(0xffffffffu, m4.x);
-      ew = __reduce_max_sync(0xffffffffu, m4.y);
-      euv = __reduce_max_sync(0xffffffffu, m4.z);
-    }
-    // outside the fixed-point range (or zero): convert to zeros, the taps take over
-    const int cp = fx_in_range(ep) && ep ? ep : 2111, cw = fx_in_range(ew) && ew ? ew : 2111;
-    const int cuv = fx_in_range(euv) && euv ? euv : 2111;
-    long long* ia = reinterpret_cast<long long*>(a);
-    long long* ib = reinterpret_cast<long long*>(b);
-#pragma unroll
-    for (int c = 0; c < G::PER_A; c++) {
-      const int e = tid + c * kF3Threads;
-      const long long q = fx_from<true>((unsigned)__double2loint(va[c]), (unsigned)__double2hiint(va[c]),
-                                        e < G::NP ? cp : cw);
-      if (e < G::NP) ia[e] = q;
-      else if (e < G::NP + G::NW) ia[G::A_W + e - G::NP] = q;
-    }
-    if (own) {
-#pragma unroll
-      for (int c = 0; c < G::PER_B; c++) {
-        const int e = tid + c * kF3Threads;
-        const long long q = fx_from<true>((unsigned)__double2loint(vb[c]), (unsigned)__double2hiint(vb[c]), cuv);
-        if (e < G::NU) ib[e] = q;
-        else if (e < G::NU + G::NV) ib[G::B_V + e - G::NU] = q;
-      }
-    }
-    // order the generic writes before the TMA that refills these slots
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();  // converted
+    usable = usable << 1 | (s_out[g % 3][0] == 0);
+    const bool uv_words = s_out[g % 3][1] == 0;
+    if (tid < 2) s_out[(g + 2) % 3][tid] = 0;  // group g - 1's, read by all before the barrier
 #pragma unroll
     for (int s = 0; s + 1 < W; s++) {
       zp[s] = zp[s + 1];
       zw[s] = zw[s + 1];
-      ezp[s] = ezp[s + 1];
-      ezw[s] = ezw[s + 1];
     }
     zp[W - 1] = ia[pc];
     zw[W - 1] = ia[G::A_W + wc];
-    same = ep == ezp[W - 2] && ew == ezw[W - 2] ? same + 1 : 1;
-    usable = usable << 1 | (fx_in_range(ep) && fx_in_range(ew) ? 1u : 0u);
-    ezp[W - 1] = ep;
-    ezw[W - 1] = ew;
     if (!own || !live) continue;
 
     const int k = kb, xo = k * slab + j * pitch, q = xo + i;
-    const bool fx = fx_in_range(euv) && (usable & ((1u << W) - 1)) == (1u << W) - 1;
-    int mzp = ep, mzw = ew;  // largest exponents of the window
-    if (same < W) {
-#pragma unroll
-      for (int s = 0; s < W; s++) {
-        mzp = max(mzp, ezp[s]);
-        mzw = max(mzw, ezw[s]);
-      }
-    }
+    const bool fx = uv_words && (usable & ((1u << W) - 1)) == (1u << W) - 1;
     const long long* ap = reinterpret_cast<const long long*>(sA + (g - R) % SA * G::A_SZ);  // plane k's p
-    const auto z_sum = [&](const long long (&z)[W], const int (&e)[W], int mz) {
-      if (same >= W) return fx_stencil<ORD>(z + R, 1);
-      long long t[W];
-#pragma unroll
-      for (int s = 0; s < W; s++) t[s] = z[s] >> min(63, mz - e[s]);
-      return fx_stencil<ORD>(t + R, 1);
-    };
     const bool xint = i >= CS && i < nx - CS, yint = j >= CS && j < ny - CS, zint = k >= CS && k < nz - CS;
     const auto far = [&](const double* line, int st, int n, int at, const DirTaps<double>& d, double isig) {
       return d1_line<double, ORD>(line, st, n, at, d) * isig;
     };
     double kf[4];  // the RHS in units of sigma
-    kf[0] = xint && fx ? fx_to<true>(fx_stencil<ORD>(ap + pc, 1), fx_base<true>(ezp[R]))
+    kf[0] = xint && fx ? fx_d1<ORD>(ap + pc, 1)
                        : far(P + xo, 1, nx, i, prm.dx, prm.fx_isig[0]);
-    kf[1] = yint && fx ? fx_to<true>(fx_stencil<ORD>(ap + pc, PX), fx_base<true>(ezp[R]))
+    kf[1] = yint && fx ? fx_d1<ORD>(ap + pc, PX)
                        : far(P + (k * slab + i), pitch, ny, j, prm.dy, prm.fx_isig[1]);
-    kf[2] = zint && fx ? fx_to<true>(z_sum(zp, ezp, mzp), fx_base<true>(mzp))
+    kf[2] = zint && fx ? fx_d1<ORD>(zp + R, 1)
                        : far(P + (j * pitch + i), slab, nz, k, prm.dz, prm.fx_isig[2]);
-    const double ux = xint && fx ? fx_to<true>(fx_stencil<ORD>(ib + uc, 1), fx_base<true>(euv))
+    const double ux = xint && fx ? fx_d1<ORD>(ib + uc, 1)
                                  : far(U + xo, 1, nx, i, prm.dx, prm.fx_isig[0]);
-    const double vy = yint && fx ? fx_to<true>(fx_stencil<ORD>(ib + G::B_V + vc, TX), fx_base<true>(euv))
+    const double vy = yint && fx ? fx_d1<ORD>(ib + G::B_V + vc, TX)
                                  : far(V + (k * slab + i), pitch, ny, j, prm.dy, prm.fx_isig[1]);
-    const double wz = zint && fx ? fx_to<true>(z_sum(zw, ezw, mzw), fx_base<true>(mzw))
+    const double wz = zint && fx ? fx_d1<ORD>(zw + R, 1)
                                  : far(Wc + (j * pitch + i), slab, nz, k, prm.dz, prm.fx_isig[2]);
     kf[3] = fma(prm.fx_rho[1], wz, fma(prm.fx_rho[0], vy, ux));
 

@@ -179,3 +179,18 @@ def test_advection_2d(sbp, port, order, field):
             within(ctx.rhs(v.ravel()), port.rhs(pb, v.ravel()), 64 * EPS * bar(np.abs(v)), shape)
             within(ctx.rk4(v.ravel(), 0.0, dt, 1), port.rk4(pb, v.ravel(), 0.0, dt, 1),
                    step_bound(bar, RK4, v, 0.0, dt), shape)
+
+
+@pytest.mark.parametrize("bc", [0, 1])
+@pytest.mark.parametrize("order", [2, 4, 6])
+def test_wave_3d(sbp, port, order, bc):
+    nx, ny, nz = 66, 21, 19
+    pb = O.Problem(O.WAVE_3D, order, nx, ny, nz=nz, bc=bc)
+    shape = (nz, ny, nx, 4)
+    bar, dt = Bar(port, pb), 0.1 / nx
+    for fall in ((3, 2, 1), (1, 2, 9)):
+        v = steep(shape, order, fall=fall)
+        with sbp.Context(sbp.WAVE_3D, order, nx, ny, nz, bc=bc) as ctx:
+            within(ctx.rhs(v.ravel()), port.rhs(pb, v.ravel()), 64 * EPS * bar(np.abs(v)), shape)
+            within(ctx.rk4(v.ravel(), 0.0, dt, 1), port.rk4(pb, v.ravel(), 0.0, dt, 1),
+                   step_bound(bar, RK4, v, 0.0, dt), shape)
