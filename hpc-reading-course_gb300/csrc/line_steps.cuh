@@ -46,8 +46,8 @@ __device__ __forceinline__ bool fx_local(const double* c, double& out) {
   unsigned m = 0;
 #pragma unroll
   for (int k = 1; k <= R; k++) {
-    m = max(m, (unsigned)__double2hiint(c[k]) & 0x7FF00000u);
-    m = max(m, (unsigned)__double2hiint(c[-k]) & 0x7FF00000u);
+    m = max(m, (unsigned)__double2hiint(c[k]) & 0x7FFFFFFFu);
+    m = max(m, (unsigned)__double2hiint(c[-k]) & 0x7FFFFFFFu);
   }
   const int emax = (int)(m >> 20);
   long long d[R];  // v_k - v_-k
@@ -61,7 +61,12 @@ __device__ __forceinline__ bool fx_local(const double* c, double& out) {
   if constexpr (ORD == 4) s = 8 * d[0] - d[1];
   if constexpr (ORD == 6) s = 45 * d[0] - 9 * d[1] + d[2];
   out = fx_to<true>(s, fx_base<true>(emax));
-  return emax == 0 || (emax >= 64 && emax < 2031);
+  if (m - (64u << 20) < (2031u - 64u) << 20) return true;
+  if (m) return false;
+  unsigned lo = 0;  // zeros, whose sum is 0, or subnormals
+#pragma unroll
+  for (int k = 1; k <= R; k++) lo |= (unsigned)__double2loint(c[k]) | (unsigned)__double2loint(c[-k]);
+  return lo == 0;
 }
 
 template <typename T, int ORD, int KIND>

@@ -194,3 +194,26 @@ def test_wave_3d(sbp, port, order, bc):
             within(ctx.rhs(v.ravel()), port.rhs(pb, v.ravel()), 64 * EPS * bar(np.abs(v)), shape)
             within(ctx.rk4(v.ravel(), 0.0, dt, 1), port.rk4(pb, v.ravel(), 0.0, dt, 1),
                    step_bound(bar, RK4, v, 0.0, dt), shape)
+
+
+@pytest.mark.parametrize("order", [2, 4, 6])
+def test_line_steps(sbp, port, order):
+    """1D step loops: a steep line, and a stretch of subnormal values, whose products round at
+    2^-1074 (up to 16 of them per stage and point, each times dt)."""
+    n = 150
+    pb = O.Problem(O.ADVECTION_1D, order, n)
+    bar, dt = Bar(port, pb), 0.1 / n
+    shape = (n, 1)
+    rng = np.random.default_rng(order)
+    for v in (steep(shape, order, fall=(5,)), rng.uniform(0.5, 1.0, shape) * 2.0 ** -1030,
+              rng.uniform(0.5, 1.0, shape) * 2.0 ** np.where(np.arange(n) < 70, -1030.0, -900.0)[:, None]):
+        with sbp.Context(sbp.ADVECTION_1D, order, n) as ctx:
+            bound = step_bound(lambda w: bar_1d(bar, pb, w), RK4, v, 0.0, dt) + 64 * 2.0 ** -1074
+            within(ctx.rk4(v.ravel(), 0.0, dt, 1), port.rk4(pb, v.ravel(), 0.0, dt, 1), bound, shape)
+
+
+def bar_1d(bar, pb, v):
+    out = bar.d[0] @ v
+    for at in (0, -1):
+        out[at] += pb.hix * HINV[pb.order] * v[at]
+    return out
