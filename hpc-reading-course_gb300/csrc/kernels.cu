@@ -45,12 +45,18 @@ cudaError_t adv_cell_stage(int stage, const LineParams<double>& prm, cudaStream_
 template <typename T, int ORD, int KIND>
 cudaError_t line_stage(int stage, const LineParams<T>& prm, cudaStream_t s) {
   if constexpr (KIND == LK_ADV2D && sizeof(T) == 8) {
-    // us per stage at order 4, line form / cells of one / two rows per thread: 129^2 3.2 / 3.5 /
-    // 4.5, 257^2 4.4 / 4.0 / 5.4, 513^2 11.7 / 5.9 / 6.2, 801^2 19.6 / 10.3 / 10.0, 1025^2 29.3 /
-    // 14.9 / 13.9, 2049^2 103 / 56 / 47 (four rows: 49)
+    // us per stage, line form / cells of one row per thread: order 2 201^2 3.8 / 3.8, 257^2 4.0 /
+    // 4.3, 801x101 4.1 / 3.8, 361^2 5.4 / 4.6, 513^2 8.5 / 5.3; order 4 161^2 3.5 / 3.7, 201^2 4.9 /
+    // 3.5, 513^2 12.0 / 6.1; order 6 161^2 4.1 / 4.5, 201^2 5.9 / 4.5. With velocity fields: order 2
+    // 257^2 5.9 / 7.8, 361^2 7.5 / 8.1, 401^2 8.2 / 8.1, 513^2 13.5 / 9.3; order 4 161^2 4.6 / 6.0,
+    // 201^2 6.7 / 5.9, 257^2 6.8 / 7.0, 361^2 9.0 / 7.7; order 6 161^2 5.3 / 7.2, 201^2 7.7 / 6.7.
+    // Cells of one / two rows: 513^2 5.3 / 6.0, 6.1 / 6.4, 7.3 / 7.3 at orders 2, 4 and 6, 801^2 9.1 /
+    // 9.0, 10.7 / 10.4, 12.9 / 12.2, 2049^2 48 / 44, 57 / 50, 69 / 59; with fields 801^2 14.7 / 16.0,
+    // 15.4 / 16.5, 16.7 / 17.5, 1001^2 19.7 / 20.7, 20.6 / 21.4, 22.6 / 22.7, 2049^2 71 / 68, 79 / 73,
+    // 89 / 77.
     const long long points = (long long)prm.nx * prm.ny;
-    if (points > 40000) {
-      if (points <= 450000)
+    if (points > (ORD == 2 ? (prm.va ? 160000 : 80000) : 40000)) {
+      if (points <= (prm.va ? 1100000 : 450000))
         return prm.va ? adv_cell_stage<ORD, true, 1>(stage, prm, s) : adv_cell_stage<ORD, false, 1>(stage, prm, s);
       return prm.va ? adv_cell_stage<ORD, true, 2>(stage, prm, s) : adv_cell_stage<ORD, false, 2>(stage, prm, s);
     }

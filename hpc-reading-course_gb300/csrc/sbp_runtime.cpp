@@ -123,23 +123,31 @@ int wave_kind(const sbp_ctx* ctx) {
   return has_fields(ctx->d.problem) ? WK_VAR : WK_MMS;
 }
 
-// Whether a stage of a 2D wave context runs in its cell form (wave_cell.cuh) rather than
-// the persistent one. The cell form's short CTAs win until a grid gives every SM enough
-// tiles to fill the persistent pipeline. Measured, us per RK4 stage at order 4, cell /
-// persistent:
-//                    129^2       513^2        769^2        1025^2       1281^2       1537^2
-//   FP64 rho=K=1   6.3 / 11.5  10.3 / 18.2  17.1 / 22.4  27.6 / 30.3  42.6 / 41.4  58.2 / 54.0
-//   FP64 var.      7.8 / 13.2  13.1 / 21.1  21.8 / 27.5  37.8 / 39.8  55.7 / 55.5  76.7 / 72.4
-//   FP64 forced    7.3 / 11.9  12.6 / 19.3  21.0 / 27.3  36.1 / 39.9  52.6 / 55.4  72.0 / 72.7
-//   FP32 rho=K=1   4.7 / 7.9    6.5 / 10.4  10.2 / 13.4  15.2 / 15.8  23.0 / 20.6  36.0 / 28.6
-//   FP32 var.      5.7 / 8.6    7.7 / 12.8  12.1 / 15.1  18.6 / 19.5  30.7 / 26.0  46.2 / 37.5
-// (Fehlberg stages at 1024^2: 0.2 ms per attempt in either form.)
 // A grid of cells has at most 65535 rows of them (a narrow grid can have more).
 bool cells_fit(const sbp_ctx* ctx) { return ctx->ny <= 65535LL * kCellTY; }
-bool use_cell(const sbp_ctx* ctx) {
-  if (ctx->form != SBP_FORM_BY_SIZE) return cells_fit(ctx) && ctx->form == SBP_FORM_CELLS;
-  const bool early = ctx->fp32 || wave_kind(ctx) == WK_HOM;
-  return cells_fit(ctx) && ctx->npts <= (early ? 1150000 : 1600000);
+
+// Whether a stage of a 2D wave context runs in its cell form (wave_cell.cuh) rather than the
+// persistent one. Constant coefficients and FP32: the cell form's short CTAs win until a grid
+// gives every SM enough tiles to fill the persistent pipeline. FP64 with coefficients: they win
+// throughout, since the conversion to words and its use are spread over more warps. Measured,
+// us per RK4 stage at order 4, cells / persistent tiles, and their ratio at orders 2 and 6:
+//                  1025x1026              1283x1282             2049x2050             4097x4096
+//   FP64 rho=K=1  29.7 /  33.4 .88 .93   45.4 / 45.9 .99 1.02  102 /  92 1.11 1.18
+//   FP64 var.     38.0 /  46.2 .79 .84   55.7 / 64.9 .84  .88  127 / 139  .91  .95  475 / 493 .97 1.01
+//   FP64 forced   38.0 /  45.5 .87 .83   55.2 / 64.2 .90  .87  127 / 140  .96  .93  476 / 509 1.0  .97
+//   FP32 rho=K=1  16.7 /  17.8 .98 .90   24.6 / 22.9 1.10 1.03  63 /  50 1.21 1.25
+//   FP32 var.     18.3 /  20.0 .94 .94   28.5 / 25.1 1.11 1.11  69 /  57 1.20 1.25
+// Grids of the same points at 1:4 and 4:1 have ratios within 0.05 of the square's (1025^2: .83 to
+// .91 at rho=K=1, order 4).
+// Fehlberg stages hold up to six derivatives of a point, which costs cells CTAs per SM, and of
+// the forced problem a cosine per cell: 650x652 .98, 801x802 1.04, 1025x1026 1.10; rho=K=1 and
+// variable .97 and .95 at 1025x1026, 1.04 and 1.00 at 1283x1282 (.97 to 1.06 at orders 2 and 6).
+bool use_cell(const sbp_ctx* ctx, bool fehlberg = false) {
+  if (!cells_fit(ctx)) return false;
+  if (ctx->form != SBP_FORM_BY_SIZE) return ctx->form == SBP_FORM_CELLS;
+  const int kind = wave_kind(ctx);
+  if (fehlberg) return ctx->npts <= (kind == WK_MMS ? 450000 : 1150000);
+  return (kind != WK_HOM && !ctx->fp32) || ctx->npts <= 1150000;
 }
 
 // Encodes one 3D tensor map (x, y, component) over a state buffer of the context.
@@ -446,8 +454,11 @@ int enqueue_step(sbp_ctx* ctx, double t, double dt, const double* ct = nullptr) 
   return SBP_OK;
 }
 
-// Whether a context's RK4 steps run as one launch each (wave_step.cuh).
+// Whether a context's RK4 steps run as one launch each (wave_step.cuh). Two blocks at order 6
+// have twelve closure rows a line, all in one CTA: 9.0 us a stage at 65x66 to 129x130 against 8.2
+// to 8.8 in cells (order 4: 6.0 to 6.1 against 7.4 to 8.1).
 bool use_step(const sbp_ctx* ctx) {
+  if (ctx->ysplit && ctx->d.order == 6) return false;
   return ctx->form == SBP_FORM_BY_SIZE && ctx->wave && !ctx->fp32 && step_takes(ctx->d.order, ctx->nx, ctx->ny);
 }
 
@@ -700,7 +711,7 @@ Rk45Buffers rk45_buffers(sbp_ctx* ctx) {
 // CTAs of the last Fehlberg stage of a 2D wave problem (as launch_cell and launch_wave
 // size their grids).
 int wave_grid(const sbp_ctx* ctx) {
-  if (use_cell(ctx)) {
+  if (use_cell(ctx, true)) {
     const dim3 g = cell_grid(ctx->nx, ctx->ny);
     return (int)(g.x * g.y);
   }
@@ -754,7 +765,7 @@ int launch_rkf_wave_stage(sbp_ctx* ctx, int s, void* in, const WaveMaps* in_maps
   p.rkrtol = ctx->rk_rtol;
   p.wait_ns = ctx->wait_ns;
   set_fixed_scales(p, ctx->d.order, ctx->hix, ctx->hiy);
-  if (use_cell(ctx))
+  if (use_cell(ctx, true))
     CK(launch_cell<double>(ctx->d.order, wave_kind(ctx), ST_RKF1 + s - 1, false, p, ctx->stream));
   else
     CK(launch_wave<double>(ctx->d.order, wave_kind(ctx), ST_RKF1 + s - 1, *in_maps, p, ctx->stream));

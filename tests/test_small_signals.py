@@ -165,7 +165,8 @@ def test_wave_2d(sbp, port, kind, nx, ny, order, form):
 @pytest.mark.parametrize("field", [False, True], ids=["constant", "field"])
 @pytest.mark.parametrize("order", [2, 4, 6])
 def test_advection_2d(sbp, port, order, field):
-    for nx, ny in ((205, 203), (703, 651)):  # one and two rows per thread
+    # the line form at order 2, cells of one row per thread, of two (constant velocities), of two
+    for nx, ny in ((205, 203), (411, 401), (703, 651), (1101, 1001), (1056, 1072)):
         kw = {"a": 1.5, "b": -1.0}
         if field:
             rng = np.random.default_rng(nx)
