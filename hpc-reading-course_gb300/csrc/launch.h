@@ -169,6 +169,8 @@ bool line_steps_takes(long long nx, int kind, int elem_bytes);
 // that need none).
 template <typename T>
 cudaError_t launch_wave3d(int order, int stage, const Wave3Params<T>& prm, const Wave3Maps* maps, cudaStream_t s);
+// The CTAs its FP64 form runs.
+long long wave3d_ctas(long long nx, long long ny, long long nz);
 // Shared-memory opt-in of the 3D stage kernels of one order (outside stream capture).
 template <typename T> cudaError_t configure_wave3d(int order);
 

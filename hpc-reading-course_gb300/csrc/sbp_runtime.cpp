@@ -381,6 +381,11 @@ int launch_stage(sbp_ctx* ctx, int stage, int rk, double t, double dt, void* in,
     p.fx_rho[1] = ctx->hiz / ctx->hix;
     if (ctl) p.skip = &ctl->done;
     p.err = ctx->err;
+    p.wait_ns = ctx->wait_ns;
+    if (stage == ST_RHS && !ctl) {  // a direct launch (RHS evaluation), never a captured one
+      p.test_drop_tile = ctx->drop_tile;
+      ctx->drop_tile = 0;
+    }
     const Wave3Maps* maps = ctx->fp32 ? nullptr : (in == ctx->un ? &ctx->maps3[0] : (in == ctx->wa ? &ctx->maps3[1] : &ctx->maps3[2]));
     CK(launch_wave3d<T>(ctx->d.order, stage, p, maps, ctx->stream));
   } else {
@@ -1327,9 +1332,16 @@ int sbp_test_wave_form(sbp_ctx* ctx, int form) {
 
 int sbp_test_drop_tile(sbp_ctx* ctx, long long tile) {
   if (!ctx) return SBP_ERR_INVALID;
-  if (!ctx->wave) return fail(ctx, SBP_ERR_UNSUPPORTED, "the tile-drop test aid exists for the 2D wave kernels");
-  const int ty = wave_tile_height((int)ctx->es, wave_kind(ctx));
-  const long long ntiles = ((ctx->nx + kWaveTX - 1) / kWaveTX) * ((ctx->ny + ty - 1) / ty);
+  const bool fixed3 = ctx->three_d && !ctx->fp32;
+  if (!ctx->wave && !fixed3)
+    return fail(ctx, SBP_ERR_UNSUPPORTED, "the tile-drop test aid exists for the 2D and the FP64 3D wave kernels");
+  long long ntiles;
+  if (fixed3) {
+    ntiles = wave3d_ctas(ctx->nx, ctx->ny, ctx->nz);
+  } else {
+    const int ty = wave_tile_height((int)ctx->es, wave_kind(ctx));
+    ntiles = ((ctx->nx + kWaveTX - 1) / kWaveTX) * ((ctx->ny + ty - 1) / ty);
+  }
   if (tile < 0 || tile >= ntiles) return fail(ctx, SBP_ERR_INVALID, "tile index out of range");
   ctx->drop_tile = (int)(tile + 1);
   return SBP_OK;

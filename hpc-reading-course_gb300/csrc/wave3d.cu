@@ -427,11 +427,16 @@ inline int fixed3_chunk(long long columns, int nz) {
   return (int)(z < 4 ? 4 : (z > 12 ? 12 : z));
 }
 
+inline dim3 fixed3_grid(long long nx, long long ny, int nz) {
+  const long long gx = (nx + kF3X - 1) / kF3X, gy = (ny + kF3Y - 1) / kF3Y;
+  const int chunk = fixed3_chunk(gx * gy, nz);
+  return dim3((unsigned)gx, (unsigned)gy, (unsigned)((nz + chunk - 1) / chunk));
+}
+
 template <int ORD, int STAGE>
 cudaError_t fixed3_one(const Wave3Params<double>& prm, const Wave3Maps& maps, cudaStream_t s) {
-  const long long gx = (prm.nx + kF3X - 1) / kF3X, gy = (prm.ny + kF3Y - 1) / kF3Y;
-  const int chunk = fixed3_chunk(gx * gy, prm.nz);
-  const dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)((prm.nz + chunk - 1) / chunk));
+  const dim3 grid = fixed3_grid(prm.nx, prm.ny, prm.nz);
+  const int chunk = fixed3_chunk((long long)grid.x * grid.y, prm.nz);
   wave3d_fixed_kernel<ORD, STAGE><<<grid, kF3Threads, Fixed3<ORD, STAGE>::SMEM, s>>>(maps, prm, chunk);
   return cudaGetLastError();
 }
@@ -510,6 +515,11 @@ template <typename T, int ORD> cudaError_t configure_order() {
   return configure_stage<T, ORD, ST_LAST>();
 }
 }  // namespace
+
+long long wave3d_ctas(long long nx, long long ny, long long nz) {
+  const dim3 g = fixed3_grid(nx, ny, (int)nz);
+  return (long long)g.x * g.y * g.z;
+}
 
 template <typename T> cudaError_t configure_wave3d(int order) {
   switch (order) {

@@ -34,6 +34,10 @@ template <typename T> struct Wave3Params {
   T c_acc, c_w;           // acc (+)= c_acc * k ; w = u^n + c_w * k
   const int* skip;        // non-null and set: the kernel returns at entry
   int* err;               // error word
+  // FP64: limit of the bounded waits in ns (0: kWaitLimitNs); test aid: k + 1 makes CTA k
+  // issue no load for its first planes, so that its wait for them runs out (0: none)
+  unsigned long long wait_ns;
+  int test_drop_tile;
   // FP64 (wave3d_fixed_kernel): the RHS is formed in units of sigma_d = -hi_d/den per direction
   // (u, v, w: their own, p: sigma_x); sigma, 1/sigma, sigma_y/sigma_x and sigma_z/sigma_x,
   // and the stage's RK4 coefficients times each component's sigma

@@ -148,6 +148,8 @@ __global__ void __launch_bounds__(kF3Threads, 2)
   const int groups = k1 - k0 + 2 * R;
   const auto issue = [&](int g) {
     if (g >= groups) return;
+    if (g == 0 && prm.test_drop_tile == 1 + (int)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)))
+      return;
     const int sa = g % SA, m = k0 - R + g, kb = m - R;
     double* a = sA + sa * G::A_SZ;
     const bool own = kb >= k0;
@@ -183,7 +185,7 @@ __global__ void __launch_bounds__(kF3Threads, 2)
     double* b = sB + (own ? (kb - k0) % SB : 0) * G::B_SZ;
     long long* ia = reinterpret_cast<long long*>(a);
     long long* ib = reinterpret_cast<long long*>(b);
-    const bool late = !mbar_wait_bounded(&full[sa], (g / SA) & 1);  // the copy will not complete
+    const bool late = !mbar_wait_bounded(&full[sa], (g / SA) & 1, prm.wait_ns);  // the copy will not complete
     bool outa = false, outb = false;
 #pragma unroll
     for (int c = 0; c < G::PER_A; c++) {
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kF3Threads, 2)
       if (tid == 0) {
         atomicOr(prm.err, ERR_TMA_TIMEOUT);
         // let the copies in flight land (bounded) before the CTA's shared memory goes
-        for (int q = g; q < issued; q++) mbar_wait_bounded(&full[q % SA], (q / SA) & 1);
+        for (int q = g; q < issued; q++) mbar_wait_bounded(&full[q % SA], (q / SA) & 1, prm.wait_ns);
       }
       return;
     }

@@ -199,7 +199,7 @@ int sbp_get_stream(const sbp_ctx* ctx, void** stream);
 long long sbp_launch_count(const sbp_ctx* ctx);
 
 /* Failure detection (no counterpart in the reference, whose MPI ranks have
- * no device waits). Every mbarrier wait in the 2D wave stage kernels is
+ * no device waits). Every mbarrier wait in the 2D and 3D wave stage kernels is
  * bounded by %globaltimer; a wait that runs out sets the context's error word,
  * the kernel lets its copies in flight land and returns, and the next
  * sbp_synchronize (or the synchronous entry point that launched it) returns
@@ -208,7 +208,8 @@ long long sbp_launch_count(const sbp_ctx* ctx);
  *   the context's captured step graphs, which carry the old limit.
  * sbp_test_drop_tile: test aid for that path. The next sbp_rhs / sbp_apply of
  *   a 2D wave context issues no load for tile `tile` (row-major index of the
- *   stage kernel's tiles), so the wait for it runs out and the call returns
+ *   stage kernel's tiles), of an FP64 3D wave context none for the first planes
+ *   of CTA `tile`, so the wait for it runs out and the call returns
  *   SBP_ERR_DEVICE. Nothing faults or hangs; never applies to RK4 steps. */
 int sbp_set_wait_limit(sbp_ctx* ctx, long long ns);
 int sbp_test_drop_tile(sbp_ctx* ctx, long long tile);
