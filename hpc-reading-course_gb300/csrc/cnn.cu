@@ -47,8 +47,8 @@ __device__ __forceinline__ uint32_t pack_pair(bf16 lo, bf16 hi) {
   return (uint32_t)__bfloat16_as_ushort(lo) | ((uint32_t)__bfloat16_as_ushort(hi) << 16);
 }
 
-// The widest pixel tile: 32 x 4 pixels.
-constexpr int kConvMaxTw = 32;
+// The widest pixel tiles: 32 x 4 pixels, and for images one or two pixels high 64 x 2.
+constexpr int kConvMaxTw = 32, kConvStripTw = 64;
 // A column box: 128 / tw + 2 rows of tw pixels, rounded up to whole 1024-byte units.
 __host__ __device__ constexpr int conv_box_bytes(int tw, int rowb) {
   return ((128 / tw + 2) * tw * rowb + 1023) / 1024 * 1024;
@@ -179,6 +179,7 @@ struct TcConv {
   static constexpr uint32_t LAYOUT = CIN == 32 ? 4u : 6u;  // 64-byte / 32-byte swizzle
   static constexpr uint32_t ATOM = 8 * ROWB;
   static constexpr int NS = 6;    // column boxes in flight: two pixel tiles per CTA
+  static constexpr int slots(int tw) { return tw > kConvMaxTw ? 4 : NS; }
   static constexpr int CTAS = 2;  // resident CTAs per SM (forward pass at 8 x 258 x 257, launches not overlapped: 0.138 ms; three
                                   // CTAs with 4 boxes 0.138 ms, four with 3 boxes 0.146 ms)
   static constexpr int B_BYTES = COUT * ROWB;
@@ -188,11 +189,12 @@ struct TcConv {
   // full[NS], empty[NS], wbar, accfull[NACC], accempty[NACC], done; then the tensor-memory address
   static constexpr int NBAR = 2 * NS + 2 * NACC + 2;
   static constexpr int HEAD = (off_bar() + 8 * NBAR + 16 + 1023) / 1024 * 1024;  // weights, barriers
-  static constexpr int smem(int tw) { return HEAD + NS * box_bytes(tw) + 1024; }  // + the dynamic base's slack
+  static constexpr int smem(int tw) { return HEAD + slots(tw) * box_bytes(tw) + 1024; }  // + the dynamic base's slack
   static constexpr uint32_t IDESC = umma_idesc_bf16(128, COUT);
   static constexpr int THREADS = 192;  // producer, MMA issuer, four epilogue warps
   static_assert(B_BYTES % 256 == 0, "tiles start on swizzle atoms");
-  static_assert(CTAS * (smem(kConvMaxTw) + 1024) <= 228 * 1024, "shared memory");
+  static constexpr int SMEM_MAX = smem(kConvMaxTw) > smem(kConvStripTw) ? smem(kConvMaxTw) : smem(kConvStripTw);
+  static_assert(CTAS * (SMEM_MAX + 1024) <= 228 * 1024, "shared memory");
 };
 
 // The two halves of grid_dependency_wait. A kernel whose CTAs take several tiles does not
@@ -203,6 +205,19 @@ struct TcConv {
 // 112 without overlap.
 __device__ __forceinline__ void grid_inputs_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_let_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Waits for the last loads of a ring of n slots, the next of which would go to slot s, after
+// `round` times round: no copy may be in flight when a CTA exits.
+__device__ __forceinline__ void drain_ring(uint64_t* full, int s, int round, int n) {
+  int q = round > 0 ? s : 0, r = round > 0 ? round - 1 : 0;
+  for (int left = round > 0 ? n : s; left > 0; left--) {
+    mbar_wait_bounded(&full[q], r & 1);
+    if (++q == n) {
+      q = 0;
+      r++;
+    }
+  }
+}
 
 // The pixel tiles of a persistent CTA: every gridDim.x-th, as tile column, tile row and
 // image, stepped by carries instead of divided out of a tile number.
@@ -244,6 +259,9 @@ struct TileWalk {
 // accumulators (32 columns each); warps 2-5 read an accumulator (warp w: lanes 32 (w % 4) ..),
 // release it, and add bias, apply ReLU and store while the next tile accumulates in the other.
 // Bounded waits.
+// W, H here: the extents along and across a tile's rows. `turned`: those rows run down the image
+// (xmap is then {CIN, image height, image width, B}); the taps change places with the weights'
+// loads, and only the pixels' addresses differ.
 //
 // What bounded it was the MMA warp's instructions: with the loads, the stores and eight of
 // nine MMAs left out the forward pass (8 x 258 x 257) still took 0.161 of its 0.197 ms.
@@ -263,11 +281,11 @@ template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>::CTAS)
     conv3x3_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
                       const float* __restrict__ bias, const bf16* __restrict__ mask, void* __restrict__ y, int B, int H,
-                      int W, int tw, int th, int* err) {
+                      int W, int tw, int th, bool turned, int* err) {
   static_assert(!MASK || (!RELU && !OUT_F32), "the mask is the input gradient's, in BF16");
   using L = TcConv<CIN, COUT>;
   constexpr int NS = L::NS;
-  const int box = L::box_bytes(tw), box_tx = (th + 2) * tw * L::ROWB;
+  const int box = L::box_bytes(tw), box_tx = (th + 2) * tw * L::ROWB, ns = L::slots(tw);
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
   unsigned char* boxes = smem + L::HEAD;
@@ -304,26 +322,30 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
   if (warp == 0) {  // ---- loads
     if (lane == 0) {
       mbar_arrive_expect_tx(wbar, 9 * L::B_BYTES);
-      for (int t = 0; t < 9; t++) tma_load_3d(smem + t * L::B_BYTES, &wmap, 0, t, 0, wbar);
-      int k = 0;
+      const int along = turned ? 3 : 1, over = turned ? 1 : 3;  // taps along and across the tile's rows
+#pragma unroll
+      for (int t = 0; t < 9; t++) tma_load_3d(smem + t * L::B_BYTES, &wmap, 0, t / 3 * over + t % 3 * along, 0, wbar);
+      int s = 0, round = 0;  // the next slot, times round the ring
       bool ok = true;
       for (TileWalk t(ntw, nth); ok && t.b < B; t.next()) {
         const int w0 = t.w * tw, h0 = t.h * th, b = t.b;
-        for (int dx = 0; dx < 3; dx++, k++) {
-          const int s = k % NS;
-          if (k >= NS && !mbar_wait_bounded(&empty[s], ((k / NS) - 1) & 1)) {
+        for (int dx = 0; dx < 3; dx++) {
+          if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1)) {
             atomicOr(err, 1);
             ok = false;
             break;
           }
           mbar_arrive_expect_tx(&full[s], box_tx);
           tma_load_4d(boxes + s * box, &xmap, 0, w0 + dx - 1, h0 - 1, b, &full[s]);
+          if (++s == ns) {
+            s = 0;
+            round++;
+          }
         }
       }
       if (ntiles <= (int)gridDim.x) grid_let_next();
-      // no copy may be in flight when the CTA exits
       mbar_wait_bounded(wbar, 0);
-      for (int kk = (k >= NS ? k - NS : 0); kk < k; kk++) mbar_wait_bounded(&full[kk % NS], (kk / NS) & 1);
+      drain_ring(full, s, round, ns);
     }
   } else if (warp == 1) {  // ---- MMAs
     const uint32_t leader = lane == 0;
@@ -344,7 +366,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
         sl[dx] = slot;
         a[dx] = a0 + (uint64_t)(slot * box16);
         if (ok) ok = mbar_wait_warp(&full[slot], phase);
-        if (++slot == NS) {
+        if (++slot == ns) {
           slot = 0;
           phase ^= 1;
         }
@@ -377,7 +399,7 @@ __global__ void __launch_bounds__(TcConv<CIN, COUT>::THREADS, TcConv<CIN, COUT>:
       const int buf = it % L::NACC, b = t.b;
       const int hh = t.h * th + hm, ww = t.w * tw + wm;
       const bool inside = hh < H && ww < W;
-      const long long p = ((long long)b * H + hh) * W + ww;
+      const long long p = turned ? ((long long)b * W + ww) * H + hh : ((long long)b * H + hh) * W + ww;
       uint4 mk[MASK ? COUT / 8 : 1];
       if (MASK && inside) {
 #pragma unroll
@@ -453,26 +475,29 @@ struct TcWgrad {
   static constexpr uint32_t A_SBO = 8 * A_ROWB, B_SBO = 8 * B_ROWB;
   static constexpr int NST = 5;  // stages: the next tiles load while this one's MMAs run (8 x 258 x 257, with
                                  // the descriptors in uniform registers: 41 -> 32 us per layer)
+  static constexpr int stages(int tw) { return tw > kConvMaxTw ? 3 : NST; }
   static constexpr int stage(int tw) { return 3 * conv_box_bytes(tw, A_ROWB) + B_BYTES; }
   static constexpr int HEAD = 1024;  // barriers, tensor-memory address
-  static constexpr int smem(int tw) { return HEAD + NST * stage(tw) + 1024; }
+  static constexpr int smem(int tw) { return HEAD + stages(tw) * stage(tw) + 1024; }
   static constexpr uint32_t IDESC = umma_idesc_bf16(128, COUT) | (1u << 15) | (1u << 16);  // A, B MN-major
   static constexpr int THREADS = 192;
-  static_assert(smem(kConvMaxTw) <= 227 * 1024, "shared memory");
+  static constexpr int SMEM_MAX = smem(kConvMaxTw) > smem(kConvStripTw) ? smem(kConvMaxTw) : smem(kConvStripTw);
+  static_assert(SMEM_MAX <= 227 * 1024, "shared memory");
   // the fourth row offset of the last column reads one row of pixels past its box: the dy tile
-  static_assert(B_BYTES >= kConvMaxTw * A_ROWB, "operand reads stay in the stage");
+  static_assert(B_BYTES >= kConvStripTw * A_ROWB, "operand reads stay in the stage");
 };
 
 template <int COUT>
 __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
     conv3x3_wgrad_tc_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap dymap,
-                            float* __restrict__ dw_part, int B, int H, int W, int tw, int th, int* err) {
+                            float* __restrict__ dw_part, int B, int H, int W, int tw, int th, bool turned,
+                            int* err) {
   using L = TcWgrad<COUT>;
   constexpr int NST = L::NST, CIN = L::CIN;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* head = smem_raw + ((1024 - (smem_addr(smem_raw) & 1023)) & 1023);
   unsigned char* smem = head + L::HEAD;
-  const int box = conv_box_bytes(tw, L::A_ROWB), stage = L::stage(tw);
+  const int box = conv_box_bytes(tw, L::A_ROWB), stage = L::stage(tw), nst = L::stages(tw);
   uint64_t* full = reinterpret_cast<uint64_t*>(head);
   uint64_t* empty = full + NST;
   uint64_t* accfull = empty + NST;
@@ -498,10 +523,9 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
 
   if (warp == 0) {  // ---- loads
     if (lane == 0) {
-      int it = 0;
-      for (TileWalk t(ntw, nth); t.b < B; t.next(), it++) {
-        const int s = it % NST;
-        if (it >= NST && !mbar_wait_bounded(&empty[s], ((it / NST) - 1) & 1)) {
+      int s = 0, round = 0;  // the next stage, times round the ring
+      for (TileWalk t(ntw, nth); t.b < B; t.next()) {
+        if (round > 0 && !mbar_wait_bounded(&empty[s], (round - 1) & 1)) {
           atomicOr(err, 1);
           break;
         }
@@ -510,9 +534,13 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
         mbar_arrive_expect_tx(&full[s], 3 * (th + 2) * tw * L::A_ROWB + L::B_BYTES);
         for (int dx = 0; dx < 3; dx++) tma_load_4d(st + dx * box, &xmap, 0, w0 + dx - 1, h0 - 1, b, &full[s]);
         tma_load_4d(st + 3 * box, &dymap, 0, w0, h0, b, &full[s]);
+        if (++s == nst) {
+          s = 0;
+          round++;
+        }
       }
       if (ntiles <= (int)gridDim.x) grid_let_next();
-      for (int kk = (it >= NST ? it - NST : 0); kk < it; kk++) mbar_wait_bounded(&full[kk % NST], (kk / NST) & 1);
+      drain_ring(full, s, round, nst);
     }
   } else if (warp == 1) {  // ---- MMAs
     const uint32_t leader = lane == 0;
@@ -532,7 +560,7 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
           umma_bf16(leader, tmem + (uint32_t)(g * COUT), a + g * box16 + (2 * k * L::A_SBO >> 4),
                     b + (2 * k * L::B_SBO >> 4), L::IDESC, (it | k) != 0);
       umma_commit(leader, &empty[s]);
-      if (++s == NST) {
+      if (++s == nst) {
         s = 0;
         phase ^= 1;
       }
@@ -546,7 +574,7 @@ __global__ void __launch_bounds__(TcWgrad<COUT>::THREADS, 1)
 #pragma unroll
       for (int g = 0; g < 3; g++) {
         if (q == 3) continue;
-        const int tap = 3 * q + g;
+        const int tap = turned ? 3 * g + q : 3 * q + g;
 #pragma unroll
         for (int n0 = 0; n0 < COUT; n0 += 16) {
           uint32_t r[16];
@@ -831,6 +859,13 @@ struct sbp_cnn {
   float* loss = nullptr;
   int* err = nullptr;        // the tensor-core convolutions' error word (a bounded wait ran out)
   int tw = 0, th = 0;        // the tensor-core kernels' pixel tile: th rows of tw pixels, th * tw = 128
+  bool turned = false;       // whether those rows run down the image instead of along it
+  int across() const { return turned ? W : H; }  // the image's extent across a tile's rows, and along them
+  int along() const { return turned ? H : W; }
+  // pixel tiles of a batch
+  long long tiles(int batch) const {
+    return (long long)batch * ((across() + th - 1) / th) * ((along() + tw - 1) / tw);
+  }
   int nsm = 1;               // SMs: the persistent convolutions' grid
   float* dw_part[kLayers] = {};  // the weight gradients' per-CTA sums ([nsm][wcount(l)] each, one block)
   long long launches = 0;
@@ -885,16 +920,17 @@ EncodeTiledFn encode_fn() {
   return fn;
 }
 
-// The tensor maps of one convolution: the NHWC BF16 input ({ch, W, H, B}, box {ch, bw,
-// bh, 1}) and the weights ([cout][9][ch]: {ch, 9, cout}, box {ch, 1, cout}), rows
+// The tensor maps of one convolution: the NHWC BF16 input ({ch, W, H, B}, turned {ch, H, W, B},
+// box {ch, bw, bh, 1}) and the weights ([cout][9][ch]: {ch, 9, cout}, box {ch, 1, cout}), rows
 // swizzled over their ch * 2 bytes. Out-of-range boxes read zeros (the image border).
 cudaError_t encode_conv_maps(const sbp_cnn* c, const bf16* x, const bf16* w, int ch, int cout, int batch, int bw,
                              int bh, CUtensorMap* xm, CUtensorMap* wm) {
   EncodeTiledFn enc = encode_fn();
   if (!enc) return cudaErrorNotSupported;
   const CUtensorMapSwizzle sw = ch == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
-  const cuuint64_t xd[4] = {(cuuint64_t)ch, (cuuint64_t)c->W, (cuuint64_t)c->H, (cuuint64_t)batch};
-  const cuuint64_t xs[3] = {(cuuint64_t)ch * 2, (cuuint64_t)c->W * ch * 2, (cuuint64_t)c->H * c->W * ch * 2};
+  const cuuint64_t xd[4] = {(cuuint64_t)ch, (cuuint64_t)c->along(), (cuuint64_t)c->across(), (cuuint64_t)batch};
+  const cuuint64_t px = (cuuint64_t)ch * 2, row = (cuuint64_t)c->W * ch * 2;
+  const cuuint64_t xs[3] = {c->turned ? row : px, c->turned ? px : row, (cuuint64_t)c->H * row};
   const cuuint32_t xb[4] = {(cuuint32_t)ch, (cuuint32_t)bw, (cuuint32_t)bh, 1};
   const cuuint32_t e[4] = {1, 1, 1, 1};
   if (enc(xm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), xd, xs, xb, e, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -912,7 +948,7 @@ cudaError_t encode_conv_maps(const sbp_cnn* c, const bf16* x, const bf16* w, int
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
 cudaError_t configure_tc() {
   return cudaFuncSetAttribute(conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, TcConv<CIN, COUT>::smem(kConvMaxTw));
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, TcConv<CIN, COUT>::SMEM_MAX);
 }
 
 template <int CIN, int COUT, bool RELU, bool OUT_F32, bool MASK>
@@ -921,18 +957,18 @@ cudaError_t launch_tc(const bf16* x, const bf16* w, const float* bias, const bf1
   CUtensorMap xm, wm;
   cudaError_t e = encode_conv_maps(c, x, w, CIN, COUT, batch, c->tw, c->th + 2, &xm, &wm);
   if (e != cudaSuccess) return e;
-  const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
+  const long long tiles = c->tiles(batch);
   const long long slots = (long long)TcConv<CIN, COUT>::CTAS * c->nsm;  // persistent: every CTA resident
   const unsigned grid = (unsigned)(tiles < slots ? tiles : slots);
   return sbp::launch_overlapped(conv3x3_tc_kernel<CIN, COUT, RELU, OUT_F32, MASK>, dim3(grid),
                            dim3(TcConv<CIN, COUT>::THREADS), TcConv<CIN, COUT>::smem(c->tw), s, xm, wm, bias, mask, y,
-                           batch, c->H, c->W, c->tw, c->th, c->err);
+                           batch, c->across(), c->along(), c->tw, c->th, c->turned, c->err);
 }
 
 template <int COUT>
 cudaError_t configure_wgrad_tc() {
   return cudaFuncSetAttribute(conv3x3_wgrad_tc_kernel<COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              TcWgrad<COUT>::smem(kConvMaxTw));
+                              TcWgrad<COUT>::SMEM_MAX);
 }
 
 // Shared-memory opt-in of the tensor-core convolutions (outside stream capture).
@@ -960,7 +996,7 @@ cudaError_t conv_dgrad(int l, const bf16* dy, bf16* dx, const sbp_cnn* c, int ba
 
 // CTAs of the weight gradients: each leaves one partial sum.
 unsigned wgrad_ctas(const sbp_cnn* c, int batch) {
-  const long long tiles = (long long)batch * ((c->H + c->th - 1) / c->th) * ((c->W + c->tw - 1) / c->tw);
+  const long long tiles = c->tiles(batch);
   return (unsigned)(tiles < c->nsm ? tiles : c->nsm);
 }
 
@@ -976,11 +1012,11 @@ cudaError_t conv_wgrad(int l, const bf16* x, const bf16* dy, const sbp_cnn* c, i
   const unsigned grid = wgrad_ctas(c, batch);
   if (cout == 32)
     return sbp::launch_overlapped(conv3x3_wgrad_tc_kernel<32>, dim3(grid), dim3(TcWgrad<32>::THREADS),
-                             TcWgrad<32>::smem(c->tw), s, xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th,
-                             c->err);
+                             TcWgrad<32>::smem(c->tw), s, xm, dym, c->dw_part[l], batch, c->across(), c->along(), c->tw,
+                             c->th, c->turned, c->err);
   return sbp::launch_overlapped(conv3x3_wgrad_tc_kernel<16>, dim3(grid), dim3(TcWgrad<16>::THREADS),
-                           TcWgrad<16>::smem(c->tw), s, xm, dym, c->dw_part[l], batch, c->H, c->W, c->tw, c->th,
-                           c->err);
+                           TcWgrad<16>::smem(c->tw), s, xm, dym, c->dw_part[l], batch, c->across(), c->along(), c->tw,
+                           c->th, c->turned, c->err);
 }
 
 AllWeights all_weights(const sbp_cnn* c) {
@@ -1086,17 +1122,25 @@ int sbp_cnn_create(int height, int width, int max_batch, int device, void* strea
     return bad("cudaMalloc(activations)");
   cudaMemset(c->err, 0, 4);
   // the tensor-core kernels' tile: 128 pixels, th rows of tw, the shape whose tiles cover the
-  // image with the fewest padding pixels (ties: wider rows). tw >= 8: a row of pixels is whole
-  // swizzle atoms, so that the vertical taps can start at any row of a box; tw <= 32: wider
-  // tiles' boxes are mostly halo (64: 4 rows for 2) and five of them overfill shared memory
+  // image with the fewest padding pixels (ties: the first tried). tw >= 8: a row of pixels is
+  // whole swizzle atoms, so that the vertical taps can start at any row of a box; tw <= 32: wider
+  // tiles' boxes are mostly halo (64: 4 rows for 2) and five of them overfill shared memory.
+  // Images up to four pixels wide turn the tile, one or two pixels high or wide take 64 x 2:
+  // forward pass at 8 x 32768 x 1 122 us (with upright tiles of 8 x 16 pixels 282), 8 x 1 x 32768
+  // 122 (32 x 4 pixels: 160), 8 x 20000 x 3 135 (201).
   long long best = -1;
-  for (int tw = kConvMaxTw; tw >= 8; tw /= 2) {
-    const int th = 128 / tw;
-    const long long area = (long long)((width + tw - 1) / tw) * tw * ((height + th - 1) / th) * th;
-    if (best < 0 || area < best) {
-      best = area;
-      c->tw = tw;
-      c->th = th;
+  for (int t = 0; t < (width <= 4 ? 2 : 1); t++) {
+    const int along = t ? height : width, across = t ? width : height;
+    for (int tw : {32, 16, 8, kConvStripTw}) {
+      if (tw > kConvMaxTw && across > 2) continue;
+      const int th = 128 / tw;
+      const long long area = (long long)((along + tw - 1) / tw) * tw * ((across + th - 1) / th) * th;
+      if (best < 0 || area < best) {
+        best = area;
+        c->tw = tw;
+        c->th = th;
+        c->turned = t != 0;
+      }
     }
   }
   if (configure_convs() != cudaSuccess) return bad("cudaFuncSetAttribute(convolutions)");
