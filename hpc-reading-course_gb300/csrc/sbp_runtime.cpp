@@ -467,8 +467,10 @@ bool use_step(const sbp_ctx* ctx) {
   return ctx->form == SBP_FORM_BY_SIZE && ctx->wave && !ctx->fp32 && step_takes(ctx->d.order, ctx->nx, ctx->ny);
 }
 
-// One RK4 step from `in` to `out` in one launch; ct as for enqueue_step.
+// One RK4 step from `in` to `out` in one launch. Time-dependent problems: ct is where the step's
+// three stage-time factors are in device memory.
 int enqueue_whole_step(sbp_ctx* ctx, void* in, void* out, double dt, const double* ct) {
+  if (ctx->time_dependent && !ct) return fail(ctx, SBP_ERR_INVALID, "a whole step without its stage-time factors");
   WaveParams<double> p = wave_params<double>(ctx);
   p.in = (const double*)in;
   p.wout = (double*)out;

@@ -182,7 +182,7 @@ template <typename T, int KIND> constexpr int wave_coef() { return KIND == WK_VA
 #ifndef SBP_FP64_RING_FL
 #define SBP_FP64_RING_FL 4
 #endif
-// The Fehlberg and RHS stages load no point boxes: a ring of 6 stages.
+// The Fehlberg stages load no point boxes: a ring of 6 stages (4 with coefficient planes).
 #ifndef SBP_FP64_RING_RKF
 #define SBP_FP64_RING_RKF 6
 #endif
@@ -191,9 +191,7 @@ template <typename T, int KIND, int STAGE = ST_MID> constexpr int wave_ring() {
   if (is_rkf_stage(STAGE)) return KIND == WK_HOM ? SBP_FP64_RING_RKF : 4;
   return (KIND == WK_HOM && (STAGE == ST_FIRST || STAGE == ST_LAST)) ? SBP_FP64_RING_FL : SBP_FP64_RING;
 }
-// Consumer (compute) warps of the single-instance kernels. FP64: one tile row each (the
-// Fehlberg stages of constant and variable coefficients two rows each: they hold up to
-// six derivatives of a point in registers). FP32: 16 with two rows each for constant
+// Consumer (compute) warps of the single-instance kernels. FP64: one tile row each. FP32: 16 with two rows each for constant
 // coefficients (more warps hide more load latency), 12 for variable coefficients.
 #ifndef SBP_FP32_WARPS
 #define SBP_FP32_WARPS 16
@@ -203,7 +201,7 @@ template <typename T, int KIND, int STAGE = ST_MID> constexpr int wave_ring() {
 #ifndef SBP_FP32_VAR_WARPS
 #define SBP_FP32_VAR_WARPS 12
 #endif
-template <typename T, int KIND, int STAGE = ST_MID> constexpr int wave_warps() {
+template <typename T, int KIND> constexpr int wave_warps() {
   if (sizeof(T) == 4) return KIND != WK_VAR ? SBP_FP32_WARPS : SBP_FP32_VAR_WARPS;
   return KIND == WK_HOM ? SBP_FP64_WARPS : wave_ty<T, KIND>();
 }
@@ -257,7 +255,7 @@ struct WaveTile {
   // + 192: the tile index of each stage (int[NST]; -1 marks the end)
   // Fixed-point stages, at OFF_FX: barriers[8] "exponent maxima known" (+0) and
   // "boxes converted" (+64), then per stage and converter warp the p and u/v exponent
-  // maxima (int[8][8][2], +128).
+  // maxima, or whether a value had no word (int[8][8][2], +128).
   static constexpr int OFF_FX = OFF_BAR + 256;
   // Decomposed grids: eight 192-byte slots of tile geometry (that of its subdomain's
   // neighbours included): one per ring stage, the rest the exchange queue; then the
@@ -649,7 +647,7 @@ __device__ __forceinline__ void wave_tile_compute(const WaveParams<T>& prm, cons
 // The Tile type of the single-instance kernel for (T, order, kind, stage).
 template <typename T, int ORD, int KIND, int STAGE>
 using WaveStageTile = WaveTile<T, ORD, STAGE, wave_ty<T, KIND>(), 0, wave_coef<T, KIND>(), wave_ring<T, KIND, STAGE>(),
-                               wave_warps<T, KIND, STAGE>(), wave_fixed<T, KIND, STAGE>(),
+                               wave_warps<T, KIND>(), wave_fixed<T, KIND, STAGE>(),
                                wave_fixed<T, KIND, STAGE>() ? wave_conv<KIND, STAGE>() : 0>;
 
 // The producer (one lane): takes the CTA's tiles, from the dynamic queue or with a

@@ -103,15 +103,6 @@ template <int ORD, int STAGE> struct Fixed3 {
   static_assert(SMEM + 4096 <= 227 * 1024, "ring exceeds shared memory");
 };
 
-__device__ __forceinline__ void tma_load_4d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, int c,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(smem_addr(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(c), "r"(smem_addr(bar))
-      : "memory");
-}
-
 template <int ORD, int STAGE>
 __global__ void __launch_bounds__(kF3Threads, 2)
     wave3d_fixed_kernel(const __grid_constant__ Wave3Maps maps, const __grid_constant__ Wave3Params<double> prm,

@@ -63,9 +63,9 @@ template <int ORD> __host__ __device__ inline void step_reads(int& lo, int& hi, 
 }
 
 // The RK4 coefficients times each component's scale (set_fixed_scales): ca dt/6 and dt/3, cw
-// dt/2 and dt; and the forcing's factor at t, t + dt/2, t + dt where no table holds it.
+// dt/2 and dt.
 struct WaveStepCoef {
-  double ca[2][3], cw[2][3], ct[3];
+  double ca[2][3], cw[2][3];
 };
 
 // SAT of a face point, to be added to its RHS (the terms of apply_sat, one direction each).
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) wave_step_kernel(const __grid
   double ct[3] = {0, 0, 0};
   if constexpr (KIND == WK_MMS) {
 #pragma unroll
-    for (int m = 0; m < 3; m++) ct[m] = prm.ctp ? ld_l2(prm.ctp + m) : cf.ct[m];
+    for (int m = 0; m < 3; m++) ct[m] = ld_l2(prm.ctp + m);  // the forcing's factor at t, t + dt/2, t + dt
   }
   int px0 = bx0, px1 = bx1, py0 = by0;  // the rectangle the values v belong to
 
