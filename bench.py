@@ -662,8 +662,8 @@ def run_wave3d_study(args):
     w = 0.2 at the origin, --grid3d^3 points, order --order, dt = 0.2 h, 100 RK4 steps per timed run,
     FP64 and compensated FP32, state resident in HBM, timed with CUDA events on the context's stream.
     Roofs: HBM with 16 c s bytes per point and RK4 step (c = 4), and for FP64 the FP64 pipe at
-    about 33 FP64 instructions per point-stage (order 4: six derivatives of 4 instructions, two adds,
-    7 for the stage update on average). CPU: the oracle restatement on all host cores, a bounded
+    nine FP64 instructions per point-stage (the interior stencils are integer sums; two for the sum of
+    the pressure's three terms, 7 for the stage update on average). CPU: the oracle restatement on all host cores, a bounded
     number of steps."""
     import numpy as np
     import torch
@@ -700,8 +700,8 @@ def run_wave3d_study(args):
         line = {"point_stage_per_s": rate, "seconds": sec, "achieved_gbs": bytes_step * steps / sec / 1e9}
         line["hbm_frac"] = line["achieved_gbs"] / peak
         if prec == sbpgpu.FP64 and dfma:
-            line["fp64_alu_bound_point_stage_per_s"] = dfma / 33.0
-            line["fp64_alu_frac"] = rate / (dfma / 33.0)
+            line["fp64_alu_bound_point_stage_per_s"] = dfma / 9.0
+            line["fp64_alu_frac"] = rate / (dfma / 9.0)
         out[name] = line
     if not args.no_cpu:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))

@@ -37,7 +37,7 @@ template <typename T, int ORD, int KIND> struct LineSteps {
 };
 
 // den times the interior stencil sum around c by integer arithmetic with the exponent of its
-// own largest value (wave2d_fixed.cuh, the finer unit): some 100 integer instructions take half
+// own largest value (wave2d_fixed.cuh, fx_from<true>): some 100 integer instructions take half
 // the time of four FP64 FMAs at 64 clocks each. False where the values leave the fixed-point
 // range.
 template <int ORD>

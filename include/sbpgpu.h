@@ -74,7 +74,14 @@ typedef struct {
   int bc;             /* sbp_bc */
   int precision;      /* sbp_precision: SBP_FP32 keeps an FP32 state with a
                          compensated (Kahan) RK4 update; SAT weights and all
-                         norms stay FP64 */
+                         norms stay FP64. SBP_FP64: a stencil's result is as
+                         accurate as FP64 arithmetic on the values it reads, but
+                         for the RHS and RK4 stages of SBP_WAVE_HOM_2D (its
+                         decomposed and no-allocation forms and batched FP64
+                         waves included; not its grids small enough for whole
+                         steps in one launch), where the interior stencils err by
+                         a few 2^-52 of the largest value in the same tile (up
+                         to 64 x 14 points and their halo) */
   long long nx, ny;   /* grid points per direction (ny ignored in 1D) */
   double xl[2], xr[2];/* domain [xl, xr]; h = (xr - xl)/(N - 1) as the demos */
   double a, b;        /* advection velocities (x, y) */
